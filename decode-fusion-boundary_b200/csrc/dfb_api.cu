@@ -8,7 +8,7 @@
 #include "dfb_pairgemv.cuh"
 #include "dfb_tcgemv.cuh"
 #include "dfb_attnring.cuh"
-#include "dfb_prefill.cuh"
+#include "dfb_prefilltc.cuh"
 
 #include <cstdio>
 #include <cstdlib>
@@ -446,38 +446,46 @@ typedef CUresult (*TensorMapEncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cu
                                            const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
                                            CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                                            CUtensorMapFloatOOBfill);
-int tc_weight_map(const void* w, int rows, int box_rows, CUtensorMap* out) {
-  static std::mutex mu;
+// a map of [rows, cols] bf16 with `stride` elements between rows, boxes {64 columns, box_rows}, 128-byte swizzle
+int tc_encode_map(const void* p, int64_t cols, int64_t rows, int64_t stride, int box_rows, CUtensorMap* out) {
   static TensorMapEncodeTiledFn encode = nullptr;
-  static std::map<std::tuple<const void*, int, int>, CUtensorMap> cache;
-  std::lock_guard<std::mutex> lock(mu);
-  auto key = std::make_tuple(w, rows, box_rows);
-  auto it = cache.find(key);
-  if (it != cache.end()) { *out = it->second; return 0; }
-  if (!encode) {
-    void* fn = nullptr;
-    cudaDriverEntryPointQueryResult qres;
-    cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres);
-    if (e != cudaSuccess) return (int)e;
-    if (!fn || qres != cudaDriverEntryPointSuccess) return (int)cudaErrorNotSupported;
-    encode = (TensorMapEncodeTiledFn)fn;
+  {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    if (!encode) {
+      void* fn = nullptr;
+      cudaDriverEntryPointQueryResult qres;
+      cudaError_t e = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &qres);
+      if (e != cudaSuccess) return (int)e;
+      if (!fn || qres != cudaDriverEntryPointSuccess) return (int)cudaErrorNotSupported;
+      encode = (TensorMapEncodeTiledFn)fn;
+    }
   }
-  if ((uintptr_t)w % 16) return DFB_E_BAD_ARG;
-  const cuuint64_t dims[2] = {(cuuint64_t)kTcK, (cuuint64_t)rows};       // innermost first
-  const cuuint64_t strides[1] = {(cuuint64_t)kTcK * sizeof(bf16)};       // bytes between rows
+  if ((uintptr_t)p % 16) return DFB_E_BAD_ARG;
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};       // innermost first
+  const cuuint64_t strides[1] = {(cuuint64_t)stride * sizeof(bf16)};     // bytes between rows
   const cuuint32_t box[2] = {64u, (cuuint32_t)box_rows};
   const cuuint32_t elem[2] = {1u, 1u};
-  CUtensorMap m;
-  CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(w), dims, strides, box, elem,
+  CUresult r = encode(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(p), dims, strides, box, elem,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     if (dfb_debug()) fprintf(stderr, "dfb: cuTensorMapEncodeTiled failed with %d\n", (int)r);
     return (int)cudaErrorInvalidValue;
   }
+  return 0;
+}
+int tc_weight_map(const void* w, int rows, int box_rows, CUtensorMap* out) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, int>, CUtensorMap> cache;
+  std::lock_guard<std::mutex> lock(mu);
+  auto key = std::make_tuple(w, rows, box_rows);
+  auto it = cache.find(key);
+  if (it != cache.end()) { *out = it->second; return 0; }
+  const int rc = tc_encode_map(w, kTcK, rows, kTcK, box_rows, out);
+  if (rc) return rc;
   if (cache.size() > 4096) cache.clear();
-  cache[key] = m;
-  *out = m;
+  cache[key] = *out;
   return 0;
 }
 
@@ -1429,20 +1437,56 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
     if (block_size & (block_size - 1)) return DFB_E_GEOMETRY;   // blocks of a power of two tokens (the reference's are 256)
     while ((1 << block_shift) < block_size) ++block_shift;
   }
-  const void* fn = block_tables ? (const void*)prefill_attention_kernel<true> : (const void*)prefill_attention_kernel<false>;
-  cudaError_t e = ensure_dynamic_smem(fn, kPfSmemBytes);
+  // Short prompts (whose lengths max_seqlen_q bounds on the host) stay on the mma.sync kernel: its 64-row CTAs
+  // start and finish sooner.  Measured, it is the faster one up to 384 tokens while its CTAs all have an SM of their
+  // own (one prompt of 384: 12.3 us against 12.7), and up to 128 tokens while they are resident together, three
+  // per SM (16 prompts of 64: 6.7 against 9.3 us; 16 of 128 no longer: 13.3 against 9.6).
+  const int64_t short_ctas = (int64_t)batch * ((max_seqlen_q + kPfTile - 1) / kPfTile) * q_heads;
+  const int sms = sm_count_cached();
+  if (!block_tables && max_seqlen_q <= (short_ctas <= sms ? 384 : 128) && short_ctas <= 3 * sms) {
+    const void* fn = (const void*)prefill_short_kernel;
+    cudaError_t e = ensure_dynamic_smem(fn, kPfShortSmemBytes);
+    if (e != cudaSuccess) return (int)e;
+    prefer_carveout(fn, 100);
+    PrefillShortArgs s = {};
+    s.q = (const bf16*)q; s.k = (const bf16*)k; s.v = (const bf16*)v; s.out = (bf16*)out;
+    s.cu_seqlens = cu_seqlens_q; s.cu_seqlens_k = cu_seqlens_k ? cu_seqlens_k : cu_seqlens_q;
+    s.q_stride = q_stride; s.k_stride = k_stride; s.v_stride = v_stride; s.out_stride = out_stride;
+    s.q_heads = q_heads; s.kv_heads = kv_heads; s.scale = scale;
+    const dim3 grid((max_seqlen_q + kPfTile - 1) / kPfTile, q_heads, batch);
+    prefill_short_kernel<<<grid, 128, kPfShortSmemBytes, (cudaStream_t)stream>>>(s);
+    DFB_CUDA(cudaGetLastError());
+    return 0;
+  }
+  // query heads that share a KV head go in pairs where their number allows it
+  const bool pairs = (q_heads / kv_heads) % 2 == 0;
+  auto kernel = block_tables ? (pairs ? prefill_tc_kernel<true, true> : prefill_tc_kernel<true, false>)
+                             : (pairs ? prefill_tc_kernel<false, true> : prefill_tc_kernel<false, false>);
+  cudaError_t e = ensure_dynamic_smem((const void*)kernel, kPfSmemBytes);
   if (e != cudaSuccess) return (int)e;
-  prefer_carveout(fn, 100);   // two CTAs of 68 KB per SM (registers allow no more)
   PrefillArgs a = {};
   a.q = (const bf16*)q; a.k = (const bf16*)k; a.v = (const bf16*)v; a.out = (bf16*)out;
   a.cu_seqlens = cu_seqlens_q; a.cu_seqlens_k = cu_seqlens_k ? cu_seqlens_k : cu_seqlens_q;
   a.block_tables = block_tables; a.bt_stride = block_table_stride; a.block_size = block_size; a.num_blocks = num_blocks;
   a.block_shift = block_shift;
   a.q_stride = q_stride; a.k_stride = k_stride; a.v_stride = v_stride; a.out_stride = out_stride;
-  a.q_heads = q_heads; a.kv_heads = kv_heads; a.scale = scale; a.status = status;
-  const dim3 grid((max_seqlen_q + kPfTile - 1) / kPfTile, q_heads, batch);
-  if (block_tables) prefill_attention_kernel<true><<<grid, 128, kPfSmemBytes, (cudaStream_t)stream>>>(a);
-  else prefill_attention_kernel<false><<<grid, 128, kPfSmemBytes, (cudaStream_t)stream>>>(a);
+  a.batch = batch; a.q_heads = q_heads; a.kv_heads = kv_heads; a.scale = scale; a.status = status;
+  // The maps' row counts only have to cover the boxes the kernel asks for, all of them inside a sequence (or a
+  // block of the cache); how many tokens there are is known on the device alone.
+  a.box_rows = block_tables && block_size < kPfKeys ? block_size : kPfKeys;
+  const int64_t any_rows = (int64_t)1 << 31;
+  int rc = tc_encode_map(q, (int64_t)q_heads * head_dim, any_rows, q_stride, kPfRows, &a.q_map);
+  if (!rc) rc = tc_encode_map(k, (int64_t)kv_heads * head_dim, any_rows, k_stride, a.box_rows, &a.k_map);
+  if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, any_rows, v_stride, a.box_rows, &a.v_map);
+  if (!rc) rc = tc_encode_map(q, (int64_t)q_heads * head_dim, any_rows, q_stride, 8, &a.q_map8);
+  if (!rc) rc = tc_encode_map(k, (int64_t)kv_heads * head_dim, any_rows, k_stride, 8, &a.k_map8);
+  if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, any_rows, v_stride, 8, &a.v_map8);
+  if (rc) return rc;
+  // one CTA per SM (all of its tensor memory), fewer when the longest sequence bounds the work items below that
+  const int64_t rows = pairs ? kPfRows : 2 * kPfRows;
+  const int64_t most = (int64_t)batch * ((max_seqlen_q + rows - 1) / rows) * (pairs ? q_heads / 2 : q_heads);
+  const int grid = (int)(most < sm_count_cached() ? most : sm_count_cached());
+  kernel<<<grid, kPfThreads, kPfSmemBytes, (cudaStream_t)stream>>>(a);
   DFB_CUDA(cudaGetLastError());
   return 0;
 }

@@ -1,9 +1,6 @@
-// Causal prefill attention over the prompt tokens of a batch of sequences: the step on the other side of the
-// shared paged cache.  The reference calls FlashAttention for it (flash_attn_varlen_func with causal = True,
-// layers/attention.py:64-70); this is the same computation, written against the tensor cores with mma.sync, for
-// both of its cases: without a prefix cache K / V are the fresh projections of the same tokens; with one they
-// are read back from the paged cache through the block tables, the sequence's keys outnumber its queries, and
-// query i attends to keys 0 .. i + (keys - queries) (the causal mask aligned to the last key, as FlashAttention):
+// Causal prefill attention over short prompts: the computation of dfb_prefilltc.cuh (flash_attn_varlen_func with
+// causal = True, layers/attention.py:64-70) on mma.sync, for launches that are over before a tcgen05 kernel
+// has filled its pipeline (one prompt of 128 tokens: 5.8 us against 8.6 us; of 512 tokens: 15.7 against 14.5):
 //
 //   * q [N, q_heads, 128], k / v [N, kv_heads, 128] bf16, tokens of all sequences back to back, sequence b =
 //     rows [cu_seqlens[b], cu_seqlens[b + 1]); grouped-query attention (q head h reads KV head
@@ -19,8 +16,7 @@
 //     shared memory); V fragments by ldmatrix.trans; O in fp32 registers, divided by the row sum at the end.
 //
 // P is rounded to bf16 before it multiplies V, as FlashAttention does.  mma.sync issues about once per 38 cycles
-// per SM sub-partition on this part, which bounds this kernel far below the tcgen05 peak: it is the functional
-// counterpart of the reference's prefill attention on the shared cache layout, not a roofline kernel.
+// per SM sub-partition on this part, which bounds this kernel far below the tcgen05 peak on anything longer.
 #pragma once
 
 #include "dfb_kernels.cuh"
@@ -29,25 +25,19 @@ namespace dfb {
 
 constexpr int kPfTile = 64;                      // query rows per CTA and KV positions per tile
 constexpr int kPfRowBytes = kHeadDim * 2 + 16;   // padded shared-memory row of a K / V tile
-constexpr int kPfTileBytes = kPfTile * kPfRowBytes;
-constexpr int kPfSmemBytes = 4 * kPfTileBytes;   // K and V, two buffers each
-constexpr int kKernelPrefill = 9;
+constexpr int kPfPaddedTileBytes = kPfTile * kPfRowBytes;
+constexpr int kPfShortSmemBytes = 4 * kPfPaddedTileBytes;   // K and V, two buffers each
 
-struct PrefillArgs {
+struct PrefillShortArgs {
   const __nv_bfloat16* q;
   const __nv_bfloat16* k;
   const __nv_bfloat16* v;
   __nv_bfloat16* out;
   const int* cu_seqlens;        // [batch + 1] query rows
-  const int* cu_seqlens_k;      // [batch + 1] keys; equal to cu_seqlens without a prefix cache
-  const int* block_tables;      // null: k / v hold the keys of sequence b at rows cu_seqlens_k[b] ...; else
-                                // [batch, bt_stride] physical blocks and k / v are one layer's cache
-                                // [num_blocks, block_size] rows
-  int bt_stride, block_size, block_shift, num_blocks;   // block_size = 1 << block_shift
-  long long q_stride, k_stride, v_stride, out_stride;   // elements between token rows (cache: between slots)
+  const int* cu_seqlens_k;      // [batch + 1] keys, at the same rows of k / v as the queries' by default
+  long long q_stride, k_stride, v_stride, out_stride;   // elements between token rows
   int q_heads, kv_heads;
   float scale;
-  int* status;                  // optional device status word (a block id outside the cache)
 };
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
@@ -68,10 +58,7 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* 
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(s) : "memory");
 }
 
-// PAGED: keys come from the paged cache through the block tables (block_size a power of two: the position's
-// block and offset are a shift and a mask); else they are rows of k / v, and the copy loop has no table walk.
-template <bool PAGED>
-__global__ void __launch_bounds__(128) prefill_attention_kernel(const PrefillArgs a) {
+__global__ void __launch_bounds__(128) prefill_short_kernel(const PrefillShortArgs a) {
   extern __shared__ __align__(128) unsigned char pf_smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -85,8 +72,8 @@ __global__ void __launch_bounds__(128) prefill_attention_kernel(const PrefillArg
   const int q_hi = min(q0 + kPfTile, seq_len);    // one past the CTA's last query row
   const int n_tiles = (shift + q_hi + kPfTile - 1) / kPfTile;   // causal: key positions [0, shift + q_hi)
 
-  auto k_tile = [&](int buf) { return pf_smem + buf * kPfTileBytes; };
-  auto v_tile = [&](int buf) { return pf_smem + (2 + buf) * kPfTileBytes; };
+  auto k_tile = [&](int buf) { return pf_smem + buf * kPfPaddedTileBytes; };
+  auto v_tile = [&](int buf) { return pf_smem + (2 + buf) * kPfPaddedTileBytes; };
   // every thread copies 8 + 8 pieces of 16 bytes per tile (64 rows x 16 pieces for K, the same for V); rows
   // beyond the sequence are filled with zeros so that no stale bits (a NaN pattern) ever meet a zero probability
   auto load_tile = [&](int tile, int buf) {
@@ -97,19 +84,10 @@ __global__ void __launch_bounds__(128) prefill_attention_kernel(const PrefillArg
       unsigned char* kd = k_tile(buf) + row * kPfRowBytes + 16 * piece;
       unsigned char* vd = v_tile(buf) + row * kPfRowBytes + 16 * piece;
       const int p = p0 + row;
-      long long tok = -1;                          // row of k / v that holds key p, or none
       if (p < k_len) {
-        if (PAGED) {
-          const int block = a.block_tables[(size_t)seq * a.bt_stride + (p >> a.block_shift)];
-          if (block >= 0 && block < a.num_blocks) tok = ((long long)block << a.block_shift) + (p & (a.block_size - 1));
-          else if (piece == 0) report_status(a.status, kStatusBadBlock, kKernelPrefill, seq, block);   // row read as zeros
-        } else {
-          tok = k_start + p;
-        }
-      }
-      if (tok >= 0) {
-        cp_async16(kd, a.k + (size_t)tok * a.k_stride + (size_t)kvh * kHeadDim + 8 * piece);
-        cp_async16(vd, a.v + (size_t)tok * a.v_stride + (size_t)kvh * kHeadDim + 8 * piece);
+        const size_t tok = (size_t)(k_start + p);
+        cp_async16(kd, a.k + tok * a.k_stride + (size_t)kvh * kHeadDim + 8 * piece);
+        cp_async16(vd, a.v + tok * a.v_stride + (size_t)kvh * kHeadDim + 8 * piece);
       } else {
         *reinterpret_cast<uint4*>(kd) = make_uint4(0, 0, 0, 0);
         *reinterpret_cast<uint4*>(vd) = make_uint4(0, 0, 0, 0);

@@ -1,0 +1,69 @@
+"""The tcgen05 prefill attention kernel at its edges (64-key tiles, 128-row query tiles, both query-head ratios,
+cache blocks smaller than a tile, maxima that grow along the sequence) and the line between it and the kernel for
+short prompts, against the fp32 computation."""
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+BF = torch.bfloat16
+
+
+def _reference(q, k, v, q_len, k_len, scale):
+    """fp32 causal attention of one sequence whose last q_len of k_len positions are the queries."""
+    rep = q.shape[1] // k.shape[1]
+    s = torch.einsum("qhd,khd->hqk", q.float(), k.float().repeat_interleave(rep, 1)) * scale
+    hidden = torch.arange(k_len)[None, :] > torch.arange(q_len)[:, None] + (k_len - q_len)
+    s = s.masked_fill(hidden, float("-inf"))
+    return torch.einsum("hqk,khd->qhd", torch.softmax(s, -1), v.float().repeat_interleave(rep, 1))
+
+
+@pytest.mark.parametrize("q_heads,kv_heads", [(16, 8), (8, 8), (12, 4)])
+@pytest.mark.parametrize("lens,growing", [((384, 385), False), ((129, 127, 64, 65, 511, 1, 128), False), ((640, 2048), True),
+                                          ((1,) * 40 + (257,), False)])
+def test_fresh_prompts(cuda_device, q_heads, kv_heads, lens, growing):
+    from dfb_b200.kv_store import prefill_attention
+
+    rng = np.random.Generator(np.random.Philox(key=sum(lens) + q_heads))
+    n, d = sum(lens), 128
+    q, k, v = (torch.from_numpy(rng.standard_normal((n, h, d), dtype=np.float32)) for h in (q_heads, kv_heads, kv_heads))
+    if growing:      # later keys score higher, so that the running maximum of a row has to be raised again and again
+        k *= torch.cat([1 + torch.arange(m) / 60.0 for m in lens])[:, None, None]
+    q, k, v = q.to(BF), k.to(BF), v.to(BF)
+    cu = torch.tensor(np.cumsum([0, *lens]), dtype=torch.int32, device="cuda")
+    got = prefill_attention(q.cuda(), k.cuda(), v.cuda(), cu, max(lens), d ** -0.5).float().cpu()
+    start = 0
+    for m in lens:
+        want = _reference(q[start:start + m], k[start:start + m], v[start:start + m], m, m, d ** -0.5)
+        assert float((got[start:start + m] - want).abs().max()) <= (2.0 ** -5 if growing else 2.0 ** -6), m
+        start += m
+
+
+@pytest.mark.parametrize("block_size", [4, 16, 64, 256])
+@pytest.mark.parametrize("q_heads,kv_heads", [(16, 8), (8, 8)])
+def test_prefix_cache_block_sizes(cuda_device, block_size, q_heads, kv_heads):
+    from dfb_b200.kv_store import prefill_attention
+
+    rng = np.random.Generator(np.random.Philox(key=block_size + q_heads))
+    case, d = ((300, 44), (128, 128), (65, 1), (500, 333)), 128
+    need = [-(-k // block_size) for k, _ in case]
+    pool = rng.permutation(sum(need) + 2).tolist()
+    kc, vc = (torch.from_numpy(rng.standard_normal((sum(need) + 2, block_size, kv_heads, d), dtype=np.float32)).to(BF)
+              for _ in range(2))
+    tables = [[pool.pop() for _ in range(m)] for m in need]
+    q = torch.from_numpy(rng.standard_normal((sum(m for _, m in case), q_heads, d), dtype=np.float32)).to(BF)
+    # what lies behind the end of a sequence in its last block never counts
+    for (k_len, _), t in zip(case, tables):
+        if k_len % block_size:
+            vc[t[-1], k_len % block_size:] = float("nan")
+    cu_q, cu_k = (torch.tensor(np.cumsum([0, *x]), dtype=torch.int32, device="cuda") for x in ([c[1] for c in case], [c[0] for c in case]))
+    bt = torch.tensor([t + [0] * (max(need) - len(t)) for t in tables], dtype=torch.int32, device="cuda")
+    got = prefill_attention(q.cuda(), kc.cuda(), vc.cuda(), cu_q, max(c[1] for c in case), d ** -0.5, cu_seqlens_k=cu_k,
+                            block_table=bt).float().cpu()
+    start = 0
+    for (k_len, q_len), t in zip(case, tables):
+        k, v = kc[t].flatten(0, 1)[:k_len], vc[t].flatten(0, 1)[:k_len]
+        want = _reference(q[start:start + q_len], k, v, q_len, k_len, d ** -0.5)
+        assert float((got[start:start + q_len] - want).abs().max()) <= 2.0 ** -6, (k_len, q_len)
+        start += q_len
