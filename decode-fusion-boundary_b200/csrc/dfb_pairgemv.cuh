@@ -14,14 +14,15 @@
 //     reads 16 bytes of rows g and g+8 per 32-column block (A fragments of two
 //     MMAs, conflict-free thanks to the padding) and the matching 16 bytes of
 //     x[batch g] (B fragments) from a bf16 copy of x in shared memory;
-//   * the residual add + RMSNorm is done ONE WARP PER BATCH ROW: the rows of h
-//     and of the residual arrive by bulk copies (TMA), a lane owns four 16-byte
-//     pieces of its row, the sum of squares needs one butterfly and no
-//     cross-warp step, every lane computes one root, and the normalised row is
-//     written in place; the eight rows proceed in parallel without a barrier
-//     between them (with every thread handling all rows, the cross-warp
-//     reduction and eight roots per thread made this prologue the longest part
-//     of the kernel after its dependency);
+//   * the residual add + RMSNorm is done ONE WARP PER BATCH ROW: a lane loads
+//     four 16-byte pieces of its row of h and of the residual straight into
+//     registers, the sum of squares needs one butterfly and no cross-warp step,
+//     every lane computes one root; the eight rows proceed in parallel without a
+//     barrier between them.  Plain loads, because in this chain the weights come
+//     by bulk copies and the load / store unit is idle: fetching the rows by bulk
+//     copies into shared memory took 0.7 us more until x was ready, in each of
+//     the 57 launches of a step (4 rows x 500 tokens: 620 -> 592 us per step, 8 x
+//     576: 737 -> 702);
 //   * cross-warp reduction in shared memory, one thread per output for the
 //     epilogue (store / SwiGLU / logits + greedy argmax);
 //   * PSTAGES = 0 keeps the weights in REGISTERS instead of shared-memory
@@ -29,7 +30,7 @@
 //     have read from the stage straight from global memory (eight 128-bit
 //     loads per tile, requested before the dependency wait; the next tile's
 //     once the MMAs have consumed them).  The CTA then holds 33 KB of shared
-//     memory instead of 101-135 KB, so that it fits on an SM beside its
+//     memory instead of 85-119 KB, so that it fits on an SM beside its
 //     predecessor's CTAs and its weights stream while that kernel still runs,
 //     as in the FP32 chain.
 #pragma once
@@ -44,8 +45,7 @@ struct PairSmem {
   static constexpr int kRowStride = 2 * kK + 64;       // bytes
   static constexpr int kStageBytes = 16 * kRowStride;  // 33,792
   static constexpr int kXBytes = kMaxRows * kRowStride; // bf16 copy of x, same padding
-  static constexpr int kResBytes = kMaxRows * 2 * kK;   // residual rows as fetched by the bulk copies
-  static constexpr int bytes(int stages) { return stages * kStageBytes + kXBytes + kResBytes + 8 * (stages + 1) + 16; }
+  static constexpr int bytes(int stages) { return stages * kStageBytes + kXBytes + 8 * stages + 16; }
 };
 
 template <int PSTAGES, int MODE>
@@ -61,9 +61,7 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   unsigned char* stage_base = dyn_smem;
   unsigned char* xsb = dyn_smem + PSTAGES * SM::kStageBytes;                 // [8][kRowStride] bf16 x
-  unsigned char* rstage = xsb + SM::kXBytes;                                 // [8][2 K] residual rows
-  uint64_t* full = reinterpret_cast<uint64_t*>(rstage + SM::kResBytes);
-  uint64_t* x_in = full + PSTAGES;
+  uint64_t* full = reinterpret_cast<uint64_t*>(xsb + SM::kXBytes);
   __shared__ float red[2][kWarps][128];
   __shared__ float ssq[kWarps][kMaxRows];
   __shared__ ArgmaxPart wpart[4][kMaxRows];
@@ -102,10 +100,7 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
     if (lane == 0) {
 #pragma unroll
       for (int s = 0; s < PSTAGES; ++s) mbar_init(&full[s], 1);
-      mbar_init(x_in, 1);
       fence_mbar_init();
-      // the activation rows' byte count is posted here, long before any of their copies can complete
-      if (kNorm && a.ids == nullptr && a.res_in != nullptr && a.tp_mode != 2) mbar_expect_tx(x_in, (uint32_t)(a.rows * 4 * K));
     }
     __syncwarp();
 #pragma unroll
@@ -126,31 +121,26 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
   if (threadIdx.x == 0) { trace_max(a.trace, 1); trace_min(a.trace, 3); }
 
   // ---- x (bf16) into shared memory, with the fused residual add + RMSNorm ----
-  const bool bulk_x = kNorm && a.ids == nullptr && a.res_in != nullptr && a.tp_mode != 2;
-  if (kNorm && bulk_x) {
+  const bool row_per_warp = kNorm && a.ids == nullptr && a.res_in != nullptr && a.tp_mode != 2;
+  if (kNorm && row_per_warp) {
     // warp b owns batch row b; lane l owns the 16-byte pieces l, l + 32, l + 64, l + 96 of the row
-    if (tid < 16) {                       // sixteen threads issue one row copy each
-      const int b = tid & 7;
-      if (b < a.rows) {
-        if (tid < 8) bulk_g2s(xsb + b * SM::kRowStride, a.x + (size_t)b * K, 2 * K, x_in);
-        else bulk_g2s(rstage + b * 2 * K, a.res_in + (size_t)b * K, 2 * K, x_in);
-      }
-    }
-    if (!__syncthreads_and(mbar_wait_bounded(x_in, 0) ? 1 : 0))
-      report_status(a.status, kStatusCopyTimeout, kKernelGemv, blockIdx.x, -1);
     if (a.late_trigger) pdl_launch_dependents();
     const int b = warp;
     unsigned char* xrow = xsb + b * SM::kRowStride;
     if (b < a.rows) {
+      uint4 hv[4], rv[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        hv[c] = ldg_cg(a.x + (size_t)b * K + 8 * (32 * c + lane));
+        rv[c] = ldg_cg(a.res_in + (size_t)b * K + 8 * (32 * c + lane));
+      }
       float x[4][8];
       float ss = 0.f;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        const uint4 hv = *reinterpret_cast<const uint4*>(xrow + 16 * (32 * c + lane));
-        const uint4 rv = *reinterpret_cast<const uint4*>(rstage + b * 2 * K + 16 * (32 * c + lane));
         float hf[8], rf[8];
-        unpack8(hv, hf);
-        unpack8(rv, rf);
+        unpack8(hv[c], hf);
+        unpack8(rv[c], rf);
 #pragma unroll
         for (int e = 0; e < 8; ++e) { x[c][e] = hf[e] + rf[e]; ss = fmaf(x[c][e], x[c][e], ss); }
       }

@@ -26,9 +26,9 @@
 // (one elected thread each) take every fourth stage: 4 MMAs per stage (K = 16
 // each) into the issuer's own accumulator, a commit to the stage's "empty"
 // barrier and, after the issuer's last stage of the tile, to the accumulators'
-// "full" barrier.  Eight prologue warps build the B operand: the rows of h and
-// of the residual arrive by bulk copies (TMA), then add + RMSNorm, bf16,
-// written in the swizzled K-major layout.  Four of them go on as the epilogue:
+// "full" barrier.  Eight prologue warps build the B operand, one batch row each:
+// plain loads of h and of the residual, add + RMSNorm, bf16, written in the
+// swizzled K-major layout.  Four of them go on as the epilogue:
 // they read the accumulators with tcgen05.ld, add the issuers' accumulators and
 // the two diagonal blocks (the latter through shared memory), round once to
 // bf16 and run the epilogue.  Two accumulator buffers let the MMAs of the next
@@ -69,10 +69,9 @@ struct TcSmem {
   static constexpr int kStages = kTcKbPairs;                     // the ring holds exactly one tile
   static constexpr int kStageBytes = MT * 128;
   static constexpr int kXBytes = kTcKbPairs * 2048;              // B operand: 8 x [16 rows x 128 B]
-  static constexpr int kResBytes = kMaxRows * kTcK * 2;          // residual rows as fetched by the bulk copies
   static constexpr int kRedBytes = 2 * 2 * kMaxRows * (MT / 2) * 4;   // [buffer][half][batch][row] fp32
   static constexpr int kBarBytes = 8 * (2 * kStages + 6) + 64;
-  static constexpr int bytes() { return 1024 + kStages * kStageBytes + kXBytes + kResBytes + kRedBytes + kBarBytes + 256; }
+  static constexpr int bytes() { return 1024 + kStages * kStageBytes + kXBytes + kRedBytes + kBarBytes + 256; }
 };
 
 // ---- small PTX wrappers ----------------------------------------------------------------------------------
@@ -181,16 +180,14 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemv_kernel(const __grid_con
   const uint32_t raw = smem_u32(tc_dyn_raw);
   unsigned char* dyn = tc_dyn_raw + (((raw + 1023u) & ~1023u) - raw);    // the swizzle pattern repeats every 1024 bytes
   unsigned char* stages = dyn;
-  unsigned char* xs = dyn + STAGES * SM::kStageBytes;                    // h rows as fetched, then the B operand
-  unsigned char* rstage = xs + SM::kXBytes;                              // residual rows as fetched
-  float* red = reinterpret_cast<float*>(rstage + SM::kResBytes);         // [2][2][8][R]
-  uint64_t* full = reinterpret_cast<uint64_t*>(rstage + SM::kResBytes + SM::kRedBytes);
+  unsigned char* xs = dyn + STAGES * SM::kStageBytes;                    // the B operand
+  float* red = reinterpret_cast<float*>(xs + SM::kXBytes);               // [2][2][8][R]
+  uint64_t* full = reinterpret_cast<uint64_t*>(xs + SM::kXBytes + SM::kRedBytes);
   uint64_t* empty = full + STAGES;
   uint64_t* acc_full = empty + STAGES;
   uint64_t* acc_empty = acc_full + 2;
   uint64_t* x_ready = acc_empty + 2;
-  uint64_t* x_in = x_ready + 1;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(x_in + 1);
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(x_ready + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   int* last_flag = const_cast<int*>(abort_flag) + 1;
 
@@ -203,7 +200,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemv_kernel(const __grid_con
     mbar_init(&acc_full[0], kTcIssuers); mbar_init(&acc_full[1], kTcIssuers);
     mbar_init(&acc_empty[0], 128); mbar_init(&acc_empty[1], 128);
     mbar_init(x_ready, kTcProThreads);
-    mbar_init(x_in, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -294,22 +290,8 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemv_kernel(const __grid_con
     uint4 nw4[4];   // the norm weights of this lane's four 16-byte pieces (pieces lane, lane + 32, + 64, + 96 of a row)
 #pragma unroll
     for (int c = 0; c < 4; ++c) nw4[c] = ldg_stream(a.norm_w + 8 * (32 * c + lane));
-    // The rows of h and of the residual come in by bulk copies (TMA): ordinary loads issued here would
-    // queue in the load/store unit behind the loads of the successor kernel that was let in early.
-    const bool bulk_x = a.ids == nullptr && a.res_in != nullptr;
-    if (bulk_x && pt == 0) mbar_expect_tx(x_in, (uint32_t)(a.rows * 2 * kTcK * 2));
-    named_sync(1, kTcProThreads);      // the byte count is posted before any copy can complete
     pdl_wait();
     if (pt == 0) { trace_max(a.trace, 1); trace_min(a.trace, 3); }
-    if (bulk_x && pt < 16) {
-      // sixteen threads issue one row copy each (one thread issuing all of them is slower than the copies)
-      const int b = pt & 7;
-      if (b < a.rows) {
-        if (pt < 8) bulk_g2s(xs + b * 2 * kTcK, a.x + (size_t)b * kTcK, 2 * kTcK, x_in);
-        else bulk_g2s(rstage + b * 2 * kTcK, a.res_in + (size_t)b * kTcK, 2 * kTcK, x_in);
-      }
-    }
-
     // x = h (+ residual), bf16 residual out, RMSNorm, bf16 y in the swizzled layout of the B operand.
     // Warp b owns batch row b: a lane holds four 16-byte pieces of the row, the sum of squares needs one
     // butterfly and no cross-warp step, every lane computes one root; the eight rows proceed in parallel.
@@ -318,19 +300,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemv_kernel(const __grid_con
       uint4 hv[4], rv[4];
 #pragma unroll
       for (int c = 0; c < 4; ++c) { hv[c] = make_uint4(0, 0, 0, 0); rv[c] = make_uint4(0, 0, 0, 0); }
-      if (bulk_x) {
-        if (!named_sync_and(1, kTcProThreads, tc_wait(x_in, 0, abort_flag))) {
-          if (pt == 0 && !*abort_flag) report_status(a.status, kStatusCopyTimeout, kKernelTcGemv, blockIdx.x, 4);
-          *abort_flag = 1;
-        }
-        if (b < a.rows) {
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            hv[c] = *reinterpret_cast<const uint4*>(xs + b * 2 * kTcK + 16 * (32 * c + lane));
-            rv[c] = *reinterpret_cast<const uint4*>(rstage + b * 2 * kTcK + 16 * (32 * c + lane));
-          }
-        }
-      } else if (b < a.rows) {
+      if (b < a.rows) {
         const size_t xrow = a.ids ? (size_t)clamp_token(a.ids[b], a.embed_rows, a.status, b) : (size_t)b;
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
@@ -339,7 +309,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemv_kernel(const __grid_con
         }
       }
       if (a.late_trigger) pdl_launch_dependents();   // the successor's prefetch traffic starts after x is here
-      named_sync(1, kTcProThreads);    // every row has been read before any y is written over the staging bytes
       float x[4][8];
       float ss = 0.f;
 #pragma unroll
