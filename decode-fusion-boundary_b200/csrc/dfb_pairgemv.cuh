@@ -23,6 +23,9 @@
 //     copies into shared memory took 0.7 us more until x was ready, in each of
 //     the 57 launches of a step (4 rows x 500 tokens: 620 -> 592 us per step, 8 x
 //     576: 737 -> 702);
+//   * a per-layer projection whose tiles all fit the stages runs their MMAs one
+//     after the other and has ONE barrier and ONE epilogue for all of them (8 x
+//     576: 702 -> 686 us per step);
 //   * cross-warp reduction in shared memory, one thread per output for the
 //     epilogue (store / SwiGLU / logits + greedy argmax);
 //   * PSTAGES = 0 keeps the weights in REGISTERS instead of shared-memory
@@ -62,7 +65,9 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
   unsigned char* stage_base = dyn_smem;
   unsigned char* xsb = dyn_smem + PSTAGES * SM::kStageBytes;                 // [8][kRowStride] bf16 x
   uint64_t* full = reinterpret_cast<uint64_t*>(xsb + SM::kXBytes);
-  __shared__ float red[2][kWarps][128];
+  // the per-layer projections: partial sums of all of the CTA's tiles, one barrier and one epilogue for them
+  constexpr bool kAllTiles = !kReg && MODE != kModeNormArgmax;
+  __shared__ float red[kAllTiles ? PSTAGES : 2][kWarps][128];
   __shared__ float ssq[kWarps][kMaxRows];
   __shared__ ArgmaxPart wpart[4][kMaxRows];
   __shared__ int last_flag;
@@ -266,6 +271,50 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
   if (MODE == kModeNormArgmax) sample_rows_load(a, srows, tid);   // a CTA barrier follows before the first epilogue
   int it = 0;
   bool copy_ok = true;
+  if (kAllTiles && a.n_tiles <= PSTAGES * stride) {
+    int nt = 0;
+#pragma unroll
+    for (int s = 0; s < PSTAGES; ++s) {
+      if ((int)blockIdx.x + s * stride >= a.n_tiles) break;
+      if (!mbar_wait_bounded(&full[s], 0)) copy_ok = false;
+      const unsigned char* w0p = stage_base + s * SM::kStageBytes + g * SM::kRowStride + 2 * kbase;
+      const unsigned char* w1p = w0p + 8 * SM::kRowStride;
+      float c[4][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { c[q][0] = 0.f; c[q][1] = 0.f; c[q][2] = 0.f; c[q][3] = 0.f; }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const uint4 u = *reinterpret_cast<const uint4*>(w0p + 64 * j);   // row g
+        const uint4 v = *reinterpret_cast<const uint4*>(w1p + 64 * j);   // row g + 8
+        mma_bf16_16816_full(c[(2 * j) & 3], u.x, v.x, u.y, v.y, xa[j].x, xa[j].y);
+        mma_bf16_16816_full(c[(2 * j + 1) & 3], u.z, v.z, u.w, v.w, xa[j].z, xa[j].w);
+      }
+      float* r = red[s][warp];
+      *reinterpret_cast<float2*>(r + g * 8 + 2 * t) =
+          make_float2((c[0][0] + c[1][0]) + (c[2][0] + c[3][0]), (c[0][1] + c[1][1]) + (c[2][1] + c[3][1]));
+      *reinterpret_cast<float2*>(r + (g + 8) * 8 + 2 * t) =
+          make_float2((c[0][2] + c[1][2]) + (c[2][2] + c[3][2]), (c[0][3] + c[1][3]) + (c[2][3] + c[3][3]));
+      ++nt;
+    }
+    if (threadIdx.x == 0) trace_max(a.trace, 5);
+    __syncthreads();
+    // SwiGLU: 64 outputs per tile, the matching up row 8 rows further; else 128 per tile
+    constexpr int kOut = MODE == kModeNormSwiglu ? 64 : 128;
+    for (int o = tid; o < nt * kOut; o += 256) {
+      const int s = o / kOut, i = o % kOut, b = i & 7, r = i >> 3, tile = blockIdx.x + s * stride;
+      if (b >= a.rows) continue;      // (a division of the absent rows' zeros would take the slow path: 0.35 us)
+      float v = 0.f, u = 0.f;
+#pragma unroll
+      for (int w = 0; w < kWarps; ++w) {
+        v += red[s][w][i];
+        if (MODE == kModeNormSwiglu) u += red[s][w][i + 64];
+      }
+      v = round_bf16(v);
+      if (MODE == kModeNormSwiglu) { u = round_bf16(u); v = v / (1.0f + expf(-v)) * u; }
+      a.out[(size_t)b * a.out_stride + tile * (kOut / 8) + r] = __float2bfloat16_rn(v);
+    }
+    if (threadIdx.x == 0) trace_max(a.trace, 6);
+  } else
   for (int tile = blockIdx.x; tile < a.n_tiles; tile += stride, ++it) {
     const int s = it % kStagesOr1;
     if (!kReg && !mbar_wait_bounded(&full[s], (it / kStagesOr1) & 1)) { copy_ok = false; break; }
