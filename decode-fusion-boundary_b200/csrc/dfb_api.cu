@@ -7,6 +7,7 @@
 #include "dfb_exchange.cuh"
 #include "dfb_pairgemv.cuh"
 #include "dfb_tcgemv.cuh"
+#include "dfb_attncluster.cuh"
 #include "dfb_attnring.cuh"
 #include "dfb_prefilltc.cuh"
 
@@ -83,6 +84,8 @@ struct ChainOptions {
   // counterparts (their longer post-dependency path: bulk copies of x, two issue loops, accumulator read).
   int tcgen05 = env_int("DFB_TCGEN05", 4);
   int carve_tc = 100;          // ... whose chain asks for all of an SM's L1/shared memory as shared memory
+  int attn_auto = 1;           // 1: the cluster attention kernel (dfb_attncluster.cuh) where attention_cluster() says so; 0
+                               // once one of the attention options below has been set: the kernel they select runs
   int attn_cluster = env_int("DFB_ATTN_CLUSTER", 148);  // attention grids of at most this many CTAs (and 2..16 chunks
                                // per row) launch the chunks of one (row, KV head) as a thread-block cluster that
                                // merges its partial results through distributed shared memory instead of global
@@ -406,6 +409,7 @@ int reg_grid(const Launcher& L, int n_tiles) {
 
 constexpr int kRingFlag = 256;   // bit of the split-bucket value that selects the streaming attention kernel
 constexpr int kRing32Flag = 1024;    // ... with kRingFlag: the streaming kernel with 32 positions per CTA
+constexpr int kClusterFlag = 2048;   // ... that selects the cluster attention kernel: 1, 2, 3 x = clusters of 2, 4, 8 CTAs
 constexpr int kChunk128Flag = 512;   // ... that selects 128-position chunks in the register-resident kernel
 
 // ---- kernel launch wrappers -------------------------------------------------
@@ -728,7 +732,7 @@ int launch_attention(Launcher& L, DfbHandle* h, int layer, const bf16* qkv, cons
                      int bt_stride, int bt_cols, const int* row_active, bf16* out, int rows, int nsplit_arg) {
   const bool ring = (nsplit_arg & kRingFlag) != 0;   // set by split_bucket for long contexts
   const bool chunk128 = (nsplit_arg & kChunk128Flag) != 0;   // ... and for small grids
-  const int nsplit = nsplit_arg & (kRingFlag - 1);
+  const int nsplit = nsplit_arg & (kRingFlag - 1);       // 64-position chunks that the context bound covers
   const DfbModelDesc& m = h->m;
   AttnArgs a = {};
   a.qkv = qkv; a.qkv_stride = h->qkv_rows(); a.q_size = h->q_size(); a.kv_size = h->kv_size();
@@ -747,6 +751,14 @@ int launch_attention(Launcher& L, DfbHandle* h, int layer, const bf16* qkv, cons
   // CTAs most SMs are idle during attention: 256 threads then halve each thread's
   // share of the chunk and with it the latency of the CTA.
   const int ctas = nsplit * m.kv_heads * rows;
+  if (nsplit_arg >= kClusterFlag) {
+    a.ctx_limit = nsplit * kAttnChunk;
+    a.late_trigger = L.opt->late_trigger;
+    const int cs = 2 << (nsplit_arg / kClusterFlag - 1);
+    auto kernel = cs == 8 ? cluster_attention_kernel<8> : cs == 4 ? cluster_attention_kernel<4> : cluster_attention_kernel<2>;
+    L.launch(kernel, dim3(cs, m.kv_heads, rows), dim3(kCaThreads), a, true, 0, cs);
+    return L.err;
+  }
   a.late_trigger = L.opt->late_trigger;
   if (ring && m.kv_heads == kRingHeads) {
     // long contexts / full batches: one CTA per (row, chunk) for all KV heads, K/V streamed through shared memory
@@ -792,6 +804,24 @@ int launch_attention(Launcher& L, DfbHandle* h, int layer, const bf16* qkv, cons
   return L.err;
 }
 
+// CTAs per (row, KV head) of the cluster attention kernel for a step of `rows` rows with contexts up to `chunks` x 64
+// tokens, or 0 where the chunked kernels are the faster ones.  Measured for 1 to 8 rows x 64 to 2,000 tokens: it wins
+//   * when 128 positions per CTA, what a CTA holds in flight, cover the context and the grid is large enough for the
+//     chunked kernel's many small CTAs to start late (8 rows x 192 tokens: 573 against 611 us a step; 3 rows x 512: 570
+//     against 592; 2 rows x 512 not: 561 against 547);
+//   * when there is enough to stream: from 80 chunks on (8 rows x 1,024: 720 against 813 us; 5 rows x 1,024: 698 against
+//     737; 4 rows x 1,280: 708 against 732).  Below that (6 rows x 768: 692 against 651) its second, nearly empty pass
+//     costs more than the chunked kernel's merge.
+// All CTAs have to be resident together, two per SM; 16-CTA clusters wait too long for sixteen free places at a time
+// (2 rows x 905 tokens: 8 us until the last one started).
+int attention_cluster(int rows, int chunks) {
+  if (chunks >= 3 && chunks <= 8) {
+    const int cs = chunks <= 4 ? 2 : 4;
+    return rows * cs >= 10 ? cs : 0;
+  }
+  return rows * chunks >= 80 ? (rows <= 4 ? 8 : 4) : 0;
+}
+
 // Grid of the attention kernel for a context bound: the number of 64-position chunks rounded up to a power
 // of two (one captured graph per bucket), plus kRingFlag when rows x chunks is large enough for the streaming
 // kernel to keep about two CTAs per SM busy.
@@ -799,6 +829,12 @@ int split_bucket(const DfbHandle* h, int max_context, int rows) {
   if (max_context < 1) max_context = 1;
   if (max_context > h->m.max_model_len) max_context = h->m.max_model_len;
   int need = (max_context + kAttnChunk - 1) / kAttnChunk;
+  const int cs = h->opt.attn_auto && h->m.kv_heads == kRingHeads ? attention_cluster(rows, need) : 0;
+  if (cs) {
+    int b = 1;
+    while (b < need) b <<= 1;
+    return (b > kMaxSplits ? kMaxSplits : b) + kClusterFlag * (cs == 2 ? 1 : cs == 4 ? 2 : 3);
+  }
   const bool ring64 = h->m.kv_heads == kRingHeads && h->opt.attn_ring_min > 0 && rows * need >= h->opt.attn_ring_min;
   // mid-size steps: the streaming kernel with 32 positions per CTA (its partial results fit the 32 slots up to 1024 tokens)
   const int need32 = (max_context + kAttnChunk / 2 - 1) / (kAttnChunk / 2);
@@ -976,7 +1012,7 @@ int enqueue_whole_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const St
 int get_step_graph(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, DfbHandle::StepGraph** out) {
   const bool persistent = h->step_mode == 1;
   const int io_kind = (io.burst ? 0 : io.host ? 3 : (io.out_tokens ? 2 : 1)) + (io.sampling ? 4 : 0);
-  const long long key = ((persistent ? (1ll << 40) : 0ll) + (((long long)bt_cols * 16 + rows) * 4096 + nsplit) * 2 +
+  const long long key = ((persistent ? (1ll << 40) : 0ll) + (((long long)bt_cols * 16 + rows) * 16384 + nsplit) * 2 +
                          (h->use_pdl ? 1 : 0)) * 8 + io_kind;
   auto it = h->graphs.find(key);
   if (it == h->graphs.end()) {
@@ -1287,6 +1323,7 @@ int dfb_set_option(DfbHandle* h, int option, int value) {
     case DFB_OPT_ATTN_WIDE:
       if (value < 0) return DFB_E_BAD_ARG;
       h->opt.attn_wide_ctas = value;
+      h->opt.attn_auto = 0;
       break;
     case DFB_OPT_LOOK_AHEAD:
       if (value < 0 || value > 63) return DFB_E_BAD_ARG;
@@ -1299,6 +1336,7 @@ int dfb_set_option(DfbHandle* h, int option, int value) {
     case DFB_OPT_ATTN_RING:
       if (value < 0) return DFB_E_BAD_ARG;
       h->opt.attn_ring_min = value;
+      h->opt.attn_auto = 0;
       break;
     case DFB_OPT_HOST_IO:
       if (value < 0 || value > 7) return DFB_E_BAD_ARG;
@@ -1311,14 +1349,17 @@ int dfb_set_option(DfbHandle* h, int option, int value) {
     case DFB_OPT_ATTN_RING32:
       if (value < 0) return DFB_E_BAD_ARG;
       h->opt.attn_ring32_min = value;
+      h->opt.attn_auto = 0;
       break;
     case DFB_OPT_ATTN_CHUNK128:
       if (value < 0) return DFB_E_BAD_ARG;
       h->opt.attn_chunk128 = value;
+      h->opt.attn_auto = 0;
       break;
     case DFB_OPT_ATTN_CLUSTER:
       if (value < 0) return DFB_E_BAD_ARG;
       h->opt.attn_cluster = value;
+      h->opt.attn_auto = 0;
       break;
     case DFB_OPT_TCGEN05:
       if (value < 0 || value > 7) return DFB_E_BAD_ARG;

@@ -1,0 +1,27 @@
+"""The cluster attention kernel (``dfb_attncluster.cuh``) at the edges of its pieces and passes: the grids for which the
+decoder picks clusters of 2, 4 and 8 CTAs, contexts around multiples of 16 positions per CTA, of 128 positions per
+pass and of a cache block, rows that leave most CTAs of their cluster without a position, against the fp32 oracle."""
+
+import numpy as np
+import pytest
+import torch
+
+from tests.test_gpu_kernels import _attention_case, small  # noqa: F401  (the fixture)
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("ctx_lens", [
+    (129, 1, 256, 31, 33), (255, 192, 2, 160, 161, 130, 32, 16),                                  # clusters of 2
+    (257, 64, 512), (511, 1, 65, 513 - 64, 320), (512, 257, 17, 63, 449, 384, 400, 511),          # of 4, one pass
+    (1281, 5, 2048, 1024), (2047, 127, 129, 1290),                                                # of 8
+    (2048, 1, 513, 1025, 256, 700, 1536, 2033), (1024, 15, 640, 1000, 897, 3)])                   # of 4, several passes
+@pytest.mark.parametrize("scattered", [False, True])
+def test_cluster_attention(small, ctx_lens, scattered):  # noqa: F811
+    g, w = small
+    perm = np.random.Generator(np.random.Philox(key=19)).permutation(64).tolist() if scattered else None
+    active = [i % 3 != 1 for i in range(len(ctx_lens))] if scattered else None
+    out, want, kv_got, kv_want, _ = _attention_case(g, w, len(ctx_lens), list(ctx_lens), seed=81, perm=perm,
+                                                    row_active=[int(x) for x in active] if active else None)
+    assert float((out.float() - want.float()).abs().max()) <= 2.0 ** -6
+    assert torch.equal(kv_got, kv_want)            # the active rows' new K/V bit-exactly, nothing else touched
