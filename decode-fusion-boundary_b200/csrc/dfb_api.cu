@@ -314,6 +314,10 @@ struct DfbHandle {
   unsigned int* burst_slot = nullptr;   // device
   unsigned int* publish_seq = nullptr;  // device: host-buffer steps published so far (follows the tokens to the host)
   unsigned int published = 0;           // host: the value the next published step will carry
+  // the same for the steps with device inputs and out_tokens (dfb_wait_tokens)
+  int* row_tokens = nullptr;            // pinned: tokens[8] | status[4] | sequence word
+  unsigned int* row_seq = nullptr;      // device
+  unsigned int row_published = 0;       // host
   cudaEvent_t burst_event = nullptr;
   int burst_rows = 0, burst_steps = 0;  // of the burst in flight (0 = none)
   // fixed-slot runtime (dfb_slot_* / dfb_slots_*): host-side state of every slot
@@ -336,7 +340,7 @@ struct DfbHandle {
     cudaGraphExec_t exec = nullptr;
     cudaGraph_t graph = nullptr;            // kept: the node handles below belong to it
     cudaGraphNode_t stage_node = nullptr;   // stage_inputs_kernel (device-input steps)
-    cudaGraphNode_t out_node = nullptr;     // device-to-device copy of tokens + status (device-input steps with out_tokens)
+    cudaGraphNode_t out_node = nullptr;     // publish_result_kernel (device-input steps with out_tokens)
     StageArgs stage_args = {};
     void* out_ptr = nullptr;
   };
@@ -959,6 +963,7 @@ struct StepIo {
   const StageArgs* stage = nullptr;   // device inputs: arguments of stage_inputs_kernel
   bool host = false;                  // host inputs: h->host_stage -> h->stage before, h->tokens -> h->host_tokens after
   int* out_tokens = nullptr;          // device inputs: optional copy of tokens + status
+  bool publish = false;               // ... written by a kernel that publishes them to the host as well (dfb_wait_tokens)
   bool sampling = false;              // the staged temperatures are live: the LM head samples rows with T > 1e-10
   bool burst = false;                 // inputs are already staged on the device; publish_tokens_kernel follows the chain
 };
@@ -989,7 +994,7 @@ int enqueue_whole_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const St
     p.ring = h->burst_ring; p.ring_status = h->burst_status(); p.ring_done = h->burst_done();
     publish_tokens_kernel<<<1, 32, 0, stream>>>(p);
     DFB_CUDA(cudaGetLastError());
-  } else if (io.host && (h->opt.host_io & 2)) {
+  } else if (io.publish || (io.host && (h->opt.host_io & 2))) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1); cfg.blockDim = dim3(32); cfg.stream = stream;
     cudaLaunchAttribute attr[1];
@@ -997,8 +1002,8 @@ int enqueue_whole_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const St
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = (h->use_pdl && !h->sharded()) ? 1 : 0;   // after a collective: an ordinary dependency
-    DFB_CUDA(cudaLaunchKernelEx(&cfg, publish_result_kernel, (const int*)h->tokens, h->host_tokens, kMaxRows + 4,
-                                h->publish_seq));
+    DFB_CUDA(cudaLaunchKernelEx(&cfg, publish_result_kernel, (const int*)h->tokens, io.publish ? h->row_tokens : h->host_tokens,
+                                kMaxRows + 4, io.publish ? h->row_seq : h->publish_seq, io.publish ? io.out_tokens : (int*)nullptr));
   } else if (io.host) {
     DFB_CUDA(cudaMemcpyAsync(h->host_tokens, h->tokens, sizeof(int) * (kMaxRows + 4), cudaMemcpyDeviceToHost, stream));
   } else if (io.out_tokens) {
@@ -1011,9 +1016,9 @@ int enqueue_whole_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const St
 // inputs / outputs); captured and instantiated on first use (or ahead of time by dfb_warm).
 int get_step_graph(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, DfbHandle::StepGraph** out) {
   const bool persistent = h->step_mode == 1;
-  const int io_kind = (io.burst ? 0 : io.host ? 3 : (io.out_tokens ? 2 : 1)) + (io.sampling ? 4 : 0);
+  const int io_kind = (io.burst ? 0 : io.host ? 3 : (io.out_tokens ? 2 : 1)) + (io.sampling ? 4 : 0) + (io.publish ? 8 : 0);
   const long long key = ((persistent ? (1ll << 40) : 0ll) + (((long long)bt_cols * 16 + rows) * 16384 + nsplit) * 2 +
-                         (h->use_pdl ? 1 : 0)) * 8 + io_kind;
+                         (h->use_pdl ? 1 : 0)) * 16 + io_kind;
   auto it = h->graphs.find(key);
   if (it == h->graphs.end()) {
     cudaGraph_t graph = nullptr;
@@ -1033,10 +1038,11 @@ int get_step_graph(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo
         cudaGraphNodeType type;
         e = cudaGraphNodeGetType(nodes[i], &type);
         if (e != cudaSuccess) break;
-        if (type == cudaGraphNodeTypeKernel && !g.stage_node) {
+        if (type == cudaGraphNodeTypeKernel && (!g.stage_node || (io.publish && !g.out_node))) {
           cudaKernelNodeParams kp = {};
           e = cudaGraphKernelNodeGetParams(nodes[i], &kp);
           if (e == cudaSuccess && kp.func == (void*)stage_inputs_kernel) g.stage_node = nodes[i];
+          if (e == cudaSuccess && kp.func == (void*)publish_result_kernel) g.out_node = nodes[i];
         } else if (type == cudaGraphNodeTypeMemcpy && io.out_tokens) {
           g.out_node = nodes[i];
         }
@@ -1071,7 +1077,17 @@ int run_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, 
       DFB_CUDA(cudaGraphExecKernelNodeSetParams(g.exec, g.stage_node, &kp));
       g.stage_args = args;
     }
-    if (io.out_tokens && g.out_ptr != io.out_tokens) {
+    if (io.publish && g.out_ptr != io.out_tokens) {
+      const int* tokens = h->tokens;
+      int n = kMaxRows + 4;
+      int* dev_out = io.out_tokens;
+      void* params[5] = {&tokens, &h->row_tokens, &n, &h->row_seq, &dev_out};
+      cudaKernelNodeParams kp = {};
+      kp.func = (void*)publish_result_kernel;
+      kp.gridDim = dim3(1); kp.blockDim = dim3(32); kp.sharedMemBytes = 0; kp.kernelParams = params; kp.extra = nullptr;
+      DFB_CUDA(cudaGraphExecKernelNodeSetParams(g.exec, g.out_node, &kp));
+      g.out_ptr = io.out_tokens;
+    } else if (io.out_tokens && g.out_ptr != io.out_tokens) {
       DFB_CUDA(cudaGraphExecMemcpyNodeSetParams1D(g.exec, g.out_node, io.out_tokens, h->tokens, sizeof(int) * (kMaxRows + 4),
                                                   cudaMemcpyDeviceToDevice));
       g.out_ptr = io.out_tokens;
@@ -1158,11 +1174,14 @@ int dfb_create(const DfbModelDesc* d, DfbHandle** out) {
   const size_t o_sctr = carve(sizeof(unsigned) * 4);
   const size_t o_bslot = carve(sizeof(unsigned) * 4);
   const size_t o_pseq = carve(sizeof(unsigned) * 4);
+  const size_t o_rseq = carve(sizeof(unsigned) * 4);
   e = cudaMalloc(&h->slab, off);
   if (e == cudaSuccess) e = cudaMemset(h->slab, 0, off);
   if (e == cudaSuccess) e = cudaMallocHost((void**)&h->host_stage, sizeof(int) * h->stage_ints());
   if (e == cudaSuccess) e = cudaMallocHost((void**)&h->host_tokens, sizeof(int) * (kMaxRows + 8));
   if (e == cudaSuccess) h->host_tokens[kMaxRows + 4] = 0;
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&h->row_tokens, sizeof(int) * (kMaxRows + 8));
+  if (e == cudaSuccess) h->row_tokens[kMaxRows + 4] = 0;
   if (e == cudaSuccess) e = cudaMallocHost((void**)&h->burst_ring, sizeof(int) * (kMaxBurst * kMaxRows + 8));
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&h->burst_event, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&h->capture_stream, cudaStreamNonBlocking);
@@ -1191,6 +1210,7 @@ int dfb_create(const DfbModelDesc* d, DfbHandle** out) {
   h->sample_ctr = (unsigned int*)(s + o_sctr);
   h->burst_slot = (unsigned int*)(s + o_bslot);
   h->publish_seq = (unsigned int*)(s + o_pseq);
+  h->row_seq = (unsigned int*)(s + o_rseq);
   *out = h;
   return 0;
 }
@@ -1208,6 +1228,7 @@ void dfb_destroy(DfbHandle* h) {
   if (h->window_local) cudaFree(h->window_local);
   if (h->host_stage) cudaFreeHost(h->host_stage);
   if (h->host_tokens) cudaFreeHost(h->host_tokens);
+  if (h->row_tokens) cudaFreeHost(h->row_tokens);
   if (h->burst_ring) cudaFreeHost(h->burst_ring);
   if (h->burst_event) cudaEventDestroy(h->burst_event);
   if (h->slab) cudaFree(h->slab);
@@ -1426,7 +1447,7 @@ int dfb_warm(DfbHandle* h, int32_t max_rows, int32_t max_context, int32_t kinds,
             io.sampling = sampling != 0;
             if (kind == 0) io.burst = true;
             else if (kind == 3) io.host = true;
-            else { io.stage = &a; io.out_tokens = kind == 2 ? h->tokens : nullptr; }
+            else { io.stage = &a; io.out_tokens = kind == 2 ? h->tokens : nullptr; io.publish = kind == 2; }
             DfbHandle::StepGraph* g = nullptr;
             int rc = get_step_graph(h, rows, nsplit, cols, io, &g);
             if (rc) return rc;
@@ -1568,12 +1589,39 @@ int dfb_decode_step(DfbHandle* h, const DfbStepDesc* s, dfb_stream_t stream_) {
   StepIo io;
   io.stage = &a;
   io.out_tokens = s->out_tokens;
+  if (io.out_tokens) {
+    // A step that the caller captures into a graph of their own is replayed without this function: nothing may count on
+    // the sequence word then, so it keeps the plain copy.
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    DFB_CUDA(cudaStreamIsCapturing(stream, &capture));
+    io.publish = capture == cudaStreamCaptureStatusNone;
+  }
   io.sampling = s->temperatures != nullptr;
   if (io.sampling && s->out_logits && h->step_mode == 1) return DFB_E_BAD_ARG;
   int rc = run_step(h, s->rows, split_bucket(h, bound, s->rows), s->block_table_cols, io, stream, s->out_logits);
   if (rc) return rc;
   ++h->steps;
+  if (io.publish) ++h->row_published;
   return 0;
+}
+
+// Waits until the sequence word behind published tokens has reached `want`: saves the driver's stream
+// synchronisation.  False after about a tenth of a second without it (an error, a debugger).
+static bool poll_published(const int* tokens, unsigned want) {
+  const volatile int* word = tokens + kMaxRows + 4;
+  for (long spin = 0; spin < 40000000l; ++spin)
+    if ((int)((unsigned)*word - want) >= 0) {
+      __atomic_thread_fence(__ATOMIC_ACQUIRE);
+      return true;
+    }
+  return false;
+}
+
+int dfb_wait_tokens(DfbHandle* h, int32_t* out_tokens, dfb_stream_t stream_) {
+  if (!h || !out_tokens || h->row_published == 0) return DFB_E_BAD_ARG;
+  if (!poll_published(h->row_tokens, h->row_published)) DFB_CUDA(cudaStreamSynchronize((cudaStream_t)stream_));
+  memcpy(out_tokens, h->row_tokens, sizeof(int) * (kMaxRows + 4));
+  return h->row_tokens[kMaxRows] ? DFB_E_DEVICE_STATUS : 0;
 }
 
 int dfb_decode_step_host(DfbHandle* h, int32_t rows, const int64_t* input_ids, const int64_t* positions,
@@ -1629,13 +1677,8 @@ int dfb_decode_step_host_sampled(DfbHandle* h, int32_t rows, const int64_t* inpu
   if (rc) return rc;
   bool arrived = false;
   if ((h->opt.host_io & 2) && (h->opt.host_io & 4) && h->use_graph) {
-    // The publishing kernel is the step's last node: once its sequence word has changed in pinned memory the
-    // tokens and the status are there.  Polling it saves the driver's stream synchronisation; after about a
-    // tenth of a second without it (an error, a debugger) the ordinary synchronisation takes over.
-    const int want = (int)++h->published;
-    volatile int* word = h->host_tokens + kMaxRows + 4;
-    for (long spin = 0; spin < 40000000l; ++spin)
-      if (*word == want) { arrived = true; break; }
+    // the publishing kernel is the step's last node: once its sequence word is there the tokens and the status are, too
+    arrived = poll_published(h->host_tokens, ++h->published);
   } else if (h->opt.host_io & 2) {
     ++h->published;
   }

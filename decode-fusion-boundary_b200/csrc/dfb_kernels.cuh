@@ -1064,9 +1064,14 @@ __global__ void copy_ints_kernel(const int* __restrict__ src, int* __restrict__ 
 }
 // `seq` (device) counts the steps published; its new value follows the data into host_out[n], after a
 // system-scope fence, so that a host thread polling that word sees complete data once it changes.
-__global__ void publish_result_kernel(const int* tokens_and_status, int* host_out, int n, unsigned int* seq) {
+// `dev_out`: an optional second copy in device memory.
+__global__ void publish_result_kernel(const int* tokens_and_status, int* host_out, int n, unsigned int* seq, int* dev_out) {
   pdl_wait();   // launched with a programmatic dependency on the LM head: everything before it has completed
-  if ((int)threadIdx.x < n) host_out[threadIdx.x] = tokens_and_status[threadIdx.x];
+  if ((int)threadIdx.x < n) {
+    const int v = tokens_and_status[threadIdx.x];
+    host_out[threadIdx.x] = v;
+    if (dev_out) dev_out[threadIdx.x] = v;
+  }
   __threadfence_system();
   __syncwarp();
   if (threadIdx.x == 0) {

@@ -95,7 +95,7 @@ typedef struct DfbStepDesc {
   const int32_t* row_active;  /* [rows] or NULL (= all active); 0 skips the KV write only */
   int32_t* out_tokens;        /* NULL, or int32[DFB_MAX_ROWS + 4]: greedy token ids in [0, rows) and the
                                  decoder's status word (see DfbStatus) in [DFB_MAX_ROWS, DFB_MAX_ROWS + 4),
-                                 so one device-to-host read returns both */
+                                 so one device-to-host read returns both (or dfb_wait_tokens) */
   float* out_logits;          /* [rows, vocab] or NULL; bf16-rounded logits as fp32 (parity checks) */
   const float* temperatures;  /* NULL = greedy step, or [rows] sampling temperatures (device): rows with a
                                  temperature above 1e-10 draw from softmax(logits / T), the others stay greedy
@@ -341,6 +341,12 @@ int dfb_slots_run(DfbHandle* h, int32_t max_steps, dfb_token_callback callback, 
  * torch's own generator stream is not reproduced: parity with the reference's sampler is in distribution.
  * Call it between steps (it synchronises nothing): a step in flight may see either stream position. */
 int dfb_set_seed(DfbHandle* h, uint64_t seed);
+
+/* Waits for the last dfb_decode_step that was given out_tokens and copies the same DFB_MAX_ROWS + 4 values into host
+ * memory: the step's last kernel also writes them to pinned memory, where this call polls for them (no copy, no
+ * stream synchronisation; `stream` is the step's, synchronised only when nothing arrives for a tenth of a second).
+ * Returns DFB_E_DEVICE_STATUS if a kernel recorded an error (the status word is left for dfb_read_status). */
+int dfb_wait_tokens(DfbHandle* h, int32_t* out_tokens, dfb_stream_t stream);
 
 /* Read (and clear) the device status word; synchronises nothing by itself, so
  * call it after the stream has been synchronised. */
