@@ -5,33 +5,53 @@ by ``dfb_store_kvcache`` (no Triton, no CPU fallback)."""
 
 from __future__ import annotations
 
+# Looked up at the first call (the package imports without torch and without the built library) and kept: one call of
+# store_kvcache on a short prompt takes a few microseconds, of which the imports and attribute chains of a call were two.
+_torch = _store = _prefill = _check = _stream = _bf16 = _i32 = _device = None
+
+
+def _load():
+    global _torch, _store, _prefill, _check, _stream, _bf16, _i32, _device
+    import torch
+
+    from . import native
+
+    lib = native.lib()
+    _store, _prefill, _check = lib.dfb_store_kvcache, lib.dfb_prefill_attention, native.check
+    _bf16, _i32, _device = torch.bfloat16, torch.int32, torch.cuda.current_device
+    # the raw handle of the current stream; the public call builds a Stream object (1 us) around it
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+    _stream = (lambda: raw(_device())) if raw else (lambda: torch.cuda.current_stream().cuda_stream)
+    _torch = torch
+
 
 def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> None:
     """``key`` / ``value``: ``[N, kv_heads, head_dim]`` bf16 CUDA tensors (any row
     stride); ``k_cache`` / ``v_cache``: one layer's ``[num_blocks, block_size,
     kv_heads, head_dim]`` views; ``slot_mapping``: int32 ``[N]``, -1 = skip.
     ``status``: optional int32 CUDA tensor ``[4]`` that receives a bad slot."""
-    import torch
-
-    from . import native
-
+    if _torch is None:
+        _load()
     n, num_heads, head_dim = key.shape
     d = num_heads * head_dim
-    assert key.stride(-1) == 1 and value.stride(-1) == 1
-    assert key.stride(1) == head_dim and value.stride(1) == head_dim
+    k_stride, k_head, k_one = key.stride()
+    v_stride, v_head, v_one = value.stride()
+    assert k_one == 1 and v_one == 1
+    assert k_head == head_dim and v_head == head_dim
     assert k_cache.stride(1) == d and v_cache.stride(1) == d
     assert slot_mapping.numel() == n
-    if key.dtype != torch.bfloat16 or k_cache.dtype != torch.bfloat16:
+    if key.dtype != _bf16 or k_cache.dtype != _bf16:
         raise TypeError("store_kvcache moves bf16 rows")
-    if slot_mapping.dtype != torch.int32 or not slot_mapping.is_cuda:
+    if slot_mapping.dtype != _i32 or not slot_mapping.is_cuda:
         raise TypeError("slot_mapping must be an int32 CUDA tensor")
     if n == 0:
         return
-    num_slots = k_cache.shape[0] * k_cache.shape[1]
-    native.check(native.lib().dfb_store_kvcache(
-        key.data_ptr(), value.data_ptr(), key.stride(0), value.stride(0), k_cache.data_ptr(), v_cache.data_ptr(),
-        slot_mapping.data_ptr(), n, d, num_slots, status.data_ptr() if status is not None else None,
-        torch.cuda.current_stream().cuda_stream), "dfb_store_kvcache")
+    blocks, block_size, _, _ = k_cache.shape
+    code = _store(key.data_ptr(), value.data_ptr(), k_stride, v_stride, k_cache.data_ptr(), v_cache.data_ptr(),
+                  slot_mapping.data_ptr(), n, d, blocks * block_size, status.data_ptr() if status is not None else None,
+                  _stream())
+    if code:
+        _check(code, "dfb_store_kvcache")
 
 
 def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: float, cu_seqlens_k=None,
@@ -42,20 +62,18 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
     ``[N, kv_heads, 128]``, the projections of the same tokens.  With it (prefix cache): ``k`` / ``v`` are one
     layer's cache ``[num_blocks, block_size, kv_heads, 128]`` and ``block_table`` the int32 CUDA
     ``[batch, columns]`` table.  Returns ``[N, q_heads, 128]`` bf16."""
-    import torch
-
-    from . import native
-
+    if _torch is None:
+        _load()
     n, q_heads, head_dim = q.shape
     assert q.stride(-1) == 1 and k.stride(-1) == 1 and v.stride(-1) == 1 and q.stride(1) == head_dim
-    if q.dtype != torch.bfloat16 or k.dtype != torch.bfloat16 or v.dtype != torch.bfloat16:
+    if q.dtype != _bf16 or k.dtype != _bf16 or v.dtype != _bf16:
         raise TypeError("prefill_attention takes bf16 tensors")
-    if cu_seqlens_q.dtype != torch.int32 or not cu_seqlens_q.is_cuda:
+    if cu_seqlens_q.dtype != _i32 or not cu_seqlens_q.is_cuda:
         raise TypeError("cu_seqlens_q must be an int32 CUDA tensor")
     if block_table is not None:
         num_blocks, block_size, kv_heads = k.shape[0], k.shape[1], k.shape[2]
         assert k.stride(2) == head_dim and v.stride(2) == head_dim and k.stride(0) == block_size * k.stride(1)
-        if block_table.dtype != torch.int32 or block_table.stride(-1) != 1 or cu_seqlens_k is None:
+        if block_table.dtype != _i32 or block_table.stride(-1) != 1 or cu_seqlens_k is None:
             raise TypeError("the prefix-cache case needs an int32 block table and cu_seqlens_k")
         k_stride, v_stride = k.stride(1), v.stride(1)
         bt_ptr, bt_stride = block_table.data_ptr(), block_table.stride(0)
@@ -65,13 +83,14 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
         num_blocks = block_size = 0
         k_stride, v_stride = k.stride(0), v.stride(0)
         bt_ptr, bt_stride = None, 0
-    out = torch.empty(n, q_heads, head_dim, dtype=torch.bfloat16, device=q.device)
+    out = _torch.empty((n, q_heads, head_dim), dtype=_bf16, device=q.device)
     if n == 0:
         return out
-    native.check(native.lib().dfb_prefill_attention(
+    code = _prefill(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_seqlens_q.data_ptr(),
         cu_seqlens_k.data_ptr() if cu_seqlens_k is not None else None, cu_seqlens_q.numel() - 1, int(max_seqlen_q),
-        q.stride(0), k_stride, v_stride, out.stride(0), q_heads, kv_heads, head_dim, float(softmax_scale),
-        bt_ptr, bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else None,
-        torch.cuda.current_stream().cuda_stream), "dfb_prefill_attention")
+        q.stride(0), k_stride, v_stride, q_heads * head_dim, q_heads, kv_heads, head_dim, float(softmax_scale),
+        bt_ptr, bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else None, _stream())
+    if code:
+        _check(code, "dfb_prefill_attention")
     return out
