@@ -10,6 +10,7 @@
 #include "dfb_attncluster.cuh"
 #include "dfb_attnring.cuh"
 #include "dfb_prefilltc.cuh"
+#include "dfb_wide.cuh"
 
 #include <cstdio>
 #include <cstdlib>
@@ -329,6 +330,28 @@ struct DfbHandle {
     std::vector<int> table;     // the slot's block table (physical block ids)
   };
   std::vector<Slot> slots;
+  // Steps of 9 to 32 slots at once (dfb_wide.cuh).  Buffers of 32 rows in one slab, allocated with the first slot.
+  struct Wide {
+    void* slab = nullptr;
+    int* stage = nullptr;            // device: ids[32] | positions[32] | active[32] | temperatures[32] | block tables[32, max_pages]
+    int* host_stage = nullptr;       // pinned copy
+    int* host_tokens = nullptr;      // pinned: tokens[32] | status[4] | sequence word
+    bf16 *hbuf = nullptr, *res[2] = {nullptr, nullptr}, *qkv = nullptr, *attn = nullptr, *act = nullptr;
+    float* part_o = nullptr;
+    float2* part_ml = nullptr;
+    unsigned int *tickets = nullptr, *seq = nullptr;
+    ArgmaxPart* parts = nullptr;
+    int* tokens = nullptr;
+    unsigned int published = 0;
+    std::map<int, cudaGraphExec_t> graphs;      // by groups of 8 rows, attention grid, sampling
+  } wide;
+  bool tuned = false;                // an option that selects kernels has been set: no wide steps
+  void drop_graphs() {
+    for (auto& kv : graphs) { cudaGraphExecDestroy(kv.second.exec); cudaGraphDestroy(kv.second.graph); }
+    graphs.clear();
+    for (auto& kv : wide.graphs) cudaGraphExecDestroy(kv.second);
+    wide.graphs.clear();
+  }
   int* burst_status() const { return burst_ring + kMaxBurst * kMaxRows; }
   volatile int* burst_done() const { return burst_ring + kMaxBurst * kMaxRows + 4; }
   cudaStream_t capture_stream = nullptr;
@@ -1097,6 +1120,155 @@ int run_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, 
   return 0;
 }
 
+// ---- steps of 9 to 32 rows (dfb_wide.cuh) ------------------------------------------------------------------
+bool wide_usable(const DfbHandle* h) {
+  return h->full_geometry && !h->sharded() && h->step_mode == 0 && !h->tuned && !h->trace_on && h->m.vocab % 16 == 0 &&
+         h->m.max_model_len <= kMaxSplits * kAttnChunk;
+}
+
+int wide_prepare(DfbHandle* h) {
+  DfbHandle::Wide& w = h->wide;
+  if (w.slab) return 0;
+  const DfbModelDesc& m = h->m;
+  size_t off = 0;
+  auto carve = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
+  const size_t stage_ints = kWideRows * (4 + h->max_pages);
+  const size_t o_stage = carve(sizeof(int) * stage_ints), o_h = carve(sizeof(bf16) * kWideRows * m.hidden);
+  const size_t o_r0 = carve(sizeof(bf16) * kWideRows * m.hidden), o_r1 = carve(sizeof(bf16) * kWideRows * m.hidden);
+  const size_t o_qkv = carve(sizeof(bf16) * kWideRows * h->qkv_rows()), o_attn = carve(sizeof(bf16) * kWideRows * h->q_size());
+  const size_t o_act = carve(sizeof(bf16) * kWideRows * m.intermediate);
+  const size_t o_po = carve(sizeof(float) * kWideRows * m.kv_heads * kMaxSplits * 2 * kHeadDim);
+  const size_t o_ml = carve(sizeof(float2) * kWideRows * m.kv_heads * kMaxSplits * 2);
+  const size_t o_tk = carve(sizeof(unsigned) * (kWideRows * m.kv_heads + 1)), o_seq = carve(sizeof(unsigned));
+  const size_t o_parts = carve(sizeof(ArgmaxPart) * kWideRows * h->sm_count), o_tok = carve(sizeof(int) * kWideRows);
+  void* slab = nullptr;
+  DFB_CUDA(cudaMalloc(&slab, off));
+  cudaError_t e = cudaMemset(slab, 0, off);
+  if (e == cudaSuccess && !w.host_stage) e = cudaMallocHost((void**)&w.host_stage, sizeof(int) * stage_ints);
+  if (e == cudaSuccess && !w.host_tokens) e = cudaMallocHost((void**)&w.host_tokens, sizeof(int) * (kWideRows + 8));
+  if (e != cudaSuccess) { cudaFree(slab); return (int)e; }
+  w.host_tokens[kWideRows + 4] = 0;
+  char* s = (char*)slab;
+  w.stage = (int*)(s + o_stage); w.hbuf = (bf16*)(s + o_h); w.res[0] = (bf16*)(s + o_r0); w.res[1] = (bf16*)(s + o_r1);
+  w.qkv = (bf16*)(s + o_qkv); w.attn = (bf16*)(s + o_attn); w.act = (bf16*)(s + o_act); w.part_o = (float*)(s + o_po);
+  w.part_ml = (float2*)(s + o_ml); w.tickets = (unsigned*)(s + o_tk); w.seq = (unsigned*)(s + o_seq);
+  w.parts = (ArgmaxPart*)(s + o_parts); w.tokens = (int*)(s + o_tok);
+  w.slab = slab;
+  return 0;
+}
+
+template <int NG, int MODE>
+void launch_wide_norm(Launcher& L, const GemvArgs& a, int grid, bool allow_pdl = true) {
+  auto kernel = wide_norm_kernel<NG, MODE>;
+  constexpr int smem = WideSmem<NG, MODE>::bytes();
+  cudaError_t e = ensure_dynamic_smem((const void*)kernel, smem);
+  if (e != cudaSuccess) { L.err = (int)e; return; }
+  L.launch(kernel, dim3(grid), dim3(256), a, allow_pdl, smem);
+}
+template <int K, int NG>
+void launch_wide_store(Launcher& L, const GemvArgs& a, int n) {
+  auto kernel = wide_store_kernel<K, NG>;
+  constexpr int smem = WideStoreSmem<K, NG>::bytes();
+  cudaError_t e = ensure_dynamic_smem((const void*)kernel, smem);
+  if (e != cudaSuccess) { L.err = (int)e; return; }
+  L.launch(kernel, dim3(n / 16 * 2), dim3(256), a, true, smem, 2);
+}
+
+// the step's kernels for NG groups of 8 rows; `chunks`: grid of the attention kernel
+template <int NG>
+int enqueue_wide(DfbHandle* h, int chunks, bool sampling, cudaStream_t stream) {
+  const DfbModelDesc& m = h->m;
+  DfbHandle::Wide& w = h->wide;
+  DFB_CUDA(cudaMemcpyAsync(w.stage, w.host_stage, sizeof(int) * kWideRows * (4 + h->max_pages), cudaMemcpyHostToDevice, stream));
+  Launcher L{stream, h->use_pdl};
+  L.opt = &h->opt;
+  L.carve = 100;      // every kernel of this chain is sized to fit beside its neighbour in all of the shared memory
+  auto norm = [&](const bf16* x, const int* ids, const bf16* res_in, bf16* res_out, const void* nw, const void* wt) {
+    GemvArgs a = {};
+    a.w = (const bf16*)wt; a.rows = 8 * NG; a.k = m.hidden; a.x = x; a.ids = ids; a.res_in = res_in; a.res_out = res_out;
+    a.norm_w = (const bf16*)nw; a.eps = m.eps; a.status = h->status; a.embed_rows = h->embed_rows();
+    return a;
+  };
+  auto store = [&](const bf16* x, const void* wt) {
+    GemvArgs a = {};
+    a.w = (const bf16*)wt; a.rows = 8 * NG; a.x = x; a.out = w.hbuf; a.out_stride = m.hidden; a.status = h->status;
+    return a;
+  };
+  int cur = 0;
+  for (int l = 0; l < m.layers; ++l) {
+    const DfbLayerWeights& lw = h->layers[l];
+    GemvArgs q = l == 0 ? norm((const bf16*)m.embed, w.stage, nullptr, w.res[0], lw.ln_in, lw.wqkv)
+                        : norm(w.hbuf, nullptr, w.res[cur], w.res[cur ^ 1], lw.ln_in, lw.wqkv);
+    if (l) cur ^= 1;
+    q.n_tiles = h->qkv_rows() / 16; q.out = w.qkv; q.out_stride = h->qkv_rows();
+    launch_wide_norm<NG, kModeNormStore>(L, q, (q.n_tiles + 1) / 2, l != 0);
+    AttnArgs a = {};
+    a.qkv = w.qkv; a.qkv_stride = h->qkv_rows(); a.q_size = h->q_size(); a.kv_size = h->kv_size();
+    a.positions = w.stage + kWideRows; a.row_active = w.stage + 2 * kWideRows; a.block_tables = w.stage + 4 * kWideRows;
+    a.bt_stride = h->max_pages; a.packed_rows = kWideRows;
+    a.q_norm = (const bf16*)lw.q_norm; a.k_norm = (const bf16*)lw.k_norm; a.cos_sin = m.rope_cos_sin; a.eps = m.eps;
+    a.scale = 1.0f / sqrtf((float)m.head_dim);
+    a.k_cache = (bf16*)m.k_cache + (size_t)l * h->kv_layer_elems; a.v_cache = (bf16*)m.v_cache + (size_t)l * h->kv_layer_elems;
+    a.block_size = m.block_size; a.kv_heads = m.kv_heads; a.num_blocks = m.num_blocks; a.max_pos = m.max_model_len;
+    a.out = w.attn; a.part_o = w.part_o; a.part_ml = w.part_ml; a.tickets = w.tickets; a.status = h->status;
+    auto attn = paged_attention_ring_kernel<kAttnChunk>;
+    DFB_CUDA(ensure_dynamic_smem((const void*)attn, kRingSmemBytes));
+    L.launch(attn, dim3(chunks), dim3(kRingThreads), a, true, kRingSmemBytes);
+    launch_wide_store<2048, NG>(L, store(w.attn, lw.wo), m.hidden);
+    GemvArgs u = norm(w.hbuf, nullptr, w.res[cur], w.res[cur ^ 1], lw.ln_post, lw.wgu);
+    cur ^= 1;
+    u.n_tiles = m.intermediate / 8; u.gate_rows = m.intermediate; u.out = w.act; u.out_stride = m.intermediate;
+    launch_wide_norm<NG, kModeNormSwiglu>(L, u, (u.n_tiles + 2) / 3);
+    launch_wide_store<3072, NG>(L, store(w.act, lw.wd), m.hidden);
+    if (L.err) return L.err;
+  }
+  GemvArgs v = norm(w.hbuf, nullptr, w.res[cur], nullptr, m.final_norm, h->lm_head());
+  v.n_tiles = m.vocab / 16; v.vocab = m.vocab; v.parts = w.parts; v.ticket = w.tickets + kWideRows * m.kv_heads;
+  v.tokens = w.tokens; v.sample_ctr = h->sample_ctr; v.sample_seed = h->sample_seed;
+  v.temps = sampling ? reinterpret_cast<const float*>(w.stage + 3 * kWideRows) : nullptr;
+  launch_wide_norm<NG, kModeNormArgmax>(L, v, v.n_tiles < h->sm_count ? v.n_tiles : h->sm_count);
+  if (L.err) return L.err;
+  publish_wide_kernel<<<1, 64, 0, stream>>>(w.tokens, h->status, w.host_tokens, w.seq);
+  DFB_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// inputs of `rows` (9 to 32) rows are in wide.host_stage; returns when the tokens are in wide.host_tokens
+int wide_step(DfbHandle* h, int rows, int total_chunks, bool sampling, cudaStream_t stream) {
+  DfbHandle::Wide& w = h->wide;
+  const int groups = (rows + 7) / 8;
+  int chunks = 64;                  // few grids, so that few graphs: the attention CTAs without a chunk leave at once
+  while (chunks < total_chunks) chunks <<= 1;
+  auto enqueue = [&](cudaStream_t s) {
+    return groups == 2 ? enqueue_wide<2>(h, chunks, sampling, s) : groups == 3 ? enqueue_wide<3>(h, chunks, sampling, s)
+                                                                                : enqueue_wide<4>(h, chunks, sampling, s);
+  };
+  if (h->use_graph) {
+    const int key = ((chunks * 8 + groups) * 2 + (sampling ? 1 : 0)) * 2 + (h->use_pdl ? 1 : 0);
+    auto it = w.graphs.find(key);
+    if (it == w.graphs.end()) {
+      cudaGraph_t graph = nullptr;
+      cudaGraphExec_t exec = nullptr;
+      DFB_CUDA(cudaStreamBeginCapture(h->capture_stream, cudaStreamCaptureModeThreadLocal));
+      const int rc = enqueue(h->capture_stream);
+      cudaError_t e = cudaStreamEndCapture(h->capture_stream, &graph);
+      if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
+      if (e != cudaSuccess) return (int)e;
+      e = cudaGraphInstantiate(&exec, graph, 0);
+      cudaGraphDestroy(graph);
+      if (e != cudaSuccess) return (int)e;
+      it = w.graphs.emplace(key, exec).first;
+    }
+    DFB_CUDA(cudaGraphLaunch(it->second, stream));
+  } else {
+    const int rc = enqueue(stream);
+    if (rc) return rc;
+  }
+  ++w.published;
+  ++h->steps;
+  return 0;
+}
+
 }  // namespace
 
 extern "C" {
@@ -1219,7 +1391,10 @@ void dfb_destroy(DfbHandle* h) {
   if (!h) return;
   // a burst in flight still writes the pinned token ring: let it finish before anything is freed
   if (h->burst_steps && h->burst_event) cudaEventSynchronize(h->burst_event);
-  for (auto& kv : h->graphs) { cudaGraphExecDestroy(kv.second.exec); cudaGraphDestroy(kv.second.graph); }
+  h->drop_graphs();
+  if (h->wide.slab) cudaFree(h->wide.slab);
+  if (h->wide.host_stage) cudaFreeHost(h->wide.host_stage);
+  if (h->wide.host_tokens) cudaFreeHost(h->wide.host_tokens);
   if (h->capture_stream) cudaStreamDestroy(h->capture_stream);
   for (int r = 0; r < kMaxRanks; ++r) {
     if (h->loopback[r]) cudaFree(h->loopback[r]);
@@ -1244,8 +1419,7 @@ int dfb_set_tensor_parallel(DfbHandle* h, const DfbTensorParallel* tp) {
   h->tp = *tp;
   // the narrow o_proj / down_proj shards run on the FP32 kernels at every batch; two rows stay there as a whole
   if (h->opt.row_max_rows == 1) h->opt.row_max_rows = 2;
-  for (auto& kv : h->graphs) { cudaGraphExecDestroy(kv.second.exec); cudaGraphDestroy(kv.second.graph); }
-  h->graphs.clear();
+  h->drop_graphs();
   return 0;
 }
 
@@ -1279,8 +1453,7 @@ int dfb_tp_open_peers(DfbHandle* h, const void* handles) {
     h->windows[r] = (unsigned char*)mapped;
   }
   h->direct = true;
-  for (auto& kv : h->graphs) { cudaGraphExecDestroy(kv.second.exec); cudaGraphDestroy(kv.second.graph); }
-  h->graphs.clear();
+  h->drop_graphs();
   return 0;
 }
 
@@ -1297,18 +1470,12 @@ int dfb_tp_open_loopback(DfbHandle* h) {
     h->windows[r] = h->loopback[r];
   }
   h->direct = true;
-  for (auto& kv : h->graphs) { cudaGraphExecDestroy(kv.second.exec); cudaGraphDestroy(kv.second.graph); }
-  h->graphs.clear();
+  h->drop_graphs();
   return 0;
 }
 
 int dfb_set_option(DfbHandle* h, int option, int value) {
   if (!h) return DFB_E_BAD_ARG;
-  // every option below may change which kernels a captured step holds
-  auto drop_graphs = [&]() {
-    for (auto& kv : h->graphs) { cudaGraphExecDestroy(kv.second.exec); cudaGraphDestroy(kv.second.graph); }
-    h->graphs.clear();
-  };
   switch (option) {
     case DFB_OPT_USE_GRAPH: h->use_graph = value != 0; return 0;
     case DFB_OPT_USE_PDL: h->use_pdl = value != 0; return 0;
@@ -1408,7 +1575,10 @@ int dfb_set_option(DfbHandle* h, int option, int value) {
       break;
     default: return DFB_E_BAD_ARG;
   }
-  drop_graphs();
+  // every option above that did not return may change which kernels a captured step holds
+  if (option != DFB_OPT_TRACE && option != DFB_OPT_PEER_WAIT_US && option != DFB_OPT_HOST_IO && option != DFB_OPT_PERSIST_CTAS)
+    h->tuned = true;
+  h->drop_graphs();
   return 0;
 }
 
@@ -1556,8 +1726,7 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
 int dfb_set_seed(DfbHandle* h, uint64_t seed) {
   if (!h) return DFB_E_BAD_ARG;
   // the seed is a kernel argument of every captured LM head; the noise stream restarts at step 0
-  for (auto& kv : h->graphs) { cudaGraphExecDestroy(kv.second.exec); cudaGraphDestroy(kv.second.graph); }
-  h->graphs.clear();
+  h->drop_graphs();
   h->sample_seed = seed;
   DFB_CUDA(cudaMemset(h->sample_ctr, 0, sizeof(unsigned)));
   return 0;
@@ -1605,10 +1774,10 @@ int dfb_decode_step(DfbHandle* h, const DfbStepDesc* s, dfb_stream_t stream_) {
   return 0;
 }
 
-// Waits until the sequence word behind published tokens has reached `want`: saves the driver's stream
+// Waits until a sequence word behind published tokens has reached `want`: saves the driver's stream
 // synchronisation.  False after about a tenth of a second without it (an error, a debugger).
-static bool poll_published(const int* tokens, unsigned want) {
-  const volatile int* word = tokens + kMaxRows + 4;
+static bool poll_published(const int* word_, unsigned want) {
+  const volatile int* word = word_;
   for (long spin = 0; spin < 40000000l; ++spin)
     if ((int)((unsigned)*word - want) >= 0) {
       __atomic_thread_fence(__ATOMIC_ACQUIRE);
@@ -1619,7 +1788,7 @@ static bool poll_published(const int* tokens, unsigned want) {
 
 int dfb_wait_tokens(DfbHandle* h, int32_t* out_tokens, dfb_stream_t stream_) {
   if (!h || !out_tokens || h->row_published == 0) return DFB_E_BAD_ARG;
-  if (!poll_published(h->row_tokens, h->row_published)) DFB_CUDA(cudaStreamSynchronize((cudaStream_t)stream_));
+  if (!poll_published(h->row_tokens + kMaxRows + 4, h->row_published)) DFB_CUDA(cudaStreamSynchronize((cudaStream_t)stream_));
   memcpy(out_tokens, h->row_tokens, sizeof(int) * (kMaxRows + 4));
   return h->row_tokens[kMaxRows] ? DFB_E_DEVICE_STATUS : 0;
 }
@@ -1678,7 +1847,7 @@ int dfb_decode_step_host_sampled(DfbHandle* h, int32_t rows, const int64_t* inpu
   bool arrived = false;
   if ((h->opt.host_io & 2) && (h->opt.host_io & 4) && h->use_graph) {
     // the publishing kernel is the step's last node: once its sequence word is there the tokens and the status are, too
-    arrived = poll_published(h->host_tokens, ++h->published);
+    arrived = poll_published(h->host_tokens + kMaxRows + 4, ++h->published);
   } else if (h->opt.host_io & 2) {
     ++h->published;
   }
@@ -1739,6 +1908,47 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
     live[n_live++] = i;
   }
   int first_error = 0;
+  // More rows than one launch of the ordinary kernels holds: all of them in one pass over the weights.  (After a tuning
+  // option has been set the step keeps to the kernels that the option speaks of, in launches of 8 rows.)
+  if (n_live > kMaxRows && wide_usable(h)) {
+    if (h->burst_steps) return DFB_E_BAD_ARG;
+    DfbHandle::Wide& w = h->wide;
+    int rc = wide_prepare(h);
+    if (rc) return rc;
+    int* hs = w.host_stage;
+    int chunks = 0;
+    bool sampled = false;
+    for (int r = 0; r < kWideRows; ++r) {
+      const bool on = r < n_live;
+      const DfbHandle::Slot* s = on ? &h->slots[live[r]] : nullptr;
+      hs[r] = on ? (int)s->token : 0;
+      hs[kWideRows + r] = on ? (int)s->position : -1;
+      hs[2 * kWideRows + r] = on ? 1 : 0;
+      const float t = on ? s->temperature : 0.f;
+      memcpy(&hs[3 * kWideRows + r], &t, sizeof(t));
+      int* bt = hs + 4 * kWideRows + r * h->max_pages;
+      const int cols = on ? (int)s->table.size() : 0;
+      for (int c = 0; c < h->max_pages; ++c) bt[c] = c < cols ? s->table[c] : 0;
+      if (on) chunks += (int)(s->position / kAttnChunk) + 1;
+      sampled = sampled || t > 1e-10f;
+    }
+    rc = wide_step(h, n_live, chunks, sampled, (cudaStream_t)stream);
+    if (rc) return rc;
+    if (!poll_published(w.host_tokens + kWideRows + 4, w.published)) DFB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
+    for (int r = 0; r < n_live; ++r) {
+      DfbHandle::Slot& s = h->slots[live[r]];
+      s.token = w.host_tokens[r];
+      s.position += 1;
+      sampled_tokens[live[r]] = w.host_tokens[r];
+      emitted[live[r]] = 1;
+    }
+    if (w.host_tokens[kWideRows]) {
+      for (int i = 0; i < 4; ++i) h->last_status[i] = w.host_tokens[kWideRows + i];
+      DFB_CUDA(cudaMemsetAsync(h->status, 0, sizeof(int) * 4, (cudaStream_t)stream));
+      return DFB_E_DEVICE_STATUS;
+    }
+    return 0;
+  }
   for (int g0 = 0; g0 < n_live; g0 += kMaxRows) {
     const int rows = n_live - g0 < kMaxRows ? n_live - g0 : kMaxRows;
     int64_t ids[kMaxRows], pos[kMaxRows];

@@ -100,8 +100,24 @@ template <int CH>
 __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(const AttnArgs a) {
   static_assert(CH == kAttnChunk || 2 * CH == kAttnChunk, "64 or 32 positions per CTA");
   if (!a.late_trigger) pdl_launch_dependents();
-  const int split = blockIdx.x, row = blockIdx.y;
+  int split = blockIdx.x, row = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (a.packed_rows) {
+    // up to 32 rows of uneven lengths: CTA i takes the i-th chunk of all rows' chunks one after the other, so that the
+    // grid is as large as the work (20 rows: 165 CTAs instead of 20 x 32); a negative position = no row
+    const int p = lane < a.packed_rows ? a.positions[lane] : -1;
+    const int n = p < 0 ? 0 : (min(p, a.max_pos - 1) + CH) / CH;
+    int end = n;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int up = __shfl_up_sync(0xffffffffu, end, d);
+      if (lane >= d) end += up;
+    }
+    const unsigned before = __ballot_sync(0xffffffffu, end <= split);      // rows that end before this chunk
+    row = __popc(before);
+    if (row >= 32) return;
+    split -= __shfl_sync(0xffffffffu, end - n, row);
+  }
   if (tid == 0) { trace_min(a.trace, 0); trace_max(a.trace, 4); }
   int pos = a.positions[row];
   bool write_ok = true;
@@ -112,7 +128,7 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
   }
   int ctx = pos + 1;
   int nsplits = (ctx + CH - 1) / CH;
-  if (nsplits > (int)gridDim.x) {   // the host's context bound was too small (see paged_attention_kernel)
+  if (!a.packed_rows && nsplits > (int)gridDim.x) {   // the host's context bound was too small (see paged_attention_kernel)
     if (split == 0) report_status(a.status, kStatusBadGrid, kKernelAttention, row, pos);
     nsplits = (int)gridDim.x;
     ctx = nsplits * CH;

@@ -562,6 +562,7 @@ struct AttnArgs {
   int kv_heads;
   int num_blocks;
   int max_pos;
+  int packed_rows;              // streaming kernel: 0 = grid (chunk, row); else the 1-D grid walks the chunks of so many rows
   int ctx_limit;                // cluster kernel: contexts beyond this are an error (the caller's bound)
   int* status;                  // [4]: code, kernel id, index, observed value
   __nv_bfloat16* out;           // [rows, q_size]

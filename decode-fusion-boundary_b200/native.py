@@ -16,7 +16,7 @@ from pathlib import Path
 PKG_DIR = Path(__file__).resolve().parent
 LIB_PATH = PKG_DIR / "libdfb_decode.so"
 SOURCES = [PKG_DIR / "csrc" / "dfb_api.cu"]
-HEADERS = [PKG_DIR / "csrc" / "dfb_kernels.cuh", PKG_DIR / "csrc" / "dfb_persistent.cuh", PKG_DIR / "csrc" / "dfb_rowgemv.cuh", PKG_DIR / "csrc" / "dfb_exchange.cuh", PKG_DIR / "csrc" / "dfb_pairgemv.cuh", PKG_DIR / "csrc" / "dfb_tcgemv.cuh", PKG_DIR / "csrc" / "dfb_attncluster.cuh", PKG_DIR / "csrc" / "dfb_attnring.cuh", PKG_DIR / "csrc" / "dfb_prefill.cuh", PKG_DIR / "csrc" / "dfb_prefilltc.cuh", PKG_DIR.parent / "include" / "dfb_decode.h"]
+HEADERS = [PKG_DIR / "csrc" / "dfb_kernels.cuh", PKG_DIR / "csrc" / "dfb_persistent.cuh", PKG_DIR / "csrc" / "dfb_rowgemv.cuh", PKG_DIR / "csrc" / "dfb_exchange.cuh", PKG_DIR / "csrc" / "dfb_pairgemv.cuh", PKG_DIR / "csrc" / "dfb_tcgemv.cuh", PKG_DIR / "csrc" / "dfb_attncluster.cuh", PKG_DIR / "csrc" / "dfb_attnring.cuh", PKG_DIR / "csrc" / "dfb_wide.cuh", PKG_DIR / "csrc" / "dfb_prefill.cuh", PKG_DIR / "csrc" / "dfb_prefilltc.cuh", PKG_DIR.parent / "include" / "dfb_decode.h"]
 
 DFB_ABI_VERSION = 2
 DFB_MAX_ROWS = 8
