@@ -1122,7 +1122,7 @@ int run_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, 
 
 // ---- steps of 9 to 32 rows (dfb_wide.cuh) ------------------------------------------------------------------
 bool wide_usable(const DfbHandle* h) {
-  return h->full_geometry && !h->sharded() && h->step_mode == 0 && !h->tuned && !h->trace_on && h->m.vocab % 16 == 0 &&
+  return h->full_geometry && !h->sharded() && h->step_mode == 0 && !h->tuned && h->m.vocab % 16 == 0 &&
          h->m.max_model_len <= kMaxSplits * kAttnChunk;
 }
 
@@ -1137,8 +1137,8 @@ int wide_prepare(DfbHandle* h) {
   const size_t o_r0 = carve(sizeof(bf16) * kWideRows * m.hidden), o_r1 = carve(sizeof(bf16) * kWideRows * m.hidden);
   const size_t o_qkv = carve(sizeof(bf16) * kWideRows * h->qkv_rows()), o_attn = carve(sizeof(bf16) * kWideRows * h->q_size());
   const size_t o_act = carve(sizeof(bf16) * kWideRows * m.intermediate);
-  const size_t o_po = carve(sizeof(float) * kWideRows * m.kv_heads * kMaxSplits * 2 * kHeadDim);
-  const size_t o_ml = carve(sizeof(float2) * kWideRows * m.kv_heads * kMaxSplits * 2);
+  const size_t o_po = carve(sizeof(float) * kWideRows * m.kv_heads * kWideSplits * 2 * kHeadDim);
+  const size_t o_ml = carve(sizeof(float2) * kWideRows * m.kv_heads * kWideSplits * 2);
   const size_t o_tk = carve(sizeof(unsigned) * (kWideRows * m.kv_heads + 1)), o_seq = carve(sizeof(unsigned));
   const size_t o_parts = carve(sizeof(ArgmaxPart) * kWideRows * h->sm_count), o_tok = carve(sizeof(int) * kWideRows);
   void* slab = nullptr;
@@ -1163,7 +1163,7 @@ void launch_wide_norm(Launcher& L, const GemvArgs& a, int grid, bool allow_pdl =
   constexpr int smem = WideSmem<NG, MODE>::bytes();
   cudaError_t e = ensure_dynamic_smem((const void*)kernel, smem);
   if (e != cudaSuccess) { L.err = (int)e; return; }
-  L.launch(kernel, dim3(grid), dim3(256), a, allow_pdl, smem);
+  L.launch(kernel, dim3(grid), dim3(256), a, allow_pdl, smem, MODE == kModeNormArgmax ? 0 : kWideCluster);
 }
 template <int K, int NG>
 void launch_wide_store(Launcher& L, const GemvArgs& a, int n) {
@@ -1171,26 +1171,28 @@ void launch_wide_store(Launcher& L, const GemvArgs& a, int n) {
   constexpr int smem = WideStoreSmem<K, NG>::bytes();
   cudaError_t e = ensure_dynamic_smem((const void*)kernel, smem);
   if (e != cudaSuccess) { L.err = (int)e; return; }
-  L.launch(kernel, dim3(n / 16 * 2), dim3(256), a, true, smem, 2);
+  L.launch(kernel, dim3(n / 32 * kWideCluster), dim3(256), a, true, smem, kWideCluster);
 }
 
-// the step's kernels for NG groups of 8 rows; `chunks`: grid of the attention kernel
+// the step's kernels for NG groups of 8 rows; `chunks`: grid of the attention kernel, of 32 (half) or 64 positions each
 template <int NG>
-int enqueue_wide(DfbHandle* h, int chunks, bool sampling, cudaStream_t stream) {
+int enqueue_wide(DfbHandle* h, int chunks, bool half, bool sampling, cudaStream_t stream) {
   const DfbModelDesc& m = h->m;
   DfbHandle::Wide& w = h->wide;
   DFB_CUDA(cudaMemcpyAsync(w.stage, w.host_stage, sizeof(int) * kWideRows * (4 + h->max_pages), cudaMemcpyHostToDevice, stream));
-  Launcher L{stream, h->use_pdl};
+  Launcher L{stream, h->use_pdl, h->trace_on ? h->trace : nullptr};
   L.opt = &h->opt;
   L.carve = 100;      // every kernel of this chain is sized to fit beside its neighbour in all of the shared memory
   auto norm = [&](const bf16* x, const int* ids, const bf16* res_in, bf16* res_out, const void* nw, const void* wt) {
     GemvArgs a = {};
+    a.trace = L.next_trace();
     a.w = (const bf16*)wt; a.rows = 8 * NG; a.k = m.hidden; a.x = x; a.ids = ids; a.res_in = res_in; a.res_out = res_out;
     a.norm_w = (const bf16*)nw; a.eps = m.eps; a.status = h->status; a.embed_rows = h->embed_rows();
     return a;
   };
   auto store = [&](const bf16* x, const void* wt) {
     GemvArgs a = {};
+    a.trace = L.next_trace();
     a.w = (const bf16*)wt; a.rows = 8 * NG; a.x = x; a.out = w.hbuf; a.out_stride = m.hidden; a.status = h->status;
     return a;
   };
@@ -1211,7 +1213,8 @@ int enqueue_wide(DfbHandle* h, int chunks, bool sampling, cudaStream_t stream) {
     a.k_cache = (bf16*)m.k_cache + (size_t)l * h->kv_layer_elems; a.v_cache = (bf16*)m.v_cache + (size_t)l * h->kv_layer_elems;
     a.block_size = m.block_size; a.kv_heads = m.kv_heads; a.num_blocks = m.num_blocks; a.max_pos = m.max_model_len;
     a.out = w.attn; a.part_o = w.part_o; a.part_ml = w.part_ml; a.tickets = w.tickets; a.status = h->status;
-    auto attn = paged_attention_ring_kernel<kAttnChunk>;
+    a.trace = L.next_trace();
+    auto attn = half ? paged_attention_ring_kernel<kAttnChunk / 2> : paged_attention_ring_kernel<kAttnChunk>;
     DFB_CUDA(ensure_dynamic_smem((const void*)attn, kRingSmemBytes));
     L.launch(attn, dim3(chunks), dim3(kRingThreads), a, true, kRingSmemBytes);
     launch_wide_store<2048, NG>(L, store(w.attn, lw.wo), m.hidden);
@@ -1228,23 +1231,28 @@ int enqueue_wide(DfbHandle* h, int chunks, bool sampling, cudaStream_t stream) {
   v.temps = sampling ? reinterpret_cast<const float*>(w.stage + 3 * kWideRows) : nullptr;
   launch_wide_norm<NG, kModeNormArgmax>(L, v, v.n_tiles < h->sm_count ? v.n_tiles : h->sm_count);
   if (L.err) return L.err;
+  h->kernels_per_step = h->trace_entries = L.count;
   publish_wide_kernel<<<1, 64, 0, stream>>>(w.tokens, h->status, w.host_tokens, w.seq);
   DFB_CUDA(cudaGetLastError());
   return 0;
 }
 
-// inputs of `rows` (9 to 32) rows are in wide.host_stage; returns when the tokens are in wide.host_tokens
-int wide_step(DfbHandle* h, int rows, int total_chunks, bool sampling, cudaStream_t stream) {
+// Inputs of `rows` (9 to 32) rows are in wide.host_stage: contexts of `halves` 32-position or `wholes` 64-position chunks.
+// A chunk is a serial walk for its CTA (1.1 us per 8 positions), so the shorter ones are taken while all of their CTAs
+// are resident together, two per SM (10 rows x 512: 903 against 1,000 us per step; 20 rows with 330 of them not).
+int wide_step(DfbHandle* h, int rows, int halves, int wholes, bool sampling, cudaStream_t stream) {
   DfbHandle::Wide& w = h->wide;
   const int groups = (rows + 7) / 8;
+  const bool half = halves <= 2 * h->sm_count;
+  const int total_chunks = half ? halves : wholes;
   int chunks = 64;                  // few grids, so that few graphs: the attention CTAs without a chunk leave at once
   while (chunks < total_chunks) chunks <<= 1;
   auto enqueue = [&](cudaStream_t s) {
-    return groups == 2 ? enqueue_wide<2>(h, chunks, sampling, s) : groups == 3 ? enqueue_wide<3>(h, chunks, sampling, s)
-                                                                                : enqueue_wide<4>(h, chunks, sampling, s);
+    return groups == 2 ? enqueue_wide<2>(h, chunks, half, sampling, s) : groups == 3 ? enqueue_wide<3>(h, chunks, half, sampling, s)
+                                                                                : enqueue_wide<4>(h, chunks, half, sampling, s);
   };
   if (h->use_graph) {
-    const int key = ((chunks * 8 + groups) * 2 + (sampling ? 1 : 0)) * 2 + (h->use_pdl ? 1 : 0);
+    const int key = (((chunks * 8 + groups) * 2 + (half ? 1 : 0)) * 2 + (sampling ? 1 : 0)) * 2 + (h->use_pdl ? 1 : 0);
     auto it = w.graphs.find(key);
     if (it == w.graphs.end()) {
       cudaGraph_t graph = nullptr;
@@ -1916,7 +1924,7 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
     int rc = wide_prepare(h);
     if (rc) return rc;
     int* hs = w.host_stage;
-    int chunks = 0;
+    int halves = 0, wholes = 0;
     bool sampled = false;
     for (int r = 0; r < kWideRows; ++r) {
       const bool on = r < n_live;
@@ -1929,10 +1937,10 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
       int* bt = hs + 4 * kWideRows + r * h->max_pages;
       const int cols = on ? (int)s->table.size() : 0;
       for (int c = 0; c < h->max_pages; ++c) bt[c] = c < cols ? s->table[c] : 0;
-      if (on) chunks += (int)(s->position / kAttnChunk) + 1;
+      if (on) { halves += (int)(s->position / (kAttnChunk / 2)) + 1; wholes += (int)(s->position / kAttnChunk) + 1; }
       sampled = sampled || t > 1e-10f;
     }
-    rc = wide_step(h, n_live, chunks, sampled, (cudaStream_t)stream);
+    rc = wide_step(h, n_live, halves, wholes, sampled, (cudaStream_t)stream);
     if (rc) return rc;
     if (!poll_published(w.host_tokens + kWideRows + 4, w.published)) DFB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     for (int r = 0; r < n_live; ++r) {

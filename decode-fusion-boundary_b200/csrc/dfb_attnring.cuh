@@ -352,7 +352,7 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
     *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16(o0[0] / l0, o0[1] / l0), pack_bf16(o0[2] / l0, o0[3] / l0));
     *reinterpret_cast<uint2*>(out + kHeadDim) = make_uint2(pack_bf16(o1[0] / l1, o1[1] / l1), pack_bf16(o1[2] / l1, o1[3] / l1));
   } else {
-    const size_t pidx = ((size_t)row * a.kv_heads + warp) * kMaxSplits;
+    const size_t pidx = ((size_t)row * a.kv_heads + warp) * (a.packed_rows ? kMaxSplits * kAttnChunk / CH : kMaxSplits);
     float* po = a.part_o + (pidx + split) * 2 * kHeadDim + 4 * lane;
     *reinterpret_cast<float4*>(po) = make_float4(o0[0], o0[1], o0[2], o0[3]);
     *reinterpret_cast<float4*>(po + kHeadDim) = make_float4(o1[0], o1[1], o1[2], o1[3]);
@@ -369,16 +369,30 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
     }
     last = __shfl_sync(0xffffffffu, last, 0);
     if (last) {
-      // lane s holds (max, sum) of chunk s for both heads; weights by shuffle, partial outputs 8 chunks at a time
-      float2 ml0 = make_float2(-INFINITY, 0.f), ml1 = make_float2(-INFINITY, 0.f);
-      if (lane < nsplits) {
-        ml0 = __ldcg(&a.part_ml[(pidx + lane) * 2]);
-        ml1 = __ldcg(&a.part_ml[(pidx + lane) * 2 + 1]);
+      // lane s holds (max, sum) of chunks s and (CH = 32, packed) s + 32 for both heads; weights by shuffle, partial
+      // outputs 8 chunks at a time
+      constexpr int W = CH < kAttnChunk ? 2 : 1;
+      float2 ml0[W], ml1[W];
+      float M0 = -INFINITY, M1 = -INFINITY, S0 = 0.f, S1 = 0.f, w0[W], w1[W];
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        ml0[i] = ml1[i] = make_float2(-INFINITY, 0.f);
+        if (lane + 32 * i < nsplits) {
+          ml0[i] = __ldcg(&a.part_ml[(pidx + lane + 32 * i) * 2]);
+          ml1[i] = __ldcg(&a.part_ml[(pidx + lane + 32 * i) * 2 + 1]);
+        }
+        M0 = fmaxf(M0, ml0[i].x);
+        M1 = fmaxf(M1, ml1[i].x);
       }
-      const float M0 = warp_max(ml0.x), M1 = warp_max(ml1.x);
-      const float w0 = lane < nsplits ? exp2f((ml0.x - M0) * kLog2e) : 0.f;
-      const float w1 = lane < nsplits ? exp2f((ml1.x - M1) * kLog2e) : 0.f;
-      const float S0 = warp_sum(w0 * ml0.y), S1 = warp_sum(w1 * ml1.y);
+      M0 = warp_max(M0); M1 = warp_max(M1);
+#pragma unroll
+      for (int i = 0; i < W; ++i) {
+        w0[i] = exp2f((ml0[i].x - M0) * kLog2e);      // no such chunk: exp2(-inf) = 0
+        w1[i] = exp2f((ml1[i].x - M1) * kLog2e);
+        S0 += w0[i] * ml0[i].y;
+        S1 += w1[i] * ml1[i].y;
+      }
+      S0 = warp_sum(S0); S1 = warp_sum(S1);
       float A0[4] = {0.f, 0.f, 0.f, 0.f}, A1[4] = {0.f, 0.f, 0.f, 0.f};
       const float* ps = a.part_o + pidx * 2 * kHeadDim + 4 * lane;
       for (int sb = 0; sb < nsplits; sb += 8) {
@@ -395,7 +409,8 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
         }
 #pragma unroll
         for (int u = 0; u < 8; ++u) {
-          const float x0 = __shfl_sync(0xffffffffu, w0, (sb + u) & 31), x1 = __shfl_sync(0xffffffffu, w1, (sb + u) & 31);
+          const float x0 = __shfl_sync(0xffffffffu, sb < 32 ? w0[0] : w0[W - 1], (sb + u) & 31);
+          const float x1 = __shfl_sync(0xffffffffu, sb < 32 ? w1[0] : w1[W - 1], (sb + u) & 31);
           A0[0] = fmaf(x0, pa[u].x, A0[0]); A0[1] = fmaf(x0, pa[u].y, A0[1]); A0[2] = fmaf(x0, pa[u].z, A0[2]); A0[3] = fmaf(x0, pa[u].w, A0[3]);
           A1[0] = fmaf(x1, pb[u].x, A1[0]); A1[1] = fmaf(x1, pb[u].y, A1[1]); A1[2] = fmaf(x1, pb[u].z, A1[2]); A1[3] = fmaf(x1, pb[u].w, A1[3]);
         }

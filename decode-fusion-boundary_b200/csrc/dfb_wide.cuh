@@ -4,17 +4,22 @@
 //   * wide_norm_kernel: QKV, gate / up and the LM head (K = 1024, residual add + RMSNorm in front), the layout of
 //     pair_gemv_kernel (16 weight rows on M, 8 batch rows on N, 8 warps splitting K): a weight fragment is read from shared
 //     memory once and multiplied with NG groups.  x stays in shared memory (8 NG rows), so that the kernel keeps
-//     within 128 registers and 170 KB and its CTAs start beside their predecessor's.
-//   * wide_store_kernel: o_proj and down_proj.  A cluster of two CTAs shares a tile of 16 weight rows, each with one half of
-//     K: x is by far the larger operand here (24 rows x 6 KB against 16 x 6 KB of weights per CTA), and halving K halves
-//     what a CTA has to fetch behind its dependency; all of it is in flight at once, in registers.  The halves meet in
-//     the peer's shared memory.
+//     within 128 registers and 170 KB and its CTAs start beside their predecessor's.  Clusters of four CTAs share the
+//     norm: each normalises a quarter of the rows and writes them into all four shared memories (every CTA reading
+//     all rows of h and of the residual took 14 MB from L2 in a launch; gate / up, 20 rows: 7.3 -> 5.9 us).
+//   * wide_store_kernel: o_proj and down_proj.  A cluster of four CTAs shares 32 weight rows, each with a quarter of K: x is
+//     by far the larger operand here (24 rows x 6 KB), and splitting K divides what a CTA has to fetch behind its
+//     dependency; all of it is in flight at once, in registers.  The parts meet in the shared memory of the CTA that
+//     finishes the row (down_proj, 20 rows, two CTAs: 5.1 us, four: 4.2 us).
 //
-// Bound by mma.sync's issue rate (one per 38 clocks and sub-partition: 0.35 us per group, tile of 48 rows and layer) and
+// 20 rows, 5 - 1,500 tokens: 1,066 us per step, of which attention 15 us per layer (paged_attention_ring_kernel on a packed
+// list of chunks), LM head 80 us.
+// Bound by mma.sync's issue rate (one per 38 clocks and sub-partition: 0.3 us per group and gate / up tile of 16 rows) and
 // by the latency of the dependent launches.  Rows beyond the live ones are computed and ignored.
 #pragma once
 
 #include "dfb_attncluster.cuh"
+#include "dfb_attnring.cuh"
 #include "dfb_kernels.cuh"
 #include "dfb_pairgemv.cuh"
 
@@ -22,6 +27,8 @@ namespace dfb {
 
 constexpr int kWideRows = 32;                        // = DFB_MAX_SLOTS
 constexpr int kKernelWide = 8;
+constexpr int kWideSplits = 2 * kMaxSplits;           // partial results of a row: chunks of 32 positions at least
+constexpr int kWideCluster = 4;                       // CTAs that share the norm (QKV, gate / up) or K (o_proj, down_proj)
 
 template <int NG, int MODE>
 struct WideSmem {
@@ -57,7 +64,10 @@ __global__ void __launch_bounds__(256, MODE == kModeNormArgmax ? 1 : 2) wide_nor
   using SM = WideSmem<NG, MODE>;
   constexpr int K = PairSmem::kK, STAGES = SM::kStages, kOut = 128 * NG;
   constexpr bool kArgmax = MODE == kModeNormArgmax, kSwiglu = MODE == kModeNormSwiglu;
+  constexpr int CL = kArgmax ? 1 : kWideCluster, kOwn = 8 * NG / CL;     // rows that this CTA normalises
   pdl_launch_dependents();
+  if (CL > 1) cluster_arrive_relaxed();      // completed before the peers' shared memory is written
+  if (threadIdx.x == 0) trace_min(a.trace, 0);
   extern __shared__ __align__(128) unsigned char dyn_smem[];
   unsigned char* stage_base = dyn_smem;
   unsigned char* xsb = dyn_smem + STAGES * PairSmem::kStageBytes;               // [8 NG][kRowStride] bf16 x
@@ -93,9 +103,11 @@ __global__ void __launch_bounds__(256, MODE == kModeNormArgmax ? 1 : 2) wide_nor
   for (int c = 0; c < 4; ++c) nw[c] = ldg_stream(a.norm_w + 8 * (32 * c + lane));
   __syncthreads();          // the barriers are initialised before anyone polls them
   pdl_wait();
+  if (tid == 0) { trace_max(a.trace, 1); trace_min(a.trace, 3); }
 
-  // ---- x = h (+ residual), RMSNorm: warp w owns rows w, w + 8, ...; the next row is in flight meanwhile ----
+  // ---- x = h (+ residual), RMSNorm: a warp per row; the rows are shared out over the cluster ----
   {
+    const int first = CL > 1 ? (blockIdx.x & (CL - 1)) * kOwn : 0;
     uint4 hv[4], rv[4];
     auto load = [&](int b) {
       const size_t xrow = a.ids ? (size_t)clamp_token(a.ids[b], a.embed_rows, a.status, b) : (size_t)b;
@@ -105,10 +117,12 @@ __global__ void __launch_bounds__(256, MODE == kModeNormArgmax ? 1 : 2) wide_nor
         rv[c] = a.res_in ? ldg_cg(a.res_in + (size_t)b * K + 8 * (32 * c + lane)) : make_uint4(0, 0, 0, 0);
       }
     };
-    load(warp);
+    if (warp < kOwn) load(first + warp);
+    if (CL > 1) cluster_wait();
 #pragma unroll
-    for (int i = 0; i < NG; ++i) {
-      const int b = warp + 8 * i;
+    for (int i = 0; i < (kOwn + 7) / 8; ++i) {
+      const int b = first + warp + 8 * i;
+      if (warp + 8 * i >= kOwn) break;
       float x[4][8], ss = 0.f;
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -118,8 +132,8 @@ __global__ void __launch_bounds__(256, MODE == kModeNormArgmax ? 1 : 2) wide_nor
 #pragma unroll
         for (int e = 0; e < 8; ++e) { x[c][e] = hf[e] + rf[e]; ss = fmaf(x[c][e], x[c][e], ss); }
       }
-      if (i + 1 < NG) load(b + 8);
-      if (a.res_out && (int)blockIdx.x == b) {      // one CTA per row
+      if (8 * (i + 1) + warp < kOwn) load(b + 8);
+      if (a.res_out && (int)blockIdx.x < CL) {
 #pragma unroll
         for (int c = 0; c < 4; ++c)
           *reinterpret_cast<uint4*>(a.res_out + (size_t)b * K + 8 * (32 * c + lane)) =
@@ -134,14 +148,28 @@ __global__ void __launch_bounds__(256, MODE == kModeNormArgmax ? 1 : 2) wide_nor
         unpack8(nw[c], wf);
 #pragma unroll
         for (int e = 0; e < 8; ++e) y[e] = round_bf16(x[c][e] * rstd) * wf[e];
-        *reinterpret_cast<uint4*>(xsb + b * PairSmem::kRowStride + 16 * (32 * c + lane)) =
-            make_uint4(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]), pack_bf16(y[4], y[5]), pack_bf16(y[6], y[7]));
+        const uint32_t y0 = pack_bf16(y[0], y[1]), y1 = pack_bf16(y[2], y[3]), y2 = pack_bf16(y[4], y[5]), y3 = pack_bf16(y[6], y[7]);
+        unsigned char* dst = xsb + b * PairSmem::kRowStride + 16 * (32 * c + lane);
+        if (CL == 1) {
+          *reinterpret_cast<uint4*>(dst) = make_uint4(y0, y1, y2, y3);
+        } else {
+#pragma unroll
+          for (int r = 0; r < CL; ++r)
+            asm volatile("st.shared::cluster.v4.b32 [%0], {%1,%2,%3,%4};"
+                         ::"r"(peer_smem(dst, r)), "r"(y0), "r"(y1), "r"(y2), "r"(y3) : "memory");
+        }
       }
     }
   }
   int sampled_groups = 0;
   if (kArgmax && warp == 0) sampled_groups = wide_sample_rows(a, srows, lane);
-  __syncthreads();
+  if (CL > 1) {
+    cluster_arrive();
+    cluster_wait();
+  } else {
+    __syncthreads();
+  }
+  if (tid == 0) trace_max(a.trace, 4);
 
   // ---- one tile: this warp's K columns of 16 weight rows x 8 NG batch rows; c = (row g | g + 8, batch 2t, 2t + 1) ----
   const unsigned char* xp = xsb + g * PairSmem::kRowStride + 2 * kbase;
@@ -198,6 +226,7 @@ __global__ void __launch_bounds__(256, MODE == kModeNormArgmax ? 1 : 2) wide_nor
       }
     }
     __syncthreads();
+    if (tid == 0) trace_max(a.trace, 5);
 #pragma unroll
     for (int s = 0; s < STAGES; ++s)
       if (s < nt) park(reinterpret_cast<float*>(stage_base + s * PairSmem::kStageBytes), c[s]);
@@ -294,101 +323,97 @@ __global__ void __launch_bounds__(256, MODE == kModeNormArgmax ? 1 : 2) wide_nor
 #pragma unroll 1
     for (int s = 0; s < STAGES; ++s) mbar_wait_bounded(&full[s], 0);
   }
+  if (tid == 0) trace_max(a.trace, 2);
 }
 
-// out[8 NG, N] = x[8 NG, K] @ W[N, K]^T: clusters of two CTAs, 16 weight rows each pair, one half of K per CTA
+// out[8 NG, N] = x[8 NG, K] @ W[N, K]^T: clusters of four CTAs, 32 weight rows each cluster, a quarter of K per CTA
 template <int K, int NG>
 struct WideStoreSmem {
-  static constexpr int kHalf = K / 2, kRowStride = 2 * kHalf + 64;      // (+ 64: conflict-free fragment reads)
-  static constexpr int kRed = 8 * 128 * NG;
-  static constexpr int bytes() { return 16 * kRowStride + 4 * kRed + 4 * 64 * NG + 16; }
+  static constexpr int kPart = K / kWideCluster, kRowStride = 2 * kPart + 64;      // (+ 64: conflict-free fragment reads)
+  static constexpr int kOut = 256 * NG;                                           // outputs: group x 256 + row x 8 + batch row
+  static constexpr int bytes() { return 32 * kRowStride + 4 * 8 * kOut + 4 * kOut + 16; }
 };
 template <int K, int NG>
 __global__ void __launch_bounds__(256, 2) wide_store_kernel(const GemvArgs a) {
   using SM = WideStoreSmem<K, NG>;
-  constexpr int LJ = SM::kHalf / 256, kOut = 128 * NG;       // 32-column blocks of a warp
+  constexpr int LJ = SM::kPart / 256, kOut = SM::kOut;       // LJ: 32-column blocks of a warp
   pdl_launch_dependents();
-  cluster_arrive_relaxed();      // completed before the peer's shared memory is written: it is running by then
+  if (threadIdx.x == 0) trace_min(a.trace, 0);
+  cluster_arrive_relaxed();      // completed before a peer's shared memory is written: it is running by then
   extern __shared__ __align__(128) unsigned char dyn_smem[];
-  float* red = reinterpret_cast<float*>(dyn_smem + 16 * SM::kRowStride);
-  float* recv = red + SM::kRed;                              // the peer's half of this CTA's outputs
-  uint64_t* full = reinterpret_cast<uint64_t*>(recv + 64 * NG);
+  float* red = reinterpret_cast<float*>(dyn_smem + 32 * SM::kRowStride);      // [warp][output]
+  float* recv = red + 8 * kOut;                              // [source CTA][64 NG]: partial sums of the rows this CTA finishes
+  uint64_t* full = reinterpret_cast<uint64_t*>(recv + kOut);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
-  const int tile = blockIdx.x >> 1, rank = blockIdx.x & 1, kbase = warp * (32 * LJ) + 8 * t;
+  const int tile = blockIdx.x / kWideCluster, rank = blockIdx.x % kWideCluster, kbase = warp * (32 * LJ) + 8 * t;
   if (warp == 0) {
     if (lane == 0) {
       mbar_init(full, 1);
       fence_mbar_init();
-      mbar_expect_tx(full, 16 * 2 * SM::kHalf);
+      mbar_expect_tx(full, 32 * 2 * SM::kPart);
     }
     __syncwarp();
-    if (lane < 16)
-      bulk_g2s(dyn_smem + lane * SM::kRowStride, a.w + (size_t)(tile * 16 + lane) * K + rank * SM::kHalf, 2 * SM::kHalf, full);
+    bulk_g2s(dyn_smem + lane * SM::kRowStride, a.w + (size_t)(tile * 32 + lane) * K + rank * SM::kPart, 2 * SM::kPart, full);
   }
   __syncthreads();
   pdl_wait();
+  if (tid == 0) { trace_max(a.trace, 1); trace_min(a.trace, 3); }
 
   uint4 xb[NG][LJ];
-  const __nv_bfloat16* xp = a.x + (size_t)g * K + rank * SM::kHalf + kbase;
+  const __nv_bfloat16* xp = a.x + (size_t)g * K + rank * SM::kPart + kbase;
 #pragma unroll
   for (int n = 0; n < NG; ++n)
 #pragma unroll
     for (int j = 0; j < LJ; ++j) xb[n][j] = ldg_cg(xp + (size_t)(8 * n) * K + 32 * j);
   const bool copy_ok = mbar_wait_bounded(full, 0);
-  const unsigned char* w0p = dyn_smem + g * SM::kRowStride + 2 * kbase;
-  const unsigned char* w1p = w0p + 8 * SM::kRowStride;
-  float c[NG][4], d[NG][4];
+  float c[2][NG][4];
 #pragma unroll
-  for (int n = 0; n < NG; ++n)
+  for (int h = 0; h < 2; ++h)
 #pragma unroll
-    for (int q = 0; q < 4; ++q) { c[n][q] = 0.f; d[n][q] = 0.f; }
+    for (int n = 0; n < NG; ++n)
 #pragma unroll
-  for (int j = 0; j < LJ; ++j) {
-    const uint4 u = *reinterpret_cast<const uint4*>(w0p + 64 * j), v = *reinterpret_cast<const uint4*>(w1p + 64 * j);
+      for (int q = 0; q < 4; ++q) c[h][n][q] = 0.f;
 #pragma unroll
-    for (int n = 0; n < NG; ++n) {
-      mma_bf16_16816_full(c[n], u.x, v.x, u.y, v.y, xb[n][j].x, xb[n][j].y);
-      mma_bf16_16816_full(d[n], u.z, v.z, u.w, v.w, xb[n][j].z, xb[n][j].w);
-    }
-  }
-  float* r = red + warp * kOut + g * 8 + 2 * t;
+  for (int j = 0; j < LJ; ++j)
 #pragma unroll
-  for (int n = 0; n < NG; ++n) {
-    *reinterpret_cast<float2*>(r + 128 * n) = make_float2(c[n][0] + d[n][0], c[n][1] + d[n][1]);
-    *reinterpret_cast<float2*>(r + 128 * n + 64) = make_float2(c[n][2] + d[n][2], c[n][3] + d[n][3]);
-  }
-  __syncthreads();
-  cluster_wait();
-  // CTA `rank` finishes tile rows 8 rank ... 8 rank + 7; output of a group = row x 8 + batch row
-  float mine[(64 * NG + 255) / 256];
+    for (int h = 0; h < 2; ++h) {
+      const unsigned char* wp = dyn_smem + (16 * h + g) * SM::kRowStride + 2 * kbase + 64 * j;
+      const uint4 u = *reinterpret_cast<const uint4*>(wp), v = *reinterpret_cast<const uint4*>(wp + 8 * SM::kRowStride);
 #pragma unroll
-  for (int h = 0; h < (kOut + 255) / 256; ++h) {
-    const int o = tid + 256 * h;
-    if (o < kOut) {
-      float v = 0.f;
-#pragma unroll
-      for (int w = 0; w < 8; ++w) v += red[w * kOut + o];
-      const int n = o >> 7, q = o & 127, p = 64 * n + (q & 63);
-      if ((q >> 6) != rank) {
-        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(peer_smem(recv + p, rank ^ 1)), "f"(v) : "memory");
-      } else {
-        red[o] = v;             // (only this thread reads column o of warp 0's sums)
+      for (int n = 0; n < NG; ++n) {
+        mma_bf16_16816_full(c[h][n], u.x, v.x, u.y, v.y, xb[n][j].x, xb[n][j].y);
+        mma_bf16_16816_full(c[h][n], u.z, v.z, u.w, v.w, xb[n][j].z, xb[n][j].w);
       }
     }
+  float* r = red + warp * kOut + g * 8 + 2 * t;
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int n = 0; n < NG; ++n) {
+      *reinterpret_cast<float2*>(r + 256 * n + 128 * h) = make_float2(c[h][n][0], c[h][n][1]);
+      *reinterpret_cast<float2*>(r + 256 * n + 128 * h + 64) = make_float2(c[h][n][2], c[h][n][3]);
+    }
+  __syncthreads();
+  if (tid == 0) trace_max(a.trace, 5);
+  cluster_wait();
+  // thread: row tid / 8 of the tile, batch row tid % 8 of every group; CTA row / 8 of the cluster finishes it
+#pragma unroll
+  for (int n = 0; n < NG; ++n) {
+    float v = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) v += red[w * kOut + 256 * n + tid];
+    asm volatile("st.shared::cluster.f32 [%0], %1;"
+                 ::"r"(peer_smem(recv + rank * 64 * NG + 64 * n + (tid & 63), tid >> 6)), "f"(v) : "memory");
   }
   cluster_arrive();
   cluster_wait();
-#pragma unroll
-  for (int h = 0; h < (64 * NG + 255) / 256; ++h) {
-    const int p = tid + 256 * h;
-    if (p < 64 * NG) {
-      const int n = p >> 6, q = p & 63;
-      const float own = red[128 * n + 64 * rank + q], other = recv[p];
-      mine[h] = rank ? other + own : own + other;
-      a.out[(size_t)(8 * n + (q & 7)) * a.out_stride + tile * 16 + 8 * rank + (q >> 3)] = __float2bfloat16_rn(mine[h]);
-    }
+  if (tid < 64 * NG) {
+    const int n = tid >> 6, q = tid & 63;
+    const float v = (recv[tid] + recv[64 * NG + tid]) + (recv[2 * 64 * NG + tid] + recv[3 * 64 * NG + tid]);
+    a.out[(size_t)(8 * n + (q & 7)) * a.out_stride + tile * 32 + 8 * rank + (q >> 3)] = __float2bfloat16_rn(v);
   }
   if (!copy_ok) report_status(a.status, kStatusCopyTimeout, kKernelWide, blockIdx.x, kModeStore);
+  if (tid == 0) trace_max(a.trace, 2);
 }
 
 // Tokens and status of a wide step into pinned host memory, followed by the sequence word (see publish_result_kernel).
