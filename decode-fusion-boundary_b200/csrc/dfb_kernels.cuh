@@ -1024,6 +1024,8 @@ __global__ void __launch_bounds__(256) store_kvcache_kernel(const unsigned char*
                                                             unsigned char* __restrict__ k_cache, unsigned char* __restrict__ v_cache,
                                                             const int* __restrict__ slot_mapping, int n_tokens, int row_bytes,
                                                             long long num_slots, int* status) {
+  pdl_launch_dependents();
+  pdl_wait();
   const int half = threadIdx.x >> 7, t = threadIdx.x & 127;
   const unsigned char* src = half ? value : key;
   unsigned char* dst = half ? v_cache : k_cache;

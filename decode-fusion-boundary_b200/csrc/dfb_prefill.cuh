@@ -60,6 +60,8 @@ __device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], const void* 
 
 __global__ void __launch_bounds__(128) prefill_short_kernel(const PrefillShortArgs a) {
   extern __shared__ __align__(128) unsigned char pf_smem[];
+  pdl_launch_dependents();
+  pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   const int seq = blockIdx.z, head = blockIdx.y;

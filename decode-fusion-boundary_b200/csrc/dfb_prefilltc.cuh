@@ -252,6 +252,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_launch_dependents();
   if (warp == 10 && lane < 3) {
     const CUtensorMap* map = lane == 0 ? &a.q_map : lane == 1 ? &a.k_map : &a.v_map;
     asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
@@ -272,6 +273,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "n"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  pdl_wait();      // nothing above reads what an earlier kernel wrote
   PfWalk<PAIRS> walk;
   walk.init(a, lane);
   tc_fence_before();
