@@ -111,7 +111,7 @@ struct ChainOptions {
                                // measured slower at every batch (batch 8 / context 512: 758 us with bit 1, 719 with
                                // bit 2, 786 with both, against 709): at 2-8 rows a successor that streams its
                                // weights beside the running kernel takes bandwidth from that kernel's own stream
-  int host_io = env_int("DFB_HOST_IO", 6);   // steps from host buffers: 1 = the inputs reach the staging area by a one-warp
+  int host_io = env_int("DFB_HOST_IO", 7);   // steps from host buffers: 1 = the inputs reach the staging area by a one-warp
                                // kernel that reads pinned host memory, 2 = tokens and status are written to pinned
                                // host memory by a one-warp kernel, instead of copy nodes in the step's graph; 4 = the
                                // host then polls the sequence word that follows the tokens into pinned memory
@@ -232,13 +232,15 @@ struct Launcher {
   const void* ahead_ptr = nullptr;        // look-ahead request the next launched kernel carries (cleared by it)
   unsigned long long ahead_bytes = 0;
   bool ahead_late = false;
+  bool late_trigger = false;              // the next projection lets its successor start only behind its own dependency
   int embed_rows = 0;                     // rows of the embedding table when a kernel gathers by token id
   bool plain_next = false;  // the next launch follows a foreign kernel (a collective): no programmatic dependency
   unsigned long long* next_trace() const { return trace ? trace + 8 * count : nullptr; }
   // what every GEMV launch of a step carries: the pending look-ahead request and the embedding row count
   void fill_common(GemvArgs& a) {
     a.ahead_ptr = ahead_ptr; a.ahead_bytes = ahead_bytes; a.ahead_late = ahead_late ? 1 : 0; a.embed_rows = embed_rows;
-    a.late_trigger = opt->late_trigger;
+    a.late_trigger = opt->late_trigger || late_trigger;
+    late_trigger = false;
     ahead_ptr = nullptr; ahead_bytes = 0;
   }
   template <typename Args>
@@ -573,7 +575,6 @@ void launch_row_nb(Launcher& L, GemvArgs& a, int grid, bool allow_pdl) {
     cudaError_t e = ensure_dynamic_smem((const void*)kernel, smem);
     if (e != cudaSuccess) { L.err = (int)e; return; }
   }
-  a.late_trigger = L.opt->late_trigger;
   a.bulk_x = L.opt->bulk_x;
   L.fill_common(a);
   // The down projection has one CTA per SM's worth of work (128 CTAs): asking for at
@@ -908,7 +909,7 @@ int split_bucket(const DfbHandle* h, int max_context, int rows) {
 // memory as soon as it is resident, i.e. while kernel i runs; its CTAs that only
 // fit on the SMs after kernel i has ended, and everything its first tiles do not
 // cover, would otherwise start their HBM round trip after the dependency.
-int enqueue_step(DfbHandle* h, int rows, int nsplit, int bt_cols, cudaStream_t stream, float* logits_out) {
+int enqueue_step(DfbHandle* h, int rows, int nsplit, int bt_cols, cudaStream_t stream, float* logits_out, bool staged) {
   const DfbModelDesc& m = h->m;
   Launcher L{stream, h->use_pdl, h->trace_on ? h->trace : nullptr};
   L.opt = &h->opt;
@@ -943,9 +944,11 @@ int enqueue_step(DfbHandle* h, int rows, int nsplit, int bt_cols, cudaStream_t s
     want(4, w.wgu, b_gu);
     if (l == 0) {
       // embedding rows are gathered by token id; the residual starts as the embedding itself.
-      // No PDL on the first kernel: it must observe the staged inputs of this step.
+      // Behind a staging kernel it is a dependent launch as well (its weights are requested meanwhile), but it lets the
+      // attention kernel start only once the inputs are there: that one reads positions and block tables at once.
+      L.late_trigger = staged;
       rc = launch_norm_qkv(L, (const bf16*)m.embed, h->st_ids(), nullptr, h->res[cur], (const bf16*)w.ln_in,
-                           (const bf16*)w.wqkv, h->qkv, rows, m.hidden, h->qkv_rows(), m.eps, h->status, false);
+                           (const bf16*)w.wqkv, h->qkv, rows, m.hidden, h->qkv_rows(), m.eps, h->status, staged);
     } else {
       rc = launch_norm_qkv(L, h->hbuf, nullptr, h->res[cur], h->res[cur ^ 1], (const bf16*)w.ln_in,
                            (const bf16*)w.wqkv, h->qkv, rows, m.hidden, h->qkv_rows(), m.eps, h->status, true);
@@ -1013,6 +1016,7 @@ struct StepIo {
 
 int enqueue_whole_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, cudaStream_t stream,
                        float* logits_out) {
+  const bool staged = !io.burst && ((io.host && (h->opt.host_io & 1)) || (!io.host && io.stage));      // by a kernel
   if (io.burst) {
     // staged by the burst's one host-to-device copy, advanced on the device from step to step
   } else if (io.host && (h->opt.host_io & 1)) {
@@ -1027,7 +1031,7 @@ int enqueue_whole_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const St
   if (io.sampling && h->step_mode == 1) return DFB_E_BAD_ARG;   // the persistent kernel's LM head is greedy only
   h->lm_temps = io.sampling ? h->st_temps() : nullptr;
   int rc = h->step_mode == 1 ? enqueue_persistent(h, rows, stream, logits_out)
-                             : enqueue_step(h, rows, nsplit, bt_cols, stream, logits_out);
+                             : enqueue_step(h, rows, nsplit, bt_cols, stream, logits_out, staged);
   h->lm_temps = nullptr;
   if (rc) return rc;
   if (io.burst) {
@@ -1035,8 +1039,8 @@ int enqueue_whole_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const St
     p.tokens = h->tokens; p.status = h->status; p.ids_out = h->st_ids(); p.positions_out = h->st_pos();
     p.rows = rows; p.embed_rows = h->embed_rows(); p.slot = h->burst_slot;
     p.ring = h->burst_ring; p.ring_status = h->burst_status(); p.ring_done = h->burst_done();
-    publish_tokens_kernel<<<1, 32, 0, stream>>>(p);
-    DFB_CUDA(cudaGetLastError());
+    if (h->use_pdl && !h->sharded() && h->step_mode == 0) DFB_CUDA(launch_overlapped(publish_tokens_kernel, dim3(1), dim3(32), 0, stream, p));
+    else DFB_CUDA((publish_tokens_kernel<<<1, 32, 0, stream>>>(p), cudaGetLastError()));
   } else if (io.publish || (io.host && (h->opt.host_io & 2))) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(1); cfg.blockDim = dim3(32); cfg.stream = stream;

@@ -990,6 +990,7 @@ struct StageArgs {
   int* status;
 };
 __global__ void stage_inputs_kernel(const StageArgs a) {
+  pdl_launch_dependents();
   const int tid = threadIdx.x;
   if (tid < a.rows) {
     long long id = a.ids ? (long long)a.ids[tid] : (long long)a.prev_tokens[tid];
@@ -1063,6 +1064,7 @@ __global__ void __launch_bounds__(256) store_kvcache_kernel(const unsigned char*
 // mappings are the host allocations themselves under unified addressing).  A copy node of a CUDA graph costs
 // more than a one-warp kernel for these few hundred bytes.
 __global__ void copy_ints_kernel(const int* __restrict__ src, int* __restrict__ dst, int n) {
+  pdl_launch_dependents();
   for (int i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
 }
 // `seq` (device) counts the steps published; its new value follows the data into host_out[n], after a
@@ -1101,6 +1103,7 @@ struct PublishArgs {
 };
 __global__ void publish_tokens_kernel(const PublishArgs a) {
   const int tid = threadIdx.x;
+  pdl_wait();   // launched with a programmatic dependency on the LM head
   const unsigned slot = *a.slot;
   if (tid < a.rows) {
     const int tok = a.tokens[tid];
