@@ -1706,7 +1706,8 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
   // per SM (16 prompts of 64: 6.7 against 9.3 us; 16 of 128 no longer: 13.3 against 9.6).
   const int64_t short_ctas = (int64_t)batch * ((max_seqlen_q + kPfTile - 1) / kPfTile) * q_heads;
   const int sms = sm_count_cached();
-  if (!block_tables && max_seqlen_q <= (short_ctas <= sms ? 384 : 128) && short_ctas <= 3 * sms) {
+  static const int want_short = env_int("DFB_PF_SHORT", 384);
+  if (!block_tables && max_seqlen_q <= (short_ctas <= sms ? want_short : 128) && short_ctas <= 3 * sms) {
     const void* fn = (const void*)prefill_short_kernel;
     cudaError_t e = ensure_dynamic_smem(fn, kPfShortSmemBytes);
     if (e != cudaSuccess) return (int)e;
@@ -1721,8 +1722,12 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
     return 0;
   }
   // query heads that share a KV head go in pairs where their number allows it
-  const bool pairs = (q_heads / kv_heads) % 2 == 0;
-  auto kernel = block_tables ? (pairs ? prefill_tc_kernel<true, true> : prefill_tc_kernel<true, false>)
+  // few and short prompts: one head per CTA and the keys split over its two tiles, while every CTA has at most one item
+  const int64_t split_items = (int64_t)batch * ((max_seqlen_q + kPfRows - 1) / kPfRows) * q_heads;
+  static const int want_split = env_int("DFB_PF_SPLIT", 1);
+  const bool split = !block_tables && split_items <= sms && want_split;
+  const bool pairs = !split && (q_heads / kv_heads) % 2 == 0;
+  auto kernel = split ? prefill_tc_kernel<false, false, true> : block_tables ? (pairs ? prefill_tc_kernel<true, true> : prefill_tc_kernel<true, false>)
                              : (pairs ? prefill_tc_kernel<false, true> : prefill_tc_kernel<false, false>);
   cudaError_t e = ensure_dynamic_smem((const void*)kernel, kPfSmemBytes);
   if (e != cudaSuccess) return (int)e;
@@ -1745,7 +1750,7 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
   if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, any_rows, v_stride, 8, &a.v_map8);
   if (rc) return rc;
   // one CTA per SM (all of its tensor memory), fewer when the longest sequence bounds the work items below that
-  const int64_t rows = pairs ? kPfRows : 2 * kPfRows;
+  const int64_t rows = pairs || split ? kPfRows : 2 * kPfRows;
   const int64_t most = (int64_t)batch * ((max_seqlen_q + rows - 1) / rows) * (pairs ? q_heads / 2 : q_heads);
   const int grid = (int)(most < sm_count_cached() ? most : sm_count_cached());
   DFB_CUDA(launch_overlapped(kernel, dim3(grid), dim3(kPfThreads), kPfSmemBytes, (cudaStream_t)stream, a));

@@ -161,9 +161,9 @@ struct PfItem {
   int seq_start, seq_len, k_start, k_len, shift;
   int n_tiles;             // key tiles
 };
-template <bool PAIRS>
+template <bool PAIRS, bool SPLIT>
 struct PfWalk {
-  static constexpr int step = PAIRS ? 1 : 2;      // M tiles along the sequence in one item
+  static constexpr int step = PAIRS || SPLIT ? 1 : 2;      // M tiles along the sequence in one item
   int level, base, heads;
   // lane b's sequence: queries, keys, and their first rows (batches above 32 read them again as they go)
   int q_first, q_len, k_first, k_len;
@@ -206,7 +206,7 @@ struct PfWalk {
         int first, blocks;
         geometry(first, blocks);
         const int d = level - first;
-        const bool has = d >= 0 && (PAIRS || (d & 1) == 0) && d / step < blocks;
+        const bool has = d >= 0 && (step == 1 || (d & 1) == 0) && d / step < blocks;
         const unsigned mask = __ballot_sync(0xffffffffu, has);
         const bool mine = has && base + count + __popc(mask & ((1u << lane) - 1u)) == row;
         const unsigned hit = __ballot_sync(0xffffffffu, mine);
@@ -232,7 +232,10 @@ struct PfWalk {
 // item of CTA `cta` in round r: rounds alternate direction, so that nobody always gets the longer one
 __device__ __forceinline__ int pf_item_index(int r, int cta, int ctas) { return r * ctas + ((r & 1) ? ctas - 1 - cta : cta); }
 
-template <bool PAGED, bool PAIRS>
+// SPLIT (fresh keys, chosen while there is an SM for every item): an item is 128 query rows of ONE head, and tile t takes the key
+// tiles 2 i + t: half as long a chain for the few CTAs of a short batch.  The tiles exchange 64 columns of O each and
+// write the columns that they have merged.
+template <bool PAGED, bool PAIRS, bool SPLIT = false>
 __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_constant__ PrefillArgs a) {
   extern __shared__ unsigned char pf_raw[];
   const uint32_t raw = smem_u32(pf_raw);
@@ -259,7 +262,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
   }
   if (tid == 0) {
 #pragma unroll
-    for (int s = 0; s < kPfStages; ++s) { mbar_init(&full[s], 32); mbar_init(&empty[s], 2); }
+    for (int s = 0; s < kPfStages; ++s) { mbar_init(&full[s], 32); mbar_init(&empty[s], SPLIT ? 1 : 2); }
     mbar_init(q_full, 32);
     mbar_init(q_empty, 2);
 #pragma unroll
@@ -274,7 +277,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();      // nothing above reads what an earlier kernel wrote
-  PfWalk<PAIRS> walk;
+  static_assert(!SPLIT || (!PAGED && !PAIRS), "the split form takes fresh keys, one head at a time");
+  PfWalk<PAIRS, SPLIT> walk;
   walk.init(a, lane);
   tc_fence_before();
   __syncthreads();
@@ -292,7 +296,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
     constexpr uint32_t idesc_s = tc_idesc(128, kPfKeys);
     constexpr uint32_t idesc_o = tc_idesc(128, 128) | (1u << 16);    // B (= V) is MN-major
     const int t = __shfl_sync(0xffffffffu, warp - 8, 0);
-    const uint64_t qd = tc_smem_desc(smem_u32(qs) + t * kPfQBytes), kd = tc_smem_desc(smem_u32(ring)),
+    const uint64_t qd = tc_smem_desc(smem_u32(qs) + (SPLIT ? 0 : t) * kPfQBytes), kd = tc_smem_desc(smem_u32(ring)),
                    vd = tc_smem_desc_mn(smem_u32(ring), kPfTileBytes / 2);
     const uint32_t o_tmem = tmem + 128 * t, s_tmem = tmem + 256 + 128 * t;
     auto wait = [&](uint64_t* bar, uint32_t parity) -> bool {
@@ -326,24 +330,25 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
       }
     };
     int n = 0;                        // ring tiles consumed
+    auto place = [&](int e) -> int { return SPLIT ? 2 * e + t : e; };      // ... their place in the loader's order
     int g = 0;                        // key tiles done: buffer g & 1, phase g >> 1
     for (int r = 0; ok && walk.find(a, pf_item_index(r, cta, ctas), lane, it); ++r) {
-      const int n_tiles = __shfl_sync(0xffffffffu, it.n_tiles, 0);
+      const int n_tiles = __shfl_sync(0xffffffffu, SPLIT ? (it.n_tiles + 1) / 2 : it.n_tiles, 0);
       ok = wait(q_full, r & 1);
       for (int j = 0; ok && j < 2 && j < n_tiles; ++j, ++n) {
-        ok = wait(&full[n % kPfStages], (n / kPfStages) & 1);
-        if (ok) issue_s((g + j) & 1, n % kPfStages, j + 1 == n_tiles);
+        ok = wait(&full[place(n) % kPfStages], (place(n) / kPfStages) & 1);
+        if (ok) issue_s((g + j) & 1, place(n) % kPfStages, j + 1 == n_tiles);
       }
       for (int j = 0; ok && j < n_tiles; ++j, ++g) {
         const int b = g & 1;
-        ok = wait(&full[n % kPfStages], (n / kPfStages) & 1) && wait(&p_full[2 * t + b], (g >> 1) & 1);
+        ok = wait(&full[place(n) % kPfStages], (place(n) / kPfStages) & 1) && wait(&p_full[2 * t + b], (g >> 1) & 1);
         if (!ok) break;
-        issue_o(b, n % kPfStages, j == 0, j + 1 == n_tiles);
+        issue_o(b, place(n) % kPfStages, j == 0, j + 1 == n_tiles);
         ++n;
         if (j + 2 < n_tiles) {
-          ok = wait(&full[n % kPfStages], (n / kPfStages) & 1);
+          ok = wait(&full[place(n) % kPfStages], (place(n) / kPfStages) & 1);
           if (!ok) break;
-          issue_s(b, n % kPfStages, j + 3 == n_tiles);
+          issue_s(b, place(n) % kPfStages, j + 3 == n_tiles);
           ++n;
         }
       }
@@ -353,7 +358,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
       *abort_flag = 1;
     } else if (n > 0) {
       // the last commit has to land before the CTA's shared memory goes away
-      tc_wait(&empty[(n - 1) % kPfStages], ((n - 1) / kPfStages) & 1, abort_flag);
+      tc_wait(&empty[place(n - 1) % kPfStages], (place(n - 1) / kPfStages) & 1, abort_flag);
     }
     __syncwarp();
   } else if (warp == 10) {
@@ -406,7 +411,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
       const long long stride = is_v ? a.v_stride : a.k_stride;
       if (!wait_free(&empty[stage], ((n / kPfStages) & 1) ^ 1)) return false;
       const uint32_t base = smem_u32(ring) + stage * kPfTileBytes;
-      const int rows = min(it.k_len - p0, kPfKeys);
+      const int rows = max(min(it.k_len - p0, kPfKeys), 0);      // (split form: none in the last tile of an odd number)
       const CUtensorMap* map = is_v ? &a.v_map : &a.k_map;
       // one run of rows: fresh projections, or a cache whose blocks hold whole tiles
       if (!PAGED || a.box_rows == kPfKeys) {
@@ -485,10 +490,10 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
       if (!wait_free(q_empty, (r & 1) ^ 1)) { ok = false; break; }
       const bool q_boxes = it.seq_start + it.q0 + walk.step * kPfRows <= all_q;
       if (q_boxes) {
-        if (lane == 0) mbar_expect_tx(q_full, 2 * kPfQBytes);
+        if (lane == 0) mbar_expect_tx(q_full, (SPLIT ? 1 : 2) * kPfQBytes);
         else tc_mbar_arrive(q_full);
         __syncwarp();
-        if (lane < 4) {                                     // lane 2 t + h: half h of tile t
+        if (lane < (SPLIT ? 2 : 4)) {                                     // lane 2 t + h: half h of tile t
           const int t = lane >> 1, h = lane & 1;
           tma_load_2d(smem_u32(qs) + t * kPfQBytes + h * (kPfQBytes / 2), &a.q_map,
                       (PAIRS ? 2 * it.head + t : it.head) * kHeadDim + 64 * h, it.seq_start + it.q0 + (PAIRS ? 0 : t * kPfRows),
@@ -496,7 +501,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
         }
       } else {
 #pragma unroll 1
-        for (int t = 0; t < 2; ++t) {
+        for (int t = 0; t < (SPLIT ? 1 : 2); ++t) {
           // (rows past the end keep what was there: their results are not stored and touch no other row)
           const int first = it.q0 + (PAIRS ? 0 : t * kPfRows), rows = max(0, min(it.seq_len - first, kPfRows));
           const int x = (PAIRS ? 2 * it.head + t : it.head) * kHeadDim, y = it.seq_start + first;
@@ -505,10 +510,20 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
         push(q_full);
       }
       // in the order the issuer consumes them: K0 K1 V0 K2 V1 K3 ...
-      ok = load_tile(false, 0, kvh) && (it.n_tiles < 2 || load_tile(false, 1, kvh));
-      for (int j = 0; ok && j < it.n_tiles; ++j) {
-        ok = load_tile(true, j, kvh) && (j + 2 >= it.n_tiles || load_tile(false, j + 2, kvh));
-        if (j == 0) drain();      // the item's start waits for nothing further to be issued
+      if constexpr (SPLIT) {
+        const int own = (it.n_tiles + 1) / 2;
+        auto both = [&](bool is_v, int i) -> bool { return load_tile(is_v, 2 * i, kvh) && load_tile(is_v, 2 * i + 1, kvh); };
+        ok = both(false, 0) && (own < 2 || both(false, 1));
+        for (int j = 0; ok && j < own; ++j) {
+          ok = both(true, j) && (j + 2 >= own || both(false, j + 2));
+          if (j == 0) drain();
+        }
+      } else {
+        ok = load_tile(false, 0, kvh) && (it.n_tiles < 2 || load_tile(false, 1, kvh));
+        for (int j = 0; ok && j < it.n_tiles; ++j) {
+          ok = load_tile(true, j, kvh) && (j + 2 >= it.n_tiles || load_tile(false, j + 2, kvh));
+          if (j == 0) drain();      // the item's start waits for nothing further to be issued
+        }
       }
     }
     drain();
@@ -521,11 +536,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
     const float sl2 = a.scale * 1.4426950408889634f;       // scores in units of log2 e
     int g = 0;
     for (int r = 0; ok && walk.find(a, pf_item_index(r, cta, ctas), lane, it); ++r) {
-      const int row = it.q0 + (PAIRS ? 0 : t * kPfRows) + lrow;               // query row inside the sequence
+      const int row = it.q0 + (PAIRS || SPLIT ? 0 : t * kPfRows) + lrow;               // query row inside the sequence
       const int seen = min(it.shift + row + 1, it.k_len);                     // keys this row attends to
       const int clear = min(it.shift + row - lrow + 1, it.k_len);             // ... that every row of the tile attends to
       float m = 0.f, l = 0.f;
-      for (int j = 0; j < it.n_tiles; ++j, ++g) {
+      const int own = SPLIT ? (it.n_tiles + 1) / 2 : it.n_tiles;
+      for (int j = 0; j < own; ++j, ++g) {
         const int b = g & 1;
         ok = __all_sync(0xffffffffu, tc_wait(&s_full[2 * t + b], (g >> 1) & 1, abort_flag));
         if (!ok) break;
@@ -534,7 +550,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
         tc_ld32(s_addr + 64 * b, s);
         tc_ld32(s_addr + 64 * b + 32, s + 32);
         tc_wait_ld();
-        const int p0 = j * kPfKeys;
+        const int p0 = (SPLIT ? 2 * j + t : j) * kPfKeys;
         if (p0 + kPfKeys > clear) {       // the same for every thread of the tile
 #pragma unroll
           for (int i = 0; i < kPfKeys; ++i) s[i] = p0 + i < seen ? s[i] : -INFINITY;
@@ -546,7 +562,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
           for (int u = 0; u < 4; ++u) mx[u] = i + 4 + u < kPfKeys ? fmax3(mx[u], s[i + u], s[i + 4 + u]) : fmaxf(mx[u], s[i + u]);
         const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
         if (j == 0) {
-          m = mt;                          // key 0 is visible to every row: finite
+          m = mt;                          // key 0 is visible to every row: finite (split form, odd tiles: or -inf)
         } else {
           const bool grow = mt > m + kPfRescale;
           if (__any_sync(0xffffffffu, grow)) {
@@ -554,7 +570,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
             ok = __all_sync(0xffffffffu, tc_wait(&pv_done[t], (g - 1) & 1, abort_flag));
             if (!ok) break;
             tc_fence_after();
-            const float nm = grow ? mt : m, f = ex2_approx(m - nm);
+            const float nm = grow ? mt : m, f = SPLIT && m == -INFINITY ? 0.f : ex2_approx(m - nm);
             m = nm;
             l *= f;
 #pragma unroll 1
@@ -567,11 +583,12 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
             }
           }
         }
+        const float ref = SPLIT && m == -INFINITY ? 0.f : m;      // (no key yet: every probability is 0)
         float2 sum[2] = {splat2(0.f), splat2(0.f)};
         uint32_t p[kPfKeys / 2];
 #pragma unroll
         for (int i = 0; i < kPfKeys / 2; ++i) {
-          const float2 x = ffma2(make_float2(s[2 * i], s[2 * i + 1]), splat2(sl2), splat2(-m));
+          const float2 x = ffma2(make_float2(s[2 * i], s[2 * i + 1]), splat2(sl2), splat2(-ref));
           const float2 e = make_float2(ex2_approx(x.x), ex2_approx(x.y));
           p[i] = pack_bf16(e.x, e.y);
           sum[i & 1] = fadd2(sum[i & 1], e);
@@ -583,22 +600,17 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
         sum[0] = fadd2(sum[0], sum[1]);
         l += sum[0].x + sum[0].y;
       }
-      if (!ok) break;
-      ok = __all_sync(0xffffffffu, tc_wait(&o_full[t], r & 1, abort_flag));
+      if (!SPLIT && !ok) break;
+      ok = ok && __all_sync(0xffffffffu, tc_wait(&o_full[t], r & 1, abort_flag));
+      if (SPLIT) ok = named_sync_and(3, 256, ok);      // both tiles' products are done, or both tiles give up
       if (!ok) break;
       tc_fence_after();
       // Out through shared memory, 64 columns at a time: a row per thread in, whole 128-byte lines out (straight
       // from the registers every store instruction would touch 32 lines: 4 us for the CTA).
-      const float inv = 1.0f / l;
       unsigned char* stg = ostage + warp * 4096;
       const int wrow = row - lane;                             // first query row of this warp
       __nv_bfloat16* dst = a.out + (size_t)(it.seq_start + wrow) * a.out_stride + (size_t)(PAIRS ? 2 * it.head + t : it.head) * kHeadDim;
-#pragma unroll 1
-      for (int h = 0; h < 2; ++h) {
-        float o[64];
-        tc_ld32(o_addr + 64 * h, o);
-        tc_ld32(o_addr + 64 * h + 32, o + 32);
-        tc_wait_ld();
+      auto write_out = [&](int h, const float* o, float inv) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           uint4 v;
@@ -614,6 +626,47 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
           if (wrow + rr < it.seq_len) *reinterpret_cast<uint4*>(dst + (size_t)rr * a.out_stride + 64 * h + 8 * c) = v;
         }
         __syncwarp();
+      };
+      if constexpr (SPLIT) {
+        // exchanged through the place of the second Q tile, 32 columns at a time ([tile][column][row]), and the output
+        // staging ([tile][row] maximum and sum); tile t finishes columns 64 t ... 64 t + 63
+        float* xo = reinterpret_cast<float*>(qs + kPfQBytes);
+        float2* xm = reinterpret_cast<float2*>(ostage);
+        xm[t * kPfRows + lrow] = make_float2(m, l);
+        float o[64];
+        tc_ld32(o_addr + 64 * t, o);
+        tc_ld32(o_addr + 64 * t + 32, o + 32);
+        float wa = 0.f, wb = 0.f, sum = 1.f;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          float x[32];
+          tc_ld32(o_addr + 64 * (t ^ 1) + 32 * h, x);
+          tc_wait_ld();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) xo[(t * 32 + i) * kPfRows + lrow] = x[i];
+          named_sync(3, 256);
+          if (h == 0) {
+            const float2 other = xm[(t ^ 1) * kPfRows + lrow];
+            const float top = fmaxf(m, other.x);                 // finite: tile 0 holds key 0
+            wa = m == -INFINITY ? 0.f : ex2_approx(m - top);
+            wb = other.x == -INFINITY ? 0.f : ex2_approx(other.x - top);
+            sum = fmaf(wb, other.y, wa * l);
+          }
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[32 * h + i] = fmaf(wb, xo[((t ^ 1) * 32 + i) * kPfRows + lrow], wa * o[32 * h + i]);
+          named_sync(3, 256);
+        }
+        write_out(t, o, 1.0f / sum);
+      } else {
+        const float inv = 1.0f / l;
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+          float o[64];
+          tc_ld32(o_addr + 64 * h, o);
+          tc_ld32(o_addr + 64 * h + 32, o + 32);
+          tc_wait_ld();
+          write_out(h, o, inv);
+        }
       }
       tc_fence_before();      // the next item's P arrival orders these reads before the MMA that overwrites O
     }

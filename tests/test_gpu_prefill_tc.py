@@ -67,3 +67,27 @@ def test_prefix_cache_block_sizes(cuda_device, block_size, q_heads, kv_heads):
         want = _reference(q[start:start + q_len], k, v, q_len, k_len, d ** -0.5)
         assert float((got[start:start + q_len] - want).abs().max()) <= 2.0 ** -6, (k_len, q_len)
         start += q_len
+
+
+@pytest.mark.parametrize("q_heads,kv_heads", [(16, 8), (8, 8), (12, 4)])
+@pytest.mark.parametrize("lens,growing", [((512,), False), ((385,), False), ((449,), True), ((1024,), True), ((513, 1), False),
+                                          ((640, 65, 128), True), ((1088,), True)])
+def test_keys_split_over_both_tiles(cuda_device, q_heads, kv_heads, lens, growing):
+    """Batches whose 128-row items all have an SM: odd and even numbers of key tiles, rows whose first own tile holds no
+    visible key, maxima that keep growing, and (1,088 tokens, 16 heads) the first size past the line."""
+    from dfb_b200.kv_store import prefill_attention
+
+    rng = np.random.Generator(np.random.Philox(key=sum(lens) + q_heads))
+    n, d = sum(lens), 128
+    q, k, v = (torch.from_numpy(rng.standard_normal((n, h, d), dtype=np.float32)) for h in (q_heads, kv_heads, kv_heads))
+    if growing:
+        k *= torch.cat([1 + torch.arange(m) / 60.0 for m in lens])[:, None, None]
+        q -= 2.0      # scores far below zero as well as above
+    q, k, v = q.to(BF), k.to(BF), v.to(BF)
+    cu = torch.tensor(np.cumsum([0, *lens]), dtype=torch.int32, device="cuda")
+    got = prefill_attention(q.cuda(), k.cuda(), v.cuda(), cu, max(lens), d ** -0.5).float().cpu()
+    start = 0
+    for m in lens:
+        want = _reference(q[start:start + m], k[start:start + m], v[start:start + m], m, m, d ** -0.5)
+        assert float((got[start:start + m] - want).abs().max()) <= (2.0 ** -5 if growing else 2.0 ** -6), m
+        start += m
