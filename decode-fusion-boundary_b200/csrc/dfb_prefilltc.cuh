@@ -434,7 +434,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
                     (is_v ? a.v : a.k) + (size_t)y * stride + (size_t)kvh * kHeadDim, stride, &full[stage]);
           if (is_v)
             for (int row = rows + row0; row < kPfKeys; row += 2) st_shared_zero16(piece_dst(base, kPfTileBytes / 2, row));
-          push(&full[stage]);
+          if (rows & 7) push(&full[stage]);
+          else announce(&full[stage]);      // boxes only: nothing of this thread's is in flight
           ++n;
           return true;
         }
@@ -500,14 +501,17 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
                       smem_u32(q_full));
         }
       } else {
+        int tail = 0;
 #pragma unroll 1
         for (int t = 0; t < (SPLIT ? 1 : 2); ++t) {
           // (rows past the end keep what was there: their results are not stored and touch no other row)
           const int first = it.q0 + (PAIRS ? 0 : t * kPfRows), rows = max(0, min(it.seq_len - first, kPfRows));
           const int x = (PAIRS ? 2 * it.head + t : it.head) * kHeadDim, y = it.seq_start + first;
+          tail |= rows & 7;
           load_rows(smem_u32(qs) + t * kPfQBytes, kPfRows, rows, &a.q_map8, x, y, a.q + (size_t)y * a.q_stride + x, a.q_stride, q_full);
         }
-        push(q_full);
+        if (tail) push(q_full);
+        else announce(q_full);
       }
       // in the order the issuer consumes them: K0 K1 V0 K2 V1 K3 ...
       if constexpr (SPLIT) {
