@@ -1681,11 +1681,12 @@ int dfb_store_kvcache(const void* key, const void* value, int64_t key_stride, in
   return 0;
 }
 
-int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens_q,
+int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens_q,
                           const int32_t* cu_seqlens_k, int32_t batch, int32_t max_seqlen_q, int64_t q_stride,
                           int64_t k_stride, int64_t v_stride, int64_t out_stride, int32_t q_heads, int32_t kv_heads,
                           int32_t head_dim, float scale, const int32_t* block_tables, int32_t block_table_stride,
-                          int32_t block_size, int32_t num_blocks, int32_t* status, dfb_stream_t stream) {
+                          int32_t block_size, int32_t num_blocks, int32_t* status, int64_t q_rows, int64_t kv_rows,
+                               dfb_stream_t stream) {
   if (!q || !k || !v || !out || !cu_seqlens_q || batch < 1 || max_seqlen_q < 1) return DFB_E_BAD_ARG;
   if (head_dim != kHeadDim || q_heads < 1 || kv_heads < 1 || q_heads % kv_heads) return DFB_E_GEOMETRY;
   // 16-byte pieces of K / V rows and 4-byte pieces of Q / out rows: aligned bases, strides in multiples of 8
@@ -1700,14 +1701,16 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
     if (block_size & (block_size - 1)) return DFB_E_GEOMETRY;   // blocks of a power of two tokens (the reference's are 256)
     while ((1 << block_shift) < block_size) ++block_shift;
   }
-  // Short prompts (whose lengths max_seqlen_q bounds on the host) stay on the mma.sync kernel: its 64-row CTAs
-  // start and finish sooner.  Measured, it is the faster one up to 384 tokens while its CTAs all have an SM of their
-  // own (one prompt of 384: 12.3 us against 12.7), and up to 128 tokens while they are resident together, three
-  // per SM (16 prompts of 64: 6.7 against 9.3 us; 16 of 128 no longer: 13.3 against 9.6).
+  // The shortest prompts (whose lengths max_seqlen_q bounds on the host) stay on the mma.sync kernel: its 64-row CTAs
+  // start and finish sooner.  Measured, it is the faster one up to 192 tokens while its CTAs take half of the SMs (128
+  // tokens: 5.4 against 6.6 us, 2 x 128 5.5 against 6.6; 3 x 128 no longer: 7.9 against 6.7; 200 tokens 7.9 against
+  // 7.2), and up to 64 tokens while each has an SM (6 x 64: 6.2 against 7.0) or the other kernel would need a second
+  // round (24 x 64: 8.6 against 10.6; 12 x 64 not: 7.6 against 7.1).
   const int64_t short_ctas = (int64_t)batch * ((max_seqlen_q + kPfTile - 1) / kPfTile) * q_heads;
   const int sms = sm_count_cached();
-  static const int want_short = env_int("DFB_PF_SHORT", 384);
-  if (!block_tables && max_seqlen_q <= (short_ctas <= sms ? want_short : 128) && short_ctas <= 3 * sms) {
+  const int64_t pair_items = (int64_t)batch * ((max_seqlen_q + kPfRows - 1) / kPfRows) * q_heads / 2;
+  if (!block_tables && ((max_seqlen_q <= 192 && 2 * short_ctas <= sms) ||
+                        (max_seqlen_q <= 64 && (short_ctas <= sms || (short_ctas <= 3 * sms && pair_items > sms))))) {
     const void* fn = (const void*)prefill_short_kernel;
     cudaError_t e = ensure_dynamic_smem(fn, kPfShortSmemBytes);
     if (e != cudaSuccess) return (int)e;
@@ -1724,8 +1727,7 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
   // query heads that share a KV head go in pairs where their number allows it
   // few and short prompts: one head per CTA and the keys split over its two tiles, while every CTA has at most one item
   const int64_t split_items = (int64_t)batch * ((max_seqlen_q + kPfRows - 1) / kPfRows) * q_heads;
-  static const int want_split = env_int("DFB_PF_SPLIT", 1);
-  const bool split = !block_tables && split_items <= sms && want_split;
+  const bool split = !block_tables && split_items <= sms;
   const bool pairs = !split && (q_heads / kv_heads) % 2 == 0;
   auto kernel = split ? prefill_tc_kernel<false, false, true> : block_tables ? (pairs ? prefill_tc_kernel<true, true> : prefill_tc_kernel<true, false>)
                              : (pairs ? prefill_tc_kernel<false, true> : prefill_tc_kernel<false, false>);
@@ -1741,13 +1743,18 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
   // The maps' row counts only have to cover the boxes the kernel asks for, all of them inside a sequence (or a
   // block of the cache); how many tokens there are is known on the device alone.
   a.box_rows = block_tables && block_size < kPfKeys ? block_size : kPfKeys;
+  // (unless the caller says: then a box past the end reads zeros, and no tile of a fresh batch needs the slow tail
+  // but V where another sequence follows: a prompt of 449 tokens 13.1 -> 9.7 us, 300 + 500 tokens 13.9 -> 10.9)
   const int64_t any_rows = (int64_t)1 << 31;
-  int rc = tc_encode_map(q, (int64_t)q_heads * head_dim, any_rows, q_stride, kPfRows, &a.q_map);
-  if (!rc) rc = tc_encode_map(k, (int64_t)kv_heads * head_dim, any_rows, k_stride, a.box_rows, &a.k_map);
-  if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, any_rows, v_stride, a.box_rows, &a.v_map);
-  if (!rc) rc = tc_encode_map(q, (int64_t)q_heads * head_dim, any_rows, q_stride, 8, &a.q_map8);
-  if (!rc) rc = tc_encode_map(k, (int64_t)kv_heads * head_dim, any_rows, k_stride, 8, &a.k_map8);
-  if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, any_rows, v_stride, 8, &a.v_map8);
+  a.exact = !block_tables && q_rows > 0 && kv_rows > 0 && q_rows < any_rows && kv_rows < any_rows;
+  a.kv_rows = (int)kv_rows;
+  const int64_t map_q = a.exact ? q_rows : any_rows, map_kv = a.exact ? kv_rows : any_rows;
+  int rc = tc_encode_map(q, (int64_t)q_heads * head_dim, map_q, q_stride, kPfRows, &a.q_map);
+  if (!rc) rc = tc_encode_map(k, (int64_t)kv_heads * head_dim, map_kv, k_stride, a.box_rows, &a.k_map);
+  if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, map_kv, v_stride, a.box_rows, &a.v_map);
+  if (!rc && !a.exact) rc = tc_encode_map(q, (int64_t)q_heads * head_dim, any_rows, q_stride, 8, &a.q_map8);
+  if (!rc && !a.exact) rc = tc_encode_map(k, (int64_t)kv_heads * head_dim, any_rows, k_stride, 8, &a.k_map8);
+  if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, map_kv, v_stride, 8, &a.v_map8);
   if (rc) return rc;
   // one CTA per SM (all of its tensor memory), fewer when the longest sequence bounds the work items below that
   const int64_t rows = pairs || split ? kPfRows : 2 * kPfRows;
@@ -1755,6 +1762,14 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
   const int grid = (int)(most < sm_count_cached() ? most : sm_count_cached());
   DFB_CUDA(launch_overlapped(kernel, dim3(grid), dim3(kPfThreads), kPfSmemBytes, (cudaStream_t)stream, a));
   return 0;
+}
+
+int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens_q,
+                          const int32_t* cu_seqlens_k, int32_t batch, int32_t max_seqlen_q, int64_t q_stride,
+                          int64_t k_stride, int64_t v_stride, int64_t out_stride, int32_t q_heads, int32_t kv_heads,
+                          int32_t head_dim, float scale, const int32_t* block_tables, int32_t block_table_stride,
+                          int32_t block_size, int32_t num_blocks, int32_t* status, dfb_stream_t stream) {
+  return dfb_prefill_attention_rows(q, k, v, out, cu_seqlens_q, cu_seqlens_k, batch, max_seqlen_q, q_stride, k_stride, v_stride, out_stride, q_heads, kv_heads, head_dim, scale, block_tables, block_table_stride, block_size, num_blocks, status, 0, 0, stream);
 }
 
 int dfb_set_seed(DfbHandle* h, uint64_t seed) {

@@ -17,7 +17,7 @@ def _load():
     from . import native
 
     lib = native.lib()
-    _store, _prefill, _check = lib.dfb_store_kvcache, lib.dfb_prefill_attention, native.check
+    _store, _prefill, _check = lib.dfb_store_kvcache, lib.dfb_prefill_attention_rows, native.check
     _bf16, _i32, _device = torch.bfloat16, torch.int32, torch.cuda.current_device
     # the raw handle of the current stream; the public call builds a Stream object (1 us) around it
     raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -90,7 +90,8 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_seqlens_q.data_ptr(),
         cu_seqlens_k.data_ptr() if cu_seqlens_k is not None else None, cu_seqlens_q.numel() - 1, int(max_seqlen_q),
         q.stride(0), k_stride, v_stride, q_heads * head_dim, q_heads, kv_heads, head_dim, float(softmax_scale),
-        bt_ptr, bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else None, _stream())
+        bt_ptr, bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else None, n,
+        0 if block_table is not None else min(k.shape[0], v.shape[0]), _stream())
     if code:
         _check(code, "dfb_prefill_attention")
     return out

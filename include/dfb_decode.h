@@ -427,6 +427,13 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
                           int64_t k_stride, int64_t v_stride, int64_t out_stride, int32_t q_heads, int32_t kv_heads,
                           int32_t head_dim, float scale, const int32_t* block_tables, int32_t block_table_stride,
                           int32_t block_size, int32_t num_blocks, int32_t* status, dfb_stream_t stream);
+/* The same for a caller that knows the tensors' sizes: q holds q_rows rows and k / v (fresh keys, no block table)
+ * kv_rows each; 0 = not known.  The ends of the sequences are then fetched as fast as the rest. */
+int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens_q,
+                          const int32_t* cu_seqlens_k, int32_t batch, int32_t max_seqlen_q, int64_t q_stride,
+                          int64_t k_stride, int64_t v_stride, int64_t out_stride, int32_t q_heads, int32_t kv_heads,
+                          int32_t head_dim, float scale, const int32_t* block_tables, int32_t block_table_stride,
+                          int32_t block_size, int32_t num_blocks, int32_t* status, int64_t q_rows, int64_t kv_rows, dfb_stream_t stream);
 
 /* Final add+RMSNorm, tied LM head and greedy argmax WITHOUT any allocation.
  * (No counterpart in the reference: its LM head always runs inside a decoder
