@@ -528,6 +528,21 @@ int tc_encode_map(const void* p, int64_t cols, int64_t rows, int64_t stride, int
   }
   return 0;
 }
+// The same for activations: a map depends on its arguments alone, and an engine's buffers come back call after call (the
+// allocator hands the same ones to every layer), so each thread keeps the last map of 32 places.
+int tc_activation_map(const void* p, int64_t cols, int64_t rows, int64_t stride, int box_rows, CUtensorMap* out) {
+  struct Entry { const void* p; int64_t cols, rows, stride; int box_rows; CUtensorMap map; };
+  thread_local Entry entries[32] = {};
+  const uint64_t h = ((uint64_t)(uintptr_t)p >> 4) * 0x9E3779B97F4A7C15ull + (uint64_t)rows * 31 + (uint64_t)box_rows;
+  Entry& e = entries[(h ^ h >> 29) & 31];
+  if (e.p != p || e.cols != cols || e.rows != rows || e.stride != stride || e.box_rows != box_rows) {
+    const int rc = tc_encode_map(p, cols, rows, stride, box_rows, &e.map);
+    if (rc) { e.p = nullptr; return rc; }
+    e.p = p; e.cols = cols; e.rows = rows; e.stride = stride; e.box_rows = box_rows;
+  }
+  *out = e.map;
+  return 0;
+}
 int tc_weight_map(const void* w, int rows, int box_rows, CUtensorMap* out) {
   static std::mutex mu;
   static std::map<std::tuple<const void*, int, int>, CUtensorMap> cache;
@@ -1749,12 +1764,12 @@ int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void
   a.exact = !block_tables && q_rows > 0 && kv_rows > 0 && q_rows < any_rows && kv_rows < any_rows;
   a.kv_rows = (int)kv_rows;
   const int64_t map_q = a.exact ? q_rows : any_rows, map_kv = a.exact ? kv_rows : any_rows;
-  int rc = tc_encode_map(q, (int64_t)q_heads * head_dim, map_q, q_stride, kPfRows, &a.q_map);
-  if (!rc) rc = tc_encode_map(k, (int64_t)kv_heads * head_dim, map_kv, k_stride, a.box_rows, &a.k_map);
-  if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, map_kv, v_stride, a.box_rows, &a.v_map);
-  if (!rc && !a.exact) rc = tc_encode_map(q, (int64_t)q_heads * head_dim, any_rows, q_stride, 8, &a.q_map8);
-  if (!rc && !a.exact) rc = tc_encode_map(k, (int64_t)kv_heads * head_dim, any_rows, k_stride, 8, &a.k_map8);
-  if (!rc) rc = tc_encode_map(v, (int64_t)kv_heads * head_dim, map_kv, v_stride, 8, &a.v_map8);
+  int rc = tc_activation_map(q, (int64_t)q_heads * head_dim, map_q, q_stride, kPfRows, &a.q_map);
+  if (!rc) rc = tc_activation_map(k, (int64_t)kv_heads * head_dim, map_kv, k_stride, a.box_rows, &a.k_map);
+  if (!rc) rc = tc_activation_map(v, (int64_t)kv_heads * head_dim, map_kv, v_stride, a.box_rows, &a.v_map);
+  if (!rc && !a.exact) rc = tc_activation_map(q, (int64_t)q_heads * head_dim, any_rows, q_stride, 8, &a.q_map8);
+  if (!rc && !a.exact) rc = tc_activation_map(k, (int64_t)kv_heads * head_dim, any_rows, k_stride, 8, &a.k_map8);
+  if (!rc) rc = tc_activation_map(v, (int64_t)kv_heads * head_dim, map_kv, v_stride, 8, &a.v_map8);
   if (rc) return rc;
   // one CTA per SM (all of its tensor memory), fewer when the longest sequence bounds the work items below that
   const int64_t rows = pairs || split ? kPfRows : 2 * kPfRows;

@@ -7,18 +7,18 @@ from __future__ import annotations
 
 # Looked up at the first call (the package imports without torch and without the built library) and kept: one call of
 # store_kvcache on a short prompt takes a few microseconds, of which the imports and attribute chains of a call were two.
-_torch = _store = _prefill = _check = _stream = _bf16 = _i32 = _device = None
+_torch = _store = _prefill = _check = _stream = _bf16 = _i32 = _device = _empty = None
 
 
 def _load():
-    global _torch, _store, _prefill, _check, _stream, _bf16, _i32, _device
+    global _torch, _store, _prefill, _check, _stream, _bf16, _i32, _device, _empty
     import torch
 
     from . import native
 
     lib = native.lib()
     _store, _prefill, _check = lib.dfb_store_kvcache, lib.dfb_prefill_attention_rows, native.check
-    _bf16, _i32, _device = torch.bfloat16, torch.int32, torch.cuda.current_device
+    _bf16, _i32, _device, _empty = torch.bfloat16, torch.int32, torch.cuda.current_device, torch.empty
     # the raw handle of the current stream; the public call builds a Stream object (1 us) around it
     raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
     _stream = (lambda: raw(_device())) if raw else (lambda: torch.cuda.current_stream().cuda_stream)
@@ -65,33 +65,35 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
     if _torch is None:
         _load()
     n, q_heads, head_dim = q.shape
-    assert q.stride(-1) == 1 and k.stride(-1) == 1 and v.stride(-1) == 1 and q.stride(1) == head_dim
+    q_stride, q_head, q_one = q.stride()
+    k_strides, v_strides = k.stride(), v.stride()
+    assert q_one == 1 and k_strides[-1] == 1 and v_strides[-1] == 1 and q_head == head_dim
     if q.dtype != _bf16 or k.dtype != _bf16 or v.dtype != _bf16:
         raise TypeError("prefill_attention takes bf16 tensors")
     if cu_seqlens_q.dtype != _i32 or not cu_seqlens_q.is_cuda:
         raise TypeError("cu_seqlens_q must be an int32 CUDA tensor")
     if block_table is not None:
-        num_blocks, block_size, kv_heads = k.shape[0], k.shape[1], k.shape[2]
-        assert k.stride(2) == head_dim and v.stride(2) == head_dim and k.stride(0) == block_size * k.stride(1)
+        num_blocks, block_size, kv_heads = k.shape[:3]
+        k_stride, v_stride, kv_rows = k_strides[1], v_strides[1], 0
+        assert k_strides[2] == head_dim and v_strides[2] == head_dim and k_strides[0] == block_size * k_stride
         if block_table.dtype != _i32 or block_table.stride(-1) != 1 or cu_seqlens_k is None:
             raise TypeError("the prefix-cache case needs an int32 block table and cu_seqlens_k")
-        k_stride, v_stride = k.stride(1), v.stride(1)
         bt_ptr, bt_stride = block_table.data_ptr(), block_table.stride(0)
     else:
-        kv_heads = k.shape[1]
-        assert k.stride(1) == head_dim and v.stride(1) == head_dim
+        kv_rows, kv_heads = k.shape[:2]
+        kv_rows = min(kv_rows, v.shape[0])
+        assert k_strides[1] == head_dim and v_strides[1] == head_dim
         num_blocks = block_size = 0
-        k_stride, v_stride = k.stride(0), v.stride(0)
+        k_stride, v_stride = k_strides[0], v_strides[0]
         bt_ptr, bt_stride = None, 0
-    out = _torch.empty((n, q_heads, head_dim), dtype=_bf16, device=q.device)
+    out = _empty((n, q_heads, head_dim), dtype=_bf16, device=q.device)
     if n == 0:
         return out
     code = _prefill(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_seqlens_q.data_ptr(),
         cu_seqlens_k.data_ptr() if cu_seqlens_k is not None else None, cu_seqlens_q.numel() - 1, int(max_seqlen_q),
-        q.stride(0), k_stride, v_stride, q_heads * head_dim, q_heads, kv_heads, head_dim, float(softmax_scale),
-        bt_ptr, bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else None, n,
-        0 if block_table is not None else min(k.shape[0], v.shape[0]), _stream())
+        q_stride, k_stride, v_stride, q_heads * head_dim, q_heads, kv_heads, head_dim, float(softmax_scale), bt_ptr,
+        bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else None, n, kv_rows, _stream())
     if code:
         _check(code, "dfb_prefill_attention")
     return out
