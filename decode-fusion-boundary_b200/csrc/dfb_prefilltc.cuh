@@ -235,7 +235,7 @@ struct PfWalk {
 // item of CTA `cta` in round r: rounds alternate direction, so that nobody always gets the longer one
 __device__ __forceinline__ int pf_item_index(int r, int cta, int ctas) { return r * ctas + ((r & 1) ? ctas - 1 - cta : cta); }
 
-// SPLIT (fresh keys, chosen while there is an SM for every item): an item is 128 query rows of ONE head, and tile t takes the key
+// SPLIT (small batches; the rule is where the kernel is launched): an item is 128 query rows of ONE head, and tile t takes the key
 // tiles 2 i + t: half as long a chain for the few CTAs of a short batch.  The tiles exchange 64 columns of O each and
 // write the columns that they have merged.
 template <bool PAGED, bool PAIRS, bool SPLIT = false>
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();      // nothing above reads what an earlier kernel wrote
-  static_assert(!SPLIT || (!PAGED && !PAIRS), "the split form takes fresh keys, one head at a time");
+  static_assert(!SPLIT || !PAIRS, "the split form takes one head at a time");
   PfWalk<PAIRS, SPLIT> walk;
   walk.init(a, lane);
   tc_fence_before();
@@ -415,7 +415,14 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
       const long long stride = is_v ? a.v_stride : a.k_stride;
       if (!wait_free(&empty[stage], ((n / kPfStages) & 1) ^ 1)) return false;
       const uint32_t base = smem_u32(ring) + stage * kPfTileBytes;
-      const int rows = max(min(it.k_len - p0, kPfKeys), 0);      // (split form: none in the last tile of an odd number)
+      const int rows = min(it.k_len - p0, kPfKeys);
+      if (SPLIT && rows <= 0) {       // the last tile of an odd number: no key is visible, V meets zeros
+        if (is_v)
+          for (int row = row0; row < kPfKeys; row += 2) st_shared_zero16(piece_dst(base, kPfTileBytes / 2, row));
+        announce(&full[stage]);
+        ++n;
+        return true;
+      }
       const CUtensorMap* map = is_v ? &a.v_map : &a.k_map;
       // one run of rows: fresh projections, or a cache whose blocks hold whole tiles
       if (!PAGED || a.box_rows == kPfKeys) {

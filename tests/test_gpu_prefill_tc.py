@@ -91,3 +91,31 @@ def test_keys_split_over_both_tiles(cuda_device, q_heads, kv_heads, lens, growin
         want = _reference(q[start:start + m], k[start:start + m], v[start:start + m], m, m, d ** -0.5)
         assert float((got[start:start + m] - want).abs().max()) <= (2.0 ** -5 if growing else 2.0 ** -6), m
         start += m
+
+
+@pytest.mark.parametrize("case", [((1, 300),), ((1024, 65),), ((300, 301), (257, 64), (1, 1)), ((1600, 1100),)])
+def test_keys_split_over_both_tiles_prefix_cache(cuda_device, case):
+    """The same from the paged cache: (keys, queries) with odd and even numbers of key tiles and one key."""
+    from dfb_b200.kv_store import prefill_attention
+
+    case = tuple((max(a, b), min(a, b)) for a, b in case)
+    rng = np.random.Generator(np.random.Philox(key=sum(k for k, _ in case)))
+    d, block_size = 128, 256
+    need = [-(-k // block_size) for k, _ in case]
+    pool = rng.permutation(sum(need) + 2).tolist()
+    kc, vc = (torch.from_numpy(rng.standard_normal((sum(need) + 2, block_size, 8, d), dtype=np.float32)).to(BF) for _ in range(2))
+    tables = [[pool.pop() for _ in range(m)] for m in need]
+    q = torch.from_numpy(rng.standard_normal((sum(m for _, m in case), 16, d), dtype=np.float32)).to(BF)
+    for (k_len, _), t in zip(case, tables):
+        if k_len % block_size:
+            vc[t[-1], k_len % block_size:] = float("nan")      # what lies behind the end never counts
+    cu_q, cu_k = (torch.tensor(np.cumsum([0, *x]), dtype=torch.int32, device="cuda") for x in ([c[1] for c in case], [c[0] for c in case]))
+    bt = torch.tensor([t + [0] * (max(need) - len(t)) for t in tables], dtype=torch.int32, device="cuda")
+    got = prefill_attention(q.cuda(), kc.cuda(), vc.cuda(), cu_q, max(m for _, m in case), d ** -0.5, cu_seqlens_k=cu_k,
+                            block_table=bt).float().cpu()
+    start = 0
+    for (k_len, m), t in zip(case, tables):
+        flat = [x[t].reshape(-1, 8, d)[:k_len] for x in (kc, vc)]
+        want = _reference(q[start:start + m], *flat, m, k_len, d ** -0.5)
+        assert float((got[start:start + m] - want).abs().max()) <= 2.0 ** -6
+        start += m
