@@ -1780,7 +1780,7 @@ int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void
   const int64_t rows = pairs || split ? kPfRows : 2 * kPfRows;
   const int64_t most = split ? tiles * q_heads : (int64_t)batch * ((max_seqlen_q + rows - 1) / rows) * (pairs ? q_heads / 2 : q_heads);
   const int grid = (int)(most < sm_count_cached() ? most : sm_count_cached());
-  DFB_CUDA(launch_overlapped(kernel, dim3(grid), dim3(kPfThreads), kPfSmemBytes, (cudaStream_t)stream, a));
+  DFB_CUDA(launch_overlapped(kernel, dim3(grid), dim3(pf_threads(split)), kPfSmemBytes, (cudaStream_t)stream, a));
   return 0;
 }
 

@@ -14,20 +14,27 @@
 //     while the softmax works on S(j), so the softmax never waits for a matrix product.  MMAs of one issuing
 //     thread execute in order: S(j + 2) may be issued behind the P V that still reads P(j) from the same columns.
 //   * Warps 0-3 and 4-7 are the softmax of tile 0 and 1, one thread per query row: the row of S comes out with
-//     two tcgen05.ld, maximum, exp2, bf16, back with tcgen05.st; no shuffles, no shared memory.  O is
-//     rescaled only when a row's maximum has grown by more than 2^8 since the last time (probabilities are then
-//     at most 2^8 instead of 1: bf16 has the range, and sums and products stay fp32); the softmax threads do it
-//     themselves once P V of j - 1 has completed.
+//     two tcgen05.ld, maximum, exp2, bf16, back with tcgen05.st; no shuffles, no shared memory.
+//   * Warps 11-14 multiply the rows of O whose maximum has grown, while the softmax warps compute the exponentials
+//     of the same key tile; P V of the tile waits for both.  (The split form has no registers left for them: its
+//     softmax threads do it themselves behind the store of P.)
+//
+// Rounding: a probability is rounded to bf16 relative to its row's running maximum, so that the largest one is
+// exactly 1, and the row sum adds the rounded values.  Both count: with O rescaled only when a maximum has grown by
+// more than 2^8 the error against 64 bits was 2-8 % larger, with a sum over the unrounded values as well 11-24 % (scores
+// of four times the usual spread; 1-5 % at the usual one), which was 8-12 % of the time (4 x 2,048 tokens 72.7 us
+// against 81.4, the thirteen prompts below 117 against 134, split form 512 tokens 10.5 against 11.0).
 //
 // What bounds it: per 64 keys the two tiles need 1,250 clocks of MMA (512 for P V, 800 for S, whose N = 64 reads Q
 // from shared memory twice as often as N = 128 would; measured with nothing else in the CTA) and 1,024
-// clocks of the SM's 16 exponentials per clock; the kernel takes about 1,800: with the softmax taken out it
-// still takes 1,600, the chain P -> P V and the next S -> softmax of the tile after next.  Tried: 128-key
-// tiles with one S buffer each (1,920 per 64 keys: a tile's softmax and its products then follow one
-// another), one issuing warp for both tiles (2,400), a quarter to a half of the exponentials as polynomials on
-// the FMA pipe (2-5 % slower), the next scores fetched during this tile's exponentials (2 % slower).
-// Short batches are bound by the chain of dependent tiles instead: 512 tokens 9.8 us, 1,024 tokens 14.5.
-// 4 x 2,048 tokens: 74 us = 930 TFLOP/s (mma.sync: 307 us); thirteen prompts of 1 to 2,048 tokens: 116 us (449).
+// clocks of the SM's 16 exponentials per clock; the kernel takes about 2,000: the chain P -> P V and the next S ->
+// softmax of the tile after next, and the tensor memory's port, which the rescaling shares with both (for the thirteen
+// prompts below the softmax warps doing it cost 6 % more time, eight rescaling warps instead of four 1 %).  Tried before the rescaling
+// moved: 128-key tiles with one S buffer each (1,920 against 1,800 clocks per 64 keys: a tile's softmax and its products
+// then follow one another), one issuing warp for both tiles (2,400), a quarter to a half of the exponentials as polynomials
+// on the FMA pipe (2-5 % slower), the next scores fetched during this tile's exponentials (2 % slower).
+// Short batches are bound by the chain of dependent tiles instead: 512 tokens 11.0 us, 1,024 tokens 17.2.
+// 4 x 2,048 tokens: 81 us = 845 TFLOP/s (mma.sync: 307 us); thirteen prompts of 1 to 2,048 tokens: 134 us (449).
 // Every wait is bounded: on expiry the CTA's abort flag is raised, every role drains, status 3 is recorded and
 // the tensor memory released.
 #pragma once
@@ -70,8 +77,9 @@ constexpr int kPfTileBytes = kPfKeys * kHeadDim * 2;      // 16 KB, the same
 constexpr int kPfStages = 8;
 constexpr int kPfOutBytes = 8 * 4096;            // output staging of the eight softmax warps: 32 rows x 64 columns each
 constexpr int kPfThreads = 352;                  // 8 softmax warps, an MMA issuer per tile, the loader
-constexpr int kPfSmemBytes = 1024 + 2 * kPfQBytes + kPfStages * kPfTileBytes + kPfOutBytes + 256;
-constexpr float kPfRescale = 8.0f;               // log2 of how far a maximum may run ahead of the scale in use
+constexpr int kPfRescaleThreads = 128;           // and, but in the split form, 4 rescaling warps
+constexpr int pf_threads(bool split) { return split ? kPfThreads : kPfThreads + kPfRescaleThreads; }
+constexpr int kPfSmemBytes = 1024 + 2 * kPfQBytes + kPfStages * kPfTileBytes + kPfOutBytes + 288;
 
 __device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool live) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(live ? 16 : 0) : "memory");
@@ -109,6 +117,11 @@ __device__ __forceinline__ float2 fadd2(float2 a, float2 b) {
   return d;
 }
 __device__ __forceinline__ float2 splat2(float v) { return make_float2(v, v); }
+// sum += the two bf16 values of `p` (exact in fp32; the additions take a bf16 operand as it is)
+__device__ __forceinline__ void add_bf16x2(float2& sum, uint32_t p) {
+  asm("{\n.reg .b16 lo, hi;\nmov.b32 {lo, hi}, %2;\nadd.f32.bf16 %0, lo, %0;\nadd.f32.bf16 %1, hi, %1;\n}"
+      : "+f"(sum.x), "+f"(sum.y) : "r"(p));
+}
 // shared-memory descriptor of an MN-major operand with the 128-byte swizzle: 64-element pieces of the MN
 // dimension `mn_bytes` apart, groups of 8 K rows 1024 bytes apart
 __device__ __forceinline__ uint64_t tc_smem_desc_mn(uint32_t saddr, uint32_t mn_bytes) {
@@ -155,6 +168,23 @@ __device__ __forceinline__ void tc_st16(uint32_t taddr, const uint32_t* r) {
                  "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
 }
 __device__ __forceinline__ void tc_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+// the 128 output columns of this thread's row times f (no wait behind the last store)
+__device__ __forceinline__ void pf_rescale(uint32_t o_addr, float f) {
+#pragma unroll 1
+  for (int c = 0; c < kHeadDim; c += 64) {
+    float o[64];
+    tc_ld32(o_addr + c, o);
+    tc_ld32(o_addr + c + 32, o + 32);
+    tc_wait_ld();
+#pragma unroll
+    for (int i = 0; i < 64; i += 2) {
+      const float2 y = fmul2(make_float2(o[i], o[i + 1]), splat2(f));
+      o[i] = y.x; o[i + 1] = y.y;
+    }
+    tc_st32(o_addr + c, reinterpret_cast<const uint32_t*>(o));
+    tc_st32(o_addr + c + 32, reinterpret_cast<const uint32_t*>(o + 32));
+  }
+}
 
 // The work items in order of falling length, the same list in every role.  Item rows of one sequence are
 // numbered by `level`, its place in units of 128 keys (cached prefix + queries), so one step of the walk
@@ -239,7 +269,7 @@ __device__ __forceinline__ int pf_item_index(int r, int cta, int ctas) { return 
 // tiles 2 i + t: half as long a chain for the few CTAs of a short batch.  The tiles exchange 64 columns of O each and
 // write the columns that they have merged.
 template <bool PAGED, bool PAIRS, bool SPLIT = false>
-__global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_constant__ PrefillArgs a) {
+__global__ void __launch_bounds__(pf_threads(SPLIT), 1) prefill_tc_kernel(const __grid_constant__ PrefillArgs a) {
   extern __shared__ unsigned char pf_raw[];
   const uint32_t raw = smem_u32(pf_raw);
   unsigned char* dyn = pf_raw + (((raw + 1023u) & ~1023u) - raw);
@@ -254,7 +284,8 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
   uint64_t* p_full = s_full + 4;                             // [tile][buffer]
   uint64_t* pv_done = p_full + 4;                            // [tile], once per key tile
   uint64_t* o_full = pv_done + 2;                            // [tile], once per item
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_full + 2);
+  uint64_t* f_full = o_full + 2;                             // [tile][buffer]: the rows' factors are there
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(f_full + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -269,7 +300,7 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
     mbar_init(q_full, 32);
     mbar_init(q_empty, 2);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 128); }
+    for (int i = 0; i < 4; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], SPLIT ? 128 : 132); mbar_init(&f_full[i], 4); }
     mbar_init(&pv_done[0], 1); mbar_init(&pv_done[1], 1);
     mbar_init(&o_full[0], 1); mbar_init(&o_full[1], 1);
     *abort_flag = 0;
@@ -550,6 +581,9 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t s_addr = tmem + lanes + 256 + 128 * t, o_addr = tmem + lanes + 128 * t;
     const float sl2 = a.scale * 1.4426950408889634f;       // scores in units of log2 e
+    // this row's factor for the rescaling warps, one per S buffer; in the warp's own output staging, which it has read when
+    // the next item begins (and the last factor has been read when an item's products are done)
+    volatile float* factor = reinterpret_cast<volatile float*>(ostage + warp * 4096) + lane;
     int g = 0;
     for (int r = 0; ok && walk.find(a, pf_item_index(r, cta, ctas), lane, it); ++r) {
       const int row = it.q0 + (PAIRS || SPLIT ? 0 : t * kPfRows) + lrow;               // query row inside the sequence
@@ -577,44 +611,41 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
 #pragma unroll
           for (int u = 0; u < 4; ++u) mx[u] = i + 4 + u < kPfKeys ? fmax3(mx[u], s[i + u], s[i + 4 + u]) : fmaxf(mx[u], s[i + u]);
         const float mt = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sl2;
-        if (j == 0) {
-          m = mt;                          // key 0 is visible to every row: finite (split form, odd tiles: or -inf)
-        } else {
-          const bool grow = mt > m + kPfRescale;
-          if (__any_sync(0xffffffffu, grow)) {
-            // S(g) was issued behind P V of g - 2: at most one phase is missing
-            ok = __all_sync(0xffffffffu, tc_wait(&pv_done[t], (g - 1) & 1, abort_flag));
-            if (!ok) break;
-            tc_fence_after();
-            const float nm = grow ? mt : m, f = SPLIT && m == -INFINITY ? 0.f : ex2_approx(m - nm);
-            m = nm;
-            l *= f;
-#pragma unroll 1
-            for (int c = 0; c < 8; ++c) {
-              float o[16];
-              tc_ld16(o_addr + 16 * c, o);
-#pragma unroll
-              for (int i = 0; i < 16; ++i) o[i] *= f;
-              tc_st16(o_addr + 16 * c, reinterpret_cast<const uint32_t*>(o));
-            }
-          }
+        // key 0 is visible to every row: finite (split form, odd tiles: or -inf)
+        const float nm = j == 0 ? mt : fmaxf(m, mt);
+        const float f = SPLIT && m == -INFINITY ? 0.f : ex2_approx(m - nm);
+        const bool rescale = SPLIT && j > 0 && __any_sync(0xffffffffu, nm > m);
+        if (!SPLIT) {
+          factor[32 * b] = f;
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(&f_full[2 * t + b]);
         }
+        m = nm;
         const float ref = SPLIT && m == -INFINITY ? 0.f : m;      // (no key yet: every probability is 0)
         float2 sum[2] = {splat2(0.f), splat2(0.f)};
         uint32_t p[kPfKeys / 2];
 #pragma unroll
         for (int i = 0; i < kPfKeys / 2; ++i) {
           const float2 x = ffma2(make_float2(s[2 * i], s[2 * i + 1]), splat2(sl2), splat2(-ref));
-          const float2 e = make_float2(ex2_approx(x.x), ex2_approx(x.y));
-          p[i] = pack_bf16(e.x, e.y);
-          sum[i & 1] = fadd2(sum[i & 1], e);
+          p[i] = pack_bf16(ex2_approx(x.x), ex2_approx(x.y));
+          add_bf16x2(sum[i & 1], p[i]);
         }
         tc_st32(s_addr + 64 * b, p);
+        if (rescale) {
+          // S(g) was issued behind P V of g - 2: at most one phase is missing
+          ok = __all_sync(0xffffffffu, tc_wait(&pv_done[t], (g - 1) & 1, abort_flag));
+          if (ok) {
+            tc_fence_after();
+            pf_rescale(o_addr, f);
+          }
+        }
         tc_wait_st();
+        if (!ok) break;
         tc_fence_before();
         tc_mbar_arrive(&p_full[2 * t + b]);
+        // the row sum takes the rounded probabilities, the values that multiply V; the product does not wait for it
         sum[0] = fadd2(sum[0], sum[1]);
-        l += sum[0].x + sum[0].y;
+        l = (j == 0 ? 0.f : l * f) + (sum[0].x + sum[0].y);
       }
       if (!SPLIT && !ok) break;
       ok = ok && __all_sync(0xffffffffu, tc_wait(&o_full[t], r & 1, abort_flag));
@@ -685,6 +716,33 @@ __global__ void __launch_bounds__(kPfThreads, 1) prefill_tc_kernel(const __grid_
         }
       }
       tc_fence_before();      // the next item's P arrival orders these reads before the MMA that overwrites O
+    }
+    if (!ok) *abort_flag = 1;
+  } else if (!SPLIT) {
+    // ------------------------------ rescaling: four warps, the rows of both tiles ------------------------------
+    // O is multiplied while the softmax warps are at the exponentials of the same key tile; P V waits for both.
+    const int quarter = warp & 3;                  // the tensor memory lanes this warp may touch
+    int g = 0;
+    for (int r = 0; ok && walk.find(a, pf_item_index(r, cta, ctas), lane, it); ++r) {
+      for (int j = 0; ok && j < it.n_tiles; ++j, ++g) {
+#pragma unroll 1
+        for (int t = 0; ok && t < 2; ++t) {
+          ok = __all_sync(0xffffffffu, tc_wait(&f_full[2 * t + (g & 1)], (g >> 1) & 1, abort_flag));
+          if (!ok) break;
+          const float f = reinterpret_cast<volatile float*>(ostage + (4 * t + quarter) * 4096)[32 * (g & 1) + lane];
+          if (j > 0 && __any_sync(0xffffffffu, f != 1.f)) {
+            // S(g) was issued behind P V of g - 2: at most one phase is missing
+            ok = __all_sync(0xffffffffu, tc_wait(&pv_done[t], (g - 1) & 1, abort_flag));
+            if (!ok) break;
+            tc_fence_after();
+            pf_rescale(tmem + ((uint32_t)(32 * quarter) << 16) + 128 * t, f);
+            tc_wait_st();
+          }
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) tc_mbar_arrive(&p_full[2 * t + (g & 1)]);
+        }
+      }
     }
     if (!ok) *abort_flag = 1;
   }
