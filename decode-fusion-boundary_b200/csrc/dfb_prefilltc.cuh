@@ -580,7 +580,11 @@ __global__ void __launch_bounds__(pf_threads(SPLIT), 1) prefill_tc_kernel(const 
     const int t = warp >> 2, lrow = 32 * (warp & 3) + lane;
     const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
     const uint32_t s_addr = tmem + lanes + 256 + 128 * t, o_addr = tmem + lanes + 128 * t;
-    const float sl2 = a.scale * 1.4426950408889634f;       // scores in units of log2 e
+    // scores in units of log2 e; a positive scale is applied behind the maximum, any other one (which turns the order of
+    // the scores around, or makes them all equal) to the scores themselves
+    const float scale2 = a.scale * 1.4426950408889634f;
+    const bool ordered = scale2 > 0.f;
+    const float sl2 = ordered ? scale2 : 1.f, pre = ordered ? 1.f : scale2;
     // this row's factor for the rescaling warps, one per S buffer; in the warp's own output staging, which it has read when
     // the next item begins (and the last factor has been read when an item's products are done)
     volatile float* factor = reinterpret_cast<volatile float*>(ostage + warp * 4096) + lane;
@@ -601,9 +605,9 @@ __global__ void __launch_bounds__(pf_threads(SPLIT), 1) prefill_tc_kernel(const 
         tc_ld32(s_addr + 64 * b + 32, s + 32);
         tc_wait_ld();
         const int p0 = (SPLIT ? 2 * j + t : j) * kPfKeys;
-        if (p0 + kPfKeys > clear) {       // the same for every thread of the tile
+        if (p0 + kPfKeys > clear || !ordered) {       // the same for every thread of the tile
 #pragma unroll
-          for (int i = 0; i < kPfKeys; ++i) s[i] = p0 + i < seen ? s[i] : -INFINITY;
+          for (int i = 0; i < kPfKeys; ++i) s[i] = p0 + i < seen ? s[i] * pre : -INFINITY;
         }
         float mx[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll

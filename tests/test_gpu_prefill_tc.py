@@ -164,3 +164,34 @@ def test_error_against_64_bits(cuda_device, q_heads, kv_heads, new, cached):
             emulated += float(((r @ vh / r.sum(-1, keepdim=True)).to(BF).double() - exact).square().sum())
             err += float((got[rows, h].double() - exact).square().sum())
     assert err ** 0.5 <= 1.02 * emulated ** 0.5, (err / emulated) ** 0.5
+
+
+@pytest.mark.parametrize("scale", [-0.09, 0.0])
+@pytest.mark.parametrize("new,cached", [((100,), (0,)), ((300, 513), (0, 0)), ((640,) * 4, (0,) * 4),       # short, split, pairs
+                                        ((300, 65), (512, 256)), ((300,) * 12, (256,) * 12)])
+def test_scale_of_either_sign(cuda_device, scale, new, cached):
+    """A scale that is not positive: the largest score is the smallest product, or all scores are equal."""
+    from dfb_b200.kv_store import prefill_attention
+
+    rng = np.random.Generator(np.random.Philox(key=sum(new)))
+    d, bs, total = 128, 256, [a + b for a, b in zip(new, cached)]
+    q = torch.from_numpy(rng.standard_normal((sum(new), 16, d), dtype=np.float32)).to(BF)
+    ks, vs = ([torch.from_numpy(rng.standard_normal((n, 8, d), dtype=np.float32)).to(BF) for n in total] for _ in range(2))
+    cu_q, cu_k = (torch.tensor(np.cumsum([0, *x]), dtype=torch.int32, device="cuda") for x in (new, total))
+    if any(cached):
+        need = [-(-n // bs) for n in total]
+        kc, vc = (torch.zeros(sum(need), bs, 8, d, dtype=BF) for _ in range(2))
+        first = np.cumsum([0, *need])
+        for i, n in enumerate(total):
+            kc.flatten(0, 1)[first[i] * bs:first[i] * bs + n] = ks[i]
+            vc.flatten(0, 1)[first[i] * bs:first[i] * bs + n] = vs[i]
+        bt = torch.tensor([[first[i] + c if c < m else 0 for c in range(max(need))] for i, m in enumerate(need)],
+                          dtype=torch.int32, device="cuda")
+        got = prefill_attention(q.cuda(), kc.cuda(), vc.cuda(), cu_q, max(new), scale, cu_seqlens_k=cu_k, block_table=bt)
+    else:
+        got = prefill_attention(q.cuda(), torch.cat(ks).cuda(), torch.cat(vs).cuda(), cu_q, max(new), scale)
+    start = 0
+    for i, n in enumerate(new):
+        want = _reference(q[start:start + n], ks[i], vs[i], n, total[i], scale)
+        assert float((got[start:start + n].float().cpu() - want).abs().max()) <= 2.0 ** -6
+        start += n
