@@ -341,6 +341,7 @@ struct DfbHandle {
   int* row_tokens = nullptr;            // pinned: tokens[8] | status[4] | sequence word
   unsigned int* row_seq = nullptr;      // device
   unsigned int row_published = 0;       // host
+  bool row_waitable = false;            // the last step that was given out_tokens publishes them
   cudaEvent_t burst_event = nullptr;
   int burst_rows = 0, burst_steps = 0;  // of the burst in flight (0 = none)
   // fixed-slot runtime (dfb_slot_* / dfb_slots_*): host-side state of every slot
@@ -1836,10 +1837,14 @@ int dfb_decode_step(DfbHandle* h, const DfbStepDesc* s, dfb_stream_t stream_) {
   }
   io.sampling = s->temperatures != nullptr;
   if (io.sampling && s->out_logits && h->step_mode == 1) return DFB_E_BAD_ARG;
+  if (io.out_tokens) h->row_waitable = false;
   int rc = run_step(h, s->rows, split_bucket(h, bound, s->rows), s->block_table_cols, io, stream, s->out_logits);
   if (rc) return rc;
   ++h->steps;
-  if (io.publish) ++h->row_published;
+  if (io.publish) {
+    ++h->row_published;
+    h->row_waitable = true;
+  }
   return 0;
 }
 
@@ -1856,8 +1861,12 @@ static bool poll_published(const int* word_, unsigned want) {
 }
 
 int dfb_wait_tokens(DfbHandle* h, int32_t* out_tokens, dfb_stream_t stream_) {
-  if (!h || !out_tokens || h->row_published == 0) return DFB_E_BAD_ARG;
-  if (!poll_published(h->row_tokens + kMaxRows + 4, h->row_published)) DFB_CUDA(cudaStreamSynchronize((cudaStream_t)stream_));
+  if (!h || !out_tokens || !h->row_waitable) return DFB_E_BAD_ARG;
+  const int* word = h->row_tokens + kMaxRows + 4;
+  if (!poll_published(word, h->row_published)) {
+    DFB_CUDA(cudaStreamSynchronize((cudaStream_t)stream_));
+    if ((int)(*(const volatile unsigned*)word - h->row_published) < 0) return (int)cudaErrorNotReady;   // another stream's step
+  }
   memcpy(out_tokens, h->row_tokens, sizeof(int) * (kMaxRows + 4));
   return h->row_tokens[kMaxRows] ? DFB_E_DEVICE_STATUS : 0;
 }

@@ -345,7 +345,9 @@ int dfb_set_seed(DfbHandle* h, uint64_t seed);
 /* Waits for the last dfb_decode_step that was given out_tokens and copies the same DFB_MAX_ROWS + 4 values into host
  * memory: the step's last kernel also writes them to pinned memory, where this call polls for them (no copy, no
  * stream synchronisation; `stream` is the step's, synchronised only when nothing arrives for a tenth of a second).
- * Returns DFB_E_DEVICE_STATUS if a kernel recorded an error (the status word is left for dfb_read_status). */
+ * Returns DFB_E_DEVICE_STATUS if a kernel recorded an error (the status word is left for dfb_read_status) and
+ * DFB_E_BAD_ARG if there is no such step or the last one was captured into a graph of the caller's (it runs when the
+ * caller replays that graph, and writes its device buffer only). */
 int dfb_wait_tokens(DfbHandle* h, int32_t* out_tokens, dfb_stream_t stream);
 
 /* Read (and clear) the device status word; synchronises nothing by itself, so

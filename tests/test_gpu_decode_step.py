@@ -404,3 +404,38 @@ def test_warm_captures_every_geometry_ahead_of_time(cuda_device):
     assert dec.warm(max_rows=3, max_context=700) == held, "a step captured a graph that warm() had not prepared"
     assert warm_s < 30.0
     dec.close()
+
+
+def test_waiting_for_tokens_of_a_captured_step_is_refused(cuda_device):
+    """A step that the caller captures runs when they replay the graph: there is nothing to wait for, and the tokens of
+    the step before it must not come back in its place.  The graph's device buffer and later steps are as ever."""
+    import ctypes as C
+    from dfb_b200 import native
+
+    g = H.oracle_geometry(layers=1, vocab=2048)
+    w = O.make_weights(g, seed=67, norm="random").to(torch.bfloat16)
+    kv = O.new_kv_cache(g, 4, torch.bfloat16).cuda()
+    dec = H.make_decoder(w, kv, use_graph=False)
+    bt = torch.tensor([[0], [1]], dtype=torch.int32, device="cuda")
+    pos = torch.zeros(2, dtype=torch.int64, device="cuda")
+    ids = [torch.tensor(x, dtype=torch.int64, device="cuda") for x in ([5, 9], [700, 1200])]
+    out = (C.c_int32 * (native.DFB_MAX_ROWS + 4))()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        assert dec._lib.dfb_wait_tokens(dec._handle, out, dec._stream()) == -1      # no step yet
+        want = [dec.decode_rows(x, pos, bt) for x in ids]
+        assert want[0] != want[1]
+        dec.decode_rows(ids[0], pos, bt)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            dec.enqueue_rows(ids[1], pos, bt)
+            assert dec._lib.dfb_wait_tokens(dec._handle, out, dec._stream()) == -1
+            with pytest.raises(RuntimeError, match="bad argument"):
+                dec.decode_rows(ids[1], pos, bt)
+        graph.replay()
+        stream.synchronize()
+        assert dec.tokens_device()[:2].tolist() == want[1]
+        assert dec._lib.dfb_wait_tokens(dec._handle, out, dec._stream()) == -1
+        assert dec.decode_rows(ids[0], pos, bt) == want[0]
+    assert dec.status()[0] == 0
+    dec.close()
