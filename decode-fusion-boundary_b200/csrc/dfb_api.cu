@@ -353,7 +353,7 @@ struct DfbHandle {
     std::vector<int> table;     // the slot's block table (physical block ids)
   };
   std::vector<Slot> slots;
-  // Steps of 9 to 32 slots at once (dfb_wide.cuh).  Buffers of 32 rows in one slab, allocated with the first slot.
+  // Steps of 9 to 32 slots at once (dfb_wide.cuh).  Buffers of 32 rows in one slab, allocated by the first such step.
   struct Wide {
     void* slab = nullptr;
     int* stage = nullptr;            // device: ids[32] | positions[32] | active[32] | temperatures[32] | block tables[32, max_pages]
@@ -1183,7 +1183,9 @@ int wide_prepare(DfbHandle* h) {
   const size_t o_parts = carve(sizeof(ArgmaxPart) * kWideRows * h->sm_count), o_tok = carve(sizeof(int) * kWideRows);
   void* slab = nullptr;
   DFB_CUDA(cudaMalloc(&slab, off));
-  cudaError_t e = cudaMemset(slab, 0, off);
+  // zero before this returns: the step's stream may be ordered behind neither the legacy stream nor this one
+  cudaError_t e = cudaMemsetAsync(slab, 0, off, h->capture_stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(h->capture_stream);
   if (e == cudaSuccess && !w.host_stage) e = cudaMallocHost((void**)&w.host_stage, sizeof(int) * stage_ints);
   if (e == cudaSuccess && !w.host_tokens) e = cudaMallocHost((void**)&w.host_tokens, sizeof(int) * (kWideRows + 8));
   if (e != cudaSuccess) { cudaFree(slab); return (int)e; }

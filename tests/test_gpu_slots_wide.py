@@ -31,11 +31,11 @@ def model():
     return g, w, history
 
 
-def _step(w, history, n, temperatures, wide, steps=1):
+def _step(w, history, n, temperatures, wide, steps=1, use_graph=True, before_steps=None):
     from dfb_b200 import native
     from dfb_b200.slots import SlotRuntime
     kv = history.clone()
-    dec = H.make_decoder(w, kv)
+    dec = H.make_decoder(w, kv, use_graph=use_graph)
     if not wide:
         dec.set_option(native.DFB_OPT_BULK_X, 1)       # the default value; a decoder with a tuned chain steps 8 rows at a time
     dec.set_seed(5)
@@ -45,6 +45,10 @@ def _step(w, history, n, temperatures, wide, steps=1):
         blocks = (LENGTHS[i] + steps - 1) // 256 + 1
         rt.admit(i, 100 + 7 * i, LENGTHS[i], list(range(first, first + blocks)), temperatures[i] if temperatures else 0.0)
         first += blocks
+    if before_steps:
+        torch.cuda.synchronize()
+        with torch.cuda.stream(torch.cuda.default_stream()):
+            before_steps()
     out = [rt.step() for _ in range(steps)]
     assert dec.status()[0] == 0
     dec.close()
@@ -75,3 +79,18 @@ def test_wide_step_noise_stream_continues(model, cuda_device):
     want, _ = _step(w, history, 20, temps, wide=False, steps=2)
     assert more[0] == got[0] and more[1] != more[0]
     assert sum(more[1][i] == want[1][i] for i in range(20)) >= 18          # (a near tie may fall the other way)
+
+
+def test_first_wide_step_beside_a_busy_default_stream(model, cuda_device):
+    """The buffers of a wide step are made by the first one: they are ready for a step on a stream of its own, whatever
+    the default stream is still doing (30 products of 8,192 x 8,192 matrices, several ms)."""
+    g, w, history = model
+    want, kv_want = _step(w, history, 12, None, wide=True)
+    a = torch.zeros(8192, 8192, dtype=BF, device="cuda")
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream()
+    with torch.cuda.stream(stream):
+        got, kv_got = _step(w, history, 12, None, wide=True, use_graph=False,
+                            before_steps=lambda: [torch.mm(a, a) for _ in range(30)])
+    torch.cuda.synchronize()
+    assert got == want and torch.equal(kv_got, kv_want)
