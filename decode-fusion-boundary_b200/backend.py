@@ -198,9 +198,10 @@ class MegakernelBackend:
             self.decoder.set_seed(int(seed))
         if _get_attr(self.config, "megakernel_warm", True) and group is None:   # sharded decoders capture lazily
             # every step geometry this engine can ask for is captured now, as ModelRunner.capture_cudagraph does
-            # for the torch path (engine/model_runner.py:379-416): 160 graphs, about 0.1 s and 70 MB at 8 rows
+            # for the torch path (engine/model_runner.py:379-416): 172 graphs, about 0.1 s and 70 MB at 8 rows (those of
+            # more than 8 slots when a SlotRuntime is made)
             rows = min(int(_get_attr(self.config, "max_num_seqs", 8) or 8), 8)
-            kinds = self.decoder.WARM_HOST | self.decoder.WARM_DEVICE_TOKENS
+            kinds = self.decoder.WARM_HOST | self.decoder.WARM_DEVICE_TOKENS | self.decoder.WARM_NO_SLOTS
             if _get_attr(self.config, "megakernel_sampling", False):
                 kinds |= self.decoder.WARM_SAMPLING
             self.decoder.warm(max_rows=max(rows, 1), max_context=max_model_len, kinds=kinds)

@@ -353,8 +353,10 @@ struct DfbHandle {
     std::vector<int> table;     // the slot's block table (physical block ids)
   };
   std::vector<Slot> slots;
-  // Steps of 9 to 32 slots at once (dfb_wide.cuh).  Buffers of 32 rows in one slab, allocated by the first such step.
+  // Steps of 9 to 32 slots at once (dfb_wide.cuh).  Buffers of 32 rows in one slab, allocated by dfb_warm_slots or else by
+  // the first such step.
   struct Wide {
+    bool no_room = false;            // they could not be allocated: launches of 8 rows
     void* slab = nullptr;
     int* stage = nullptr;            // device: ids[32] | positions[32] | active[32] | temperatures[32] | block tables[32, max_pages]
     int* host_stage = nullptr;       // pinned copy
@@ -1279,42 +1281,82 @@ int enqueue_wide(DfbHandle* h, int chunks, bool half, bool sampling, cudaStream_
   return 0;
 }
 
-// Inputs of `rows` (9 to 32) rows are in wide.host_stage: contexts of `halves` 32-position or `wholes` 64-position chunks.
-// A chunk is a serial walk for its CTA (1.1 us per 8 positions), so the shorter ones are taken while all of their CTAs
-// are resident together, two per SM (10 rows x 512: 903 against 1,000 us per step; 20 rows with 330 of them not).
-int wide_step(DfbHandle* h, int rows, int halves, int wholes, bool sampling, cudaStream_t stream) {
-  DfbHandle::Wide& w = h->wide;
-  const int groups = (rows + 7) / 8;
+// Kernels and attention grid of a wide step of `rows` (9 to 32) rows whose contexts come to `halves` 32-position or
+// `wholes` 64-position chunks.  A chunk is a serial walk for its CTA (1.1 us per 8 positions), so the shorter ones are taken
+// while all of their CTAs are resident together, two per SM (10 rows x 512: 903 against 1,000 us per step; 20 rows with
+// 330 of them not).
+struct WideGeometry { int groups, chunks; bool half; };
+int wide_grid(int chunks) {      // few grids, so that few graphs: the attention CTAs without a chunk leave at once
+  int grid = 64;
+  while (grid < chunks) grid <<= 1;
+  return grid;
+}
+WideGeometry wide_geometry(const DfbHandle* h, int rows, int halves, int wholes) {
   const bool half = halves <= 2 * h->sm_count;
-  const int total_chunks = half ? halves : wholes;
-  int chunks = 64;                  // few grids, so that few graphs: the attention CTAs without a chunk leave at once
-  while (chunks < total_chunks) chunks <<= 1;
-  auto enqueue = [&](cudaStream_t s) {
-    return groups == 2 ? enqueue_wide<2>(h, chunks, half, sampling, s) : groups == 3 ? enqueue_wide<3>(h, chunks, half, sampling, s)
-                                                                                : enqueue_wide<4>(h, chunks, half, sampling, s);
-  };
-  if (h->use_graph) {
-    const int key = (((chunks * 8 + groups) * 2 + (half ? 1 : 0)) * 2 + (sampling ? 1 : 0)) * 2 + (h->use_pdl ? 1 : 0);
-    auto it = w.graphs.find(key);
-    if (it == w.graphs.end()) {
-      cudaGraph_t graph = nullptr;
-      cudaGraphExec_t exec = nullptr;
-      DFB_CUDA(cudaStreamBeginCapture(h->capture_stream, cudaStreamCaptureModeThreadLocal));
-      const int rc = enqueue(h->capture_stream);
-      cudaError_t e = cudaStreamEndCapture(h->capture_stream, &graph);
-      if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
-      if (e != cudaSuccess) return (int)e;
-      e = cudaGraphInstantiate(&exec, graph, 0);
-      cudaGraphDestroy(graph);
-      if (e != cudaSuccess) return (int)e;
-      it = w.graphs.emplace(key, exec).first;
+  return {(rows + 7) / 8, wide_grid(half ? halves : wholes), half};
+}
+
+int enqueue_wide_step(DfbHandle* h, const WideGeometry& g, bool sampling, cudaStream_t s) {
+  return g.groups == 2 ? enqueue_wide<2>(h, g.chunks, g.half, sampling, s) : g.groups == 3 ? enqueue_wide<3>(h, g.chunks, g.half, sampling, s)
+                                                                               : enqueue_wide<4>(h, g.chunks, g.half, sampling, s);
+}
+
+int get_wide_graph(DfbHandle* h, const WideGeometry& g, bool sampling, cudaGraphExec_t* out) {
+  const int key = (((g.chunks * 8 + g.groups) * 2 + (g.half ? 1 : 0)) * 2 + (sampling ? 1 : 0)) * 2 + (h->use_pdl ? 1 : 0);
+  auto it = h->wide.graphs.find(key);
+  if (it == h->wide.graphs.end()) {
+    cudaGraph_t graph = nullptr;
+    cudaGraphExec_t exec = nullptr;
+    DFB_CUDA(cudaStreamBeginCapture(h->capture_stream, cudaStreamCaptureModeThreadLocal));
+    const int rc = enqueue_wide_step(h, g, sampling, h->capture_stream);
+    cudaError_t e = cudaStreamEndCapture(h->capture_stream, &graph);
+    if (rc) { if (graph) cudaGraphDestroy(graph); return rc; }
+    if (e != cudaSuccess) return (int)e;
+    e = cudaGraphInstantiate(&exec, graph, 0);
+    cudaGraphDestroy(graph);
+    if (e != cudaSuccess) return (int)e;
+    it = h->wide.graphs.emplace(key, exec).first;
+  }
+  *out = it->second;
+  return 0;
+}
+
+// Buffers, and the graphs of every wide step with contexts up to `max_context` (7 per group count at 2,048 tokens).
+int warm_wide(DfbHandle* h, int max_context, bool sampling) {
+  h->wide.no_room = false;
+  int rc = wide_prepare(h);
+  if (rc || !h->use_graph) return rc;
+  constexpr int kHalf = kAttnChunk / 2;
+  for (int groups = 2; groups <= kWideRows / 8; ++groups) {
+    const int halves = 8 * groups * ((max_context + kHalf - 1) / kHalf), wholes = 8 * groups * ((max_context + kAttnChunk - 1) / kAttnChunk);
+    const int resident = 2 * h->sm_count;
+    for (int half = 1; half >= 0; --half) {
+      if (!half && halves <= resident) break;
+      // whole chunks begin where the half ones no longer fit: at more than half as many
+      const int last = wide_grid(half ? (halves < resident ? halves : resident) : wholes);
+      for (int grid = wide_grid(half ? 1 : resident / 2 + 1); grid <= last; grid <<= 1)
+        for (int s = 0; s < (sampling ? 2 : 1); ++s) {
+          cudaGraphExec_t exec;
+          rc = get_wide_graph(h, WideGeometry{groups, grid, half != 0}, s != 0, &exec);
+          if (rc) return rc;
+        }
     }
-    DFB_CUDA(cudaGraphLaunch(it->second, stream));
+  }
+  return 0;
+}
+
+// The step of the rows whose inputs are in wide.host_stage.
+int wide_step(DfbHandle* h, const WideGeometry& g, bool sampling, cudaStream_t stream) {
+  if (h->use_graph) {
+    cudaGraphExec_t exec;
+    const int rc = get_wide_graph(h, g, sampling, &exec);
+    if (rc) return rc;
+    DFB_CUDA(cudaGraphLaunch(exec, stream));
   } else {
-    const int rc = enqueue(stream);
+    const int rc = enqueue_wide_step(h, g, sampling, stream);
     if (rc) return rc;
   }
-  ++w.published;
+  ++h->wide.published;
   ++h->steps;
   return 0;
 }
@@ -1633,8 +1675,8 @@ int dfb_set_option(DfbHandle* h, int option, int value) {
 }
 
 int dfb_warm(DfbHandle* h, int32_t max_rows, int32_t max_context, int32_t kinds, int32_t* graphs_out) {
-  if (graphs_out) *graphs_out = h ? (int32_t)h->graphs.size() : 0;
-  if (!h || max_rows < 1 || max_rows > kMaxRows || max_context < 1 || kinds < 1 || kinds > 31) return DFB_E_BAD_ARG;
+  if (graphs_out) *graphs_out = h ? (int32_t)(h->graphs.size() + h->wide.graphs.size()) : 0;
+  if (!h || max_rows < 1 || max_rows > kMaxRows || max_context < 1 || kinds < 1 || kinds > 63 || kinds == 32) return DFB_E_BAD_ARG;
   if (max_context > h->m.max_model_len) max_context = h->m.max_model_len;
   if (!h->use_graph) return 0;
   // dummy arguments of the input staging kernel for the device-pointer kinds: a launch patches them anyway
@@ -1677,8 +1719,20 @@ int dfb_warm(DfbHandle* h, int32_t max_rows, int32_t max_context, int32_t kinds,
       if (ctx >= max_context) break;
     }
   }
-  if (graphs_out) *graphs_out = (int32_t)h->graphs.size();
+  // the slots' steps of more rows than that come from host buffers, too
+  if ((kinds & 8) && !(kinds & 32) && max_rows == kMaxRows) return dfb_warm_slots(h, max_context, kinds & 16, graphs_out);
+  if (graphs_out) *graphs_out = (int32_t)(h->graphs.size() + h->wide.graphs.size());
   return 0;
+}
+
+int dfb_warm_slots(DfbHandle* h, int32_t max_context, int32_t sampling, int32_t* graphs_out) {
+  if (graphs_out) *graphs_out = h ? (int32_t)(h->graphs.size() + h->wide.graphs.size()) : 0;
+  if (!h || max_context < 1) return DFB_E_BAD_ARG;
+  if (!wide_usable(h)) return 0;
+  const int rc = warm_wide(h, max_context < h->m.max_model_len ? max_context : h->m.max_model_len, sampling != 0);
+  if (rc == (int)cudaErrorMemoryAllocation) { h->wide.no_room = true; (void)cudaGetLastError(); return 0; }
+  if (graphs_out) *graphs_out = (int32_t)(h->graphs.size() + h->wide.graphs.size());
+  return rc;
 }
 
 int dfb_store_kvcache(const void* key, const void* value, int64_t key_stride, int64_t value_stride, void* k_cache,
@@ -1989,12 +2043,16 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
   }
   int first_error = 0;
   // More rows than one launch of the ordinary kernels holds: all of them in one pass over the weights.  (After a tuning
-  // option has been set the step keeps to the kernels that the option speaks of, in launches of 8 rows.)
-  if (n_live > kMaxRows && wide_usable(h)) {
+  // option has been set the step keeps to the kernels that the option speaks of, in launches of 8 rows; also where the
+  // buffers find no room: an engine that gave its memory to the cache goes on.)
+  if (n_live > kMaxRows && wide_usable(h) && !h->wide.no_room) {
+    const int rc = wide_prepare(h);
+    if (rc == (int)cudaErrorMemoryAllocation) { h->wide.no_room = true; (void)cudaGetLastError(); }
+    else if (rc) return rc;
+  }
+  if (n_live > kMaxRows && wide_usable(h) && !h->wide.no_room) {
     if (h->burst_steps) return DFB_E_BAD_ARG;
     DfbHandle::Wide& w = h->wide;
-    int rc = wide_prepare(h);
-    if (rc) return rc;
     int* hs = w.host_stage;
     int halves = 0, wholes = 0;
     bool sampled = false;
@@ -2012,7 +2070,12 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
       if (on) { halves += (int)(s->position / (kAttnChunk / 2)) + 1; wholes += (int)(s->position / kAttnChunk) + 1; }
       sampled = sampled || t > 1e-10f;
     }
-    rc = wide_step(h, n_live, halves, wholes, sampled, (cudaStream_t)stream);
+    const int rc = wide_step(h, wide_geometry(h, n_live, halves, wholes), sampled, (cudaStream_t)stream);
+    if (rc == (int)cudaErrorMemoryAllocation && h->use_graph) {      // (of its graph: nothing has run)
+      h->wide.no_room = true;
+      (void)cudaGetLastError();
+      return dfb_slots_step(h, sampled_tokens, emitted, stream);
+    }
     if (rc) return rc;
     if (!poll_published(w.host_tokens + kWideRows + 4, w.published)) DFB_CUDA(cudaStreamSynchronize((cudaStream_t)stream));
     for (int r = 0; r < n_live; ++r) {

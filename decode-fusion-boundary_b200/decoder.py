@@ -155,6 +155,7 @@ class StreamDecoder:
                 everyone = tensor_parallel.gather_bytes(mine.raw)
                 native.check(self._lib.dfb_tp_open_peers(handle, b"".join(everyone)), "dfb_tp_open_peers")
 
+        self._warmed = 0             # kinds of steps whose graphs have been prepared
         # persistent per-step buffers: no allocation on the step path
         self._result = torch.zeros(native.DFB_MAX_ROWS + 4, dtype=torch.int32, device="cuda")
         self._result_ptr = self._result.data_ptr()
@@ -214,19 +215,27 @@ class StreamDecoder:
             f"(kernel {st.detail[0]}, index {st.detail[1]}, value {st.detail[2]})")
 
     # -- decode --------------------------------------------------------------
-    WARM_BURST, WARM_DEVICE, WARM_DEVICE_TOKENS, WARM_HOST, WARM_SAMPLING = 1, 2, 4, 8, 16
+    WARM_BURST, WARM_DEVICE, WARM_DEVICE_TOKENS, WARM_HOST, WARM_SAMPLING, WARM_NO_SLOTS = 1, 2, 4, 8, 16, 32
 
     def warm(self, max_rows: int | None = None, max_context: int | None = None,
              kinds: int = WARM_DEVICE_TOKENS | WARM_HOST) -> int:
         """Capture the graphs of every step geometry ahead of time (``dfb_warm``; the counterpart of
         ``ModelRunner.capture_cudagraph``).  The default prepares what ``MegakernelBackend`` calls: the
-        host-buffer step of ``decode`` and the device-pointer step of ``decode_batch``.  Returns the number of
-        graphs held."""
+        host-buffer step of ``decode`` and the device-pointer step of ``decode_batch``; with 8 rows also the steps
+        of more slots than that, unless ``WARM_NO_SLOTS`` says otherwise (a ``SlotRuntime`` then prepares them).
+        Returns the number of graphs held."""
         n = C.c_int32(0)
         self._native.check(self._lib.dfb_warm(self._handle, int(max_rows or self._max_rows),
                                               int(max_context or self._max_model_len), int(kinds), C.byref(n)),
                            "dfb_warm")
+        self._warmed |= int(kinds)
         return n.value
+
+    def warm_slots(self) -> None:
+        """The graphs and buffers of the steps of 9 to 32 slots, if this decoder's other steps have been prepared."""
+        if self._warmed & self.WARM_HOST:
+            self._native.check(self._lib.dfb_warm_slots(self._handle, self._max_model_len,
+                                                        self._warmed & self.WARM_SAMPLING, None), "dfb_warm_slots")
 
     def set_seed(self, seed: int) -> None:
         """Seed of the sampling noise; restarts the noise stream (``dfb_set_seed``)."""

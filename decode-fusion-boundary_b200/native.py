@@ -50,7 +50,7 @@ EXPORTS = (
     "dfb_launch_linear", "dfb_launch_rmsnorm_gateup_swiglu", "dfb_launch_lmhead_argmax",
     "dfb_lmhead_argmax_noalloc", "dfb_set_tensor_parallel", "dfb_tp_window_handle", "dfb_tp_open_peers",
     "dfb_tp_open_loopback", "dfb_decode_step_host_sampled", "dfb_set_seed", "dfb_launch_lmhead_sample",
-    "dfb_decode_burst_enqueue", "dfb_decode_burst_collect", "dfb_decode_burst_host", "dfb_warm",
+    "dfb_decode_burst_enqueue", "dfb_decode_burst_collect", "dfb_decode_burst_host", "dfb_warm", "dfb_warm_slots",
     "dfb_store_kvcache", "dfb_slot_set", "dfb_slot_get", "dfb_slots_step", "dfb_slots_run",
     "dfb_prefill_attention", "dfb_wait_tokens", "dfb_prefill_attention_rows",
 )
@@ -145,6 +145,7 @@ def lib() -> C.CDLL:
     L.dfb_wait_tokens.argtypes = [vp, vp, vp]
     L.dfb_set_seed.argtypes = [vp, C.c_uint64]
     L.dfb_warm.argtypes = [vp, i32, i32, i32, vp]
+    L.dfb_warm_slots.argtypes = [vp, i32, i32, vp]
     L.dfb_prefill_attention.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                                         i32, i32, i32, f32, vp, i32, i32, i32, vp, vp]
     L.dfb_prefill_attention_rows.argtypes = L.dfb_prefill_attention.argtypes[:-1] + [C.c_int64, C.c_int64, vp]

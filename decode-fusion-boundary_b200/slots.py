@@ -26,6 +26,7 @@ class SlotRuntime:
         self._temperatures: dict[int, float] = {}
         self._tokens = (C.c_longlong * self.max_slots)()
         self._emitted = (C.c_int32 * self.max_slots)()
+        decoder.warm_slots()                     # no step allocates or captures
 
     def _stream(self) -> int:
         return self._dec._stream()

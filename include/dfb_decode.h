@@ -251,10 +251,13 @@ int dfb_set_option(DfbHandle* h, int option, int value);
  * context crosses a chunk or block boundary: the counterpart of ModelRunner.capture_cudagraph
  * (engine/model_runner.py:379-416), which captures the torch path's graphs for its batch sizes at start-up.
  * `kinds` is a bit mask of the entry points to prepare: 1 = bursts, 2 = dfb_decode_step without out_tokens,
- * 4 = dfb_decode_step with out_tokens, 8 = the host-buffer steps, 16 = also the sampling variants of those.
+ * 4 = dfb_decode_step with out_tokens, 8 = the host-buffer steps and, with max_rows = DFB_MAX_ROWS, those of the
+ * slots (dfb_warm_slots), 16 = also the sampling variants of those, 32 = not those of more than DFB_MAX_ROWS slots.
  * `graphs_out` (may be NULL) receives the number of graphs the decoder holds afterwards.  Options set later
  * drop the graphs again. */
 int dfb_warm(DfbHandle* h, int32_t max_rows, int32_t max_context, int32_t kinds, int32_t* graphs_out);
+/* The same for the slots' steps of more than DFB_MAX_ROWS rows alone, with their buffers (about 18 MB). */
+int dfb_warm_slots(DfbHandle* h, int32_t max_context, int32_t sampling, int32_t* graphs_out);
 
 /* Enqueue one decode step on `stream` (no host synchronisation, no allocation
  * after the first call for a given (rows, bucket)).  Replaces tg_launch_decode +
@@ -308,12 +311,13 @@ int dfb_decode_burst_host(DfbHandle* h, int32_t rows, int32_t steps, const int64
 /* Fixed-slot runtime: the decode side of a continuous-batching engine as the reference designed it (fixed rows
  * whose sequences come and go, `set_slot(row, active, start_pos, ...)`, a token callback after every step:
  * backends/megakernel/row_contract.py:1-24, csrc/tg_abi.h:185-199) and never built.  DFB_MAX_SLOTS slots live in
- * the decoder; a step packs the live ones, in slot order, into launches of at most DFB_MAX_ROWS rows — more live
- * slots than that become several launches per step — runs them from host state (one packed copy each), and then
- * holds each slot's new token and position.  A slot whose next position lies beyond its block table (the
+ * the decoder; a step packs the live ones, in slot order, into one launch of up to DFB_MAX_ROWS rows, or, when more
+ * are live, runs all of them in one pass over the weights (in launches of DFB_MAX_ROWS where that is not to be had:
+ * a tensor-parallel or persistent decoder, tuning options, no room for its buffers), from host state (one packed
+ * copy), and then holds each slot's new token and position.  A slot whose next position lies beyond its block table (the
  * scheduler has to append a block and call dfb_slot_set again) or beyond the model length sits the step out.
  * A retired slot (active = 0) is simply no longer launched, so its freed blocks are never written again; every
- * geometry is a cached graph (dfb_warm), so a change of the live set captures nothing.
+ * geometry is a cached graph (dfb_warm, dfb_warm_slots), so a change of the live set captures nothing.
  *   dfb_slot_set   admit (active = 1: next input token, pre-decode length, block table, temperature; 0 = greedy)
  *                  or retire (active = 0) a slot; also the way to give a live slot a longer block table;
  *   dfb_slot_get   the slot's state as the runtime holds it;
@@ -403,7 +407,7 @@ int dfb_launch_lmhead_sample(DfbHandle* h, const void* hidden_in, const void* re
  * (num_slots = num_blocks * block_size of one layer; row_elems = kv_heads * head_dim).  slot -1 is skipped as in
  * the reference; any other slot outside [0, num_slots) is skipped too and recorded in `status` (NULL, or a device
  * int32[4] that receives {DFB_STATUS_BAD_SLOT, kernel id, token index, slot}).  All pointers are device pointers;
- * nothing is allocated and nothing synchronised.  Prefill ATTENTION itself stays on the engine's torch path. */
+ * nothing is allocated and nothing synchronised. */
 int dfb_store_kvcache(const void* key, const void* value, int64_t key_stride, int64_t value_stride, void* k_cache,
                       void* v_cache, const int32_t* slot_mapping, int32_t n_tokens, int32_t row_elems,
                       int64_t num_slots, int32_t* status, dfb_stream_t stream);

@@ -94,3 +94,155 @@ def test_first_wide_step_beside_a_busy_default_stream(model, cuda_device):
                             before_steps=lambda: [torch.mm(a, a) for _ in range(30)])
     torch.cuda.synchronize()
     assert got == want and torch.equal(kv_got, kv_want)
+
+
+def _held(dec):
+    """Graphs that the decoder holds (of a refused call, which prepares nothing)."""
+    import ctypes as C
+    n = C.c_int32(0)
+    assert dec._lib.dfb_warm(dec._handle, 0, 1, 1, C.byref(n)) == -1
+    return n.value
+
+
+def _tables(n, lengths):
+    first = np.cumsum([0] + [lengths[i] // 256 + 2 for i in range(n)])
+    return [list(range(first[i], first[i + 1])) for i in range(n)], int(first[-1])
+
+
+@pytest.mark.parametrize("sampled", [False, True])
+def test_serving_on_the_default_kernels(model, cuda_device, sampled):
+    """Sequences that join, retire, change slots and wait for a block, with 6 to 20 live slots (8 and 9 among them), on the
+    kernels that a user gets, step for step beside a decoder that takes launches of 8.  The steps capture and
+    allocate nothing."""
+    from dfb_b200 import native
+    from dfb_b200.slots import SlotRuntime
+    g, w, _ = model
+    n_seq = 26
+    rng = np.random.Generator(np.random.Philox(key=95))
+    lens = [int(x) for x in rng.integers(1, 1400, n_seq)]
+    lens[2], lens[5] = 255, 511                                        # run out of their first blocks after one token
+    tables, blocks = _tables(n_seq, lens)
+    budget = [int(x) for x in rng.integers(3, 16, n_seq)]
+    temps = [4.0 if sampled and i % 5 == 0 else 0.0 for i in range(n_seq)]
+    history = torch.from_numpy(rng.standard_normal(tuple(O.new_kv_cache(g, blocks, BF).shape), dtype=np.float32) * 0.5).to(BF).cuda()
+    kinds = dict(kinds=8 | 16 | 32)                                    # host buffers, sampling; the slots' by the runtime
+    sides = []
+    for wide in (True, False):
+        kv = history.clone()
+        dec = H.make_decoder(w, kv)
+        if not wide:
+            dec.set_option(native.DFB_OPT_BULK_X, 1)
+        dec.set_seed(11)
+        dec.warm(**kinds)
+        sides.append((SlotRuntime(dec), dec, kv))
+    held, free = _held(sides[0][1]), None
+    assert held > _held(sides[1][1])                                   # the wide steps' graphs are there
+    slot_of, order, left = {}, list(range(n_seq)), dict(enumerate(budget))
+    free_slots = [int(x) for x in rng.permutation(32)]
+    seen, misses, draws, waited = set(), 0, 0, set()
+
+    def admit(i):
+        slot_of[i] = free_slots.pop(0)
+        for rt, _, _ in sides:
+            rt.admit(slot_of[i], 100 + 7 * i, lens[i], tables[i][:lens[i] // 256 + 1], temps[i])
+
+    targets = [20, 20, 18, 9, 8, 9, 6, 12, 20, 17, 16, 9, 8, 7, 6, 5, 4, 3]
+    for step in range(200):
+        while order and len(slot_of) < targets[min(step, len(targets) - 1)]:
+            admit(order.pop(0))
+        if not slot_of:
+            break
+        a, b = sides[0][0].step(), sides[1][0].step()
+        if step == 1:
+            torch.cuda.synchronize()
+            free = torch.cuda.mem_get_info()[0]
+        assert set(a) == set(b)
+        seen.add(len(a))
+        for i, slot in list(slot_of.items()):
+            if slot not in a:                                          # waits for its next block
+                waited.add(i)
+                for rt, _, _ in sides:
+                    rt.extend(slot, tables[i])
+                continue
+            if temps[i]:
+                draws += 1
+                if a[slot] != b[slot]:                                 # a near tie: both go on with the same token
+                    misses += 1
+                    _, _, pos = sides[1][0].state(slot)
+                    sides[1][0].admit(slot, a[slot], pos, tables[i][:pos // 256 + 1], temps[i])
+            else:
+                assert a[slot] == b[slot], (step, i)
+            left[i] -= 1
+            if left[i] == 0 or (step in (3, 5) and len(slot_of) > targets[step + 1]):
+                for rt, _, _ in sides:
+                    rt.retire(slot)
+                free_slots.append(slot_of.pop(i))
+    assert not order and waited >= {2, 5} and {8, 9} <= seen and max(seen) == 20, (seen, waited)
+    assert misses <= draws // 20, (misses, draws)
+    assert _held(sides[0][1]) == held
+    torch.cuda.synchronize()
+    assert torch.cuda.mem_get_info()[0] == free
+    kv_a, kv_b = sides[0][2], sides[1][2]
+    assert torch.equal((kv_a != history).any(-1), (kv_b != history).any(-1))
+    assert float((kv_a.float() - kv_b.float()).abs().max()) <= 2.0 ** -5
+    for _, dec, _ in sides:
+        assert dec.status()[0] == 0
+        dec.close()
+
+
+def test_warm_prepares_the_wide_steps(model, cuda_device):
+    """``dfb_warm`` of the host-buffer steps of 8 rows covers the slots' steps whatever their number, as it says."""
+    from dfb_b200.slots import SlotRuntime
+    g, w, history = model
+    dec = H.make_decoder(w, history.clone())
+    held = dec.warm(kinds=dec.WARM_HOST | dec.WARM_SAMPLING)
+    assert held == _held(dec)
+    rt = SlotRuntime(dec)
+    first = 0
+    for i in range(32):
+        rt.admit(i, 100 + 7 * i, LENGTHS[i], list(range(first, first + LENGTHS[i] // 256 + 1)), 0.5 if i % 4 == 0 else 0.0)
+        first += LENGTHS[i] // 256 + 1
+        if i >= 8:
+            rt.step()
+            for j in range(i + 1):                                      # the same position again
+                rt.admit(j, 100 + 7 * j, LENGTHS[j], list(range(sum(n // 256 + 1 for n in LENGTHS[:j]),
+                                                                sum(n // 256 + 1 for n in LENGTHS[:j + 1]))), 0.5 if j % 4 == 0 else 0.0)
+    assert _held(dec) == held
+    dec.close()
+
+
+def test_no_room_for_the_wide_buffers(model, cuda_device):
+    """A decoder whose memory went to the cache before the first step of more than 8 slots takes launches of 8."""
+    from dfb_b200.slots import SlotRuntime
+    g, w, history = model
+    want, kv_want = _step(w, history, 12, None, wide=False)
+    kv = history.clone()
+    dec = H.make_decoder(w, kv)
+    rt = SlotRuntime(dec)                                              # not warmed: prepares nothing
+    dec.warm(kinds=dec.WARM_HOST | dec.WARM_NO_SLOTS)
+    tables = [list(range(sum(n // 256 + 1 for n in LENGTHS[:i]), sum(n // 256 + 1 for n in LENGTHS[:i + 1]))) for i in range(12)]
+    for live in (range(8), range(8, 12)):                              # both launches have run once
+        for i in live:
+            rt.admit(i, 100 + 7 * i, LENGTHS[i], tables[i])
+        rt.step()
+        for i in live:
+            rt.retire(i)
+    kv.copy_(history)
+    for i in range(12):
+        rt.admit(i, 100 + 7 * i, LENGTHS[i], tables[i])
+    torch.cuda.synchronize()
+    hold = []
+    try:
+        for chunk in (1 << 30, 1 << 26, 12 << 20):
+            try:
+                while True:
+                    hold.append(torch.empty(chunk, dtype=torch.uint8, device="cuda"))
+            except torch.OutOfMemoryError:
+                pass
+        got = rt.step()
+    finally:
+        del hold
+        torch.cuda.empty_cache()
+    assert [got] == want and torch.equal(kv, kv_want)
+    assert dec.status()[0] == 0
+    dec.close()
