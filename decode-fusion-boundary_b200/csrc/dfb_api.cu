@@ -59,7 +59,8 @@ int env_int(const char* name, int fallback) {
 
 // Tuning knobs of the kernel chain.  Every decoder owns a copy (dfb_set_option
 // changes that decoder only); the standalone dfb_launch_* entry points use the
-// defaults.
+// defaults.  The values below hold unless the environment changes them
+// (options_from_environment).
 struct ChainOptions {
   int row_max_rows = 1;        // largest batch that takes the FP32 GEMV kernels (0 = never); measured: two rows run
                                // 1-2 % faster on the tensor-core kernels, one row 18 % slower
@@ -78,32 +79,31 @@ struct ChainOptions {
   int look_ahead = 0;
   int lmhead_ahead_mb = 32;    // MB of the LM head requested by the last layer
   unsigned long long peer_wait_ns = kPeerWaitNs;   // tensor parallel: limit of a wait for a peer
-  // batches above row_max_rows: K = 1024 projections on tcgen05.mma (dfb_tcgemv.cuh).  DFB_TCGEN05=<mask> in the
-  // environment changes the initial value (a diagnostic switch for the handle-less standalone launchers).
+  // batches above row_max_rows: K = 1024 projections on tcgen05.mma (dfb_tcgemv.cuh).
   // Bit mask: 1 = QKV, 2 = gate/up, 4 = LM head.  Default: the LM head only (equal to the mma.sync kernel in time);
   // the two per-layer projections are parity-tested but measured slower inside the chain than their mma.sync
   // counterparts (their longer post-dependency path: bulk copies of x, two issue loops, accumulator read).
-  int tcgen05 = env_int("DFB_TCGEN05", 4);
+  int tcgen05 = 4;
   int carve_tc = 100;          // ... whose chain asks for all of an SM's L1/shared memory as shared memory
   int attn_auto = 1;           // 1: the cluster attention kernel (dfb_attncluster.cuh) where attention_cluster() says so; 0
                                // once one of the attention options below has been set: the kernel they select runs
-  int attn_cluster = env_int("DFB_ATTN_CLUSTER", 148);  // attention grids of at most this many CTAs (and 2..16 chunks
+  int attn_cluster = 148;  // attention grids of at most this many CTAs (and 2..16 chunks
                                // per row) launch the chunks of one (row, KV head) as a thread-block cluster that
                                // merges its partial results through distributed shared memory instead of global
                                // memory and a ticket; 0 = never.  Larger grids lose more to the co-scheduling of
                                // 16-CTA clusters than the merge saves (batch 8 / context 512: 1,009 against 709 us)
-  int attn_chunk128 = env_int("DFB_ATTN_CHUNK128", 1);    // 1: context bounds of 65..128 tokens run ONE 128-position chunk
+  int attn_chunk128 = 1;    // 1: context bounds of 65..128 tokens run ONE 128-position chunk
                                // per row and KV head (256 threads, twice the K/V per thread) instead of two merged
                                // 64-position chunks (batch 1: 461 against 474 us per step); N > 1: also every grid
                                // that 128-position chunks bring to at most N CTAs (measured 2-5 % slower than
                                // 64-position chunks with a cluster merge); 0: never
-  int attn_ring32_min = env_int("DFB_ATTN_RING32", 0);   // steps with context bound <= 1024 whose rows x 32-position
+  int attn_ring32_min = 0;   // steps with context bound <= 1024 whose rows x 32-position
                                // chunks reach this value (and that the rule below does not take) run the streaming
                                // kernel with 32 positions per CTA; 0 = never.  Off: the streaming kernel's fixed
                                // cost per CTA (q/k norm and rotation for all eight heads, ring start-up) loses to
                                // the register-resident kernel at these sizes (batch 8 / context 512: 811 against
                                // 709 us per step, batch 4: 769 against 636)
-  int reg_weights = env_int("DFB_REG_WEIGHTS", 0);   // batches above row_max_rows, a bit mask: 1 = QKV and gate/up,
+  int reg_weights = 0;   // batches above row_max_rows, a bit mask: 1 = QKV and gate/up,
                                // 2 = o_proj and down_proj, 4 = LM head keep their weights in registers (loaded straight
                                // from global memory in MMA fragment order, pair_gemv_kernel<0, ...> and
                                // reg_store_gemv_kernel) instead of shared-memory stages, so that a kernel's CTAs fit
@@ -111,7 +111,7 @@ struct ChainOptions {
                                // measured slower at every batch (batch 8 / context 512: 758 us with bit 1, 719 with
                                // bit 2, 786 with both, against 709): at 2-8 rows a successor that streams its
                                // weights beside the running kernel takes bandwidth from that kernel's own stream
-  int host_io = env_int("DFB_HOST_IO", 7);   // steps from host buffers: 1 = the inputs reach the staging area by a one-warp
+  int host_io = 7;   // steps from host buffers: 1 = the inputs reach the staging area by a one-warp
                                // kernel that reads pinned host memory, 2 = tokens and status are written to pinned
                                // host memory by a one-warp kernel, instead of copy nodes in the step's graph; 4 = the
                                // host then polls the sequence word that follows the tokens into pinned memory
@@ -120,7 +120,23 @@ struct ChainOptions {
                                // streaming attention kernel (dfb_attnring.cuh), which needs about two CTAs per SM
                                // to pay; smaller ones stay on the register-resident kernel; 0 = never
 };
-const ChainOptions kDefaultOptions;
+// Diagnostic switches, also for the handle-less standalone launchers: an initial value from the environment counts like
+// one that was set.
+ChainOptions options_from_environment() {
+  ChainOptions o;
+  o.tcgen05 = env_int("DFB_TCGEN05", o.tcgen05);
+  o.attn_cluster = env_int("DFB_ATTN_CLUSTER", o.attn_cluster);
+  o.attn_chunk128 = env_int("DFB_ATTN_CHUNK128", o.attn_chunk128);
+  o.attn_ring32_min = env_int("DFB_ATTN_RING32", o.attn_ring32_min);
+  o.reg_weights = env_int("DFB_REG_WEIGHTS", o.reg_weights);
+  o.host_io = env_int("DFB_HOST_IO", o.host_io);
+  for (const char* name : {"DFB_ATTN_CLUSTER", "DFB_ATTN_CHUNK128", "DFB_ATTN_RING32"}) {
+    const char* v = getenv(name);
+    if (v && *v) o.attn_auto = 0;
+  }
+  return o;
+}
+const ChainOptions kDefaultOptions = options_from_environment();
 
 // Function attributes are per device: remember what was set for (device, function).
 std::mutex g_attr_mu;
@@ -304,7 +320,7 @@ struct DfbHandle {
   bool use_pdl = true;
   int lmhead_ctas = 0;
   bool trace_on = false;
-  ChainOptions opt;              // tuning knobs of this decoder's kernel chain
+  ChainOptions opt = options_from_environment();   // tuning knobs of this decoder's kernel chain
   int step_mode = 0;             // 0: chain of per-op kernels (default); 1: one persistent kernel per step
   int persist_ctas = 0;          // grid of the persistent kernel (0 = one CTA per SM)
   int trace_entries = 0;         // timeline entries written by the last traced step
@@ -2042,9 +2058,8 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
     live[n_live++] = i;
   }
   int first_error = 0;
-  // More rows than one launch of the ordinary kernels holds: all of them in one pass over the weights.  (After a tuning
-  // option has been set the step keeps to the kernels that the option speaks of, in launches of 8 rows; also where the
-  // buffers find no room: an engine that gave its memory to the cache goes on.)
+  // More rows than one launch of the ordinary kernels holds: all of them in one pass over the weights.  (In launches
+  // of 8 rows where wide_usable says so, or the buffers find no room: an engine that gave its memory to the cache goes on.)
   if (n_live > kMaxRows && wide_usable(h) && !h->wide.no_room) {
     const int rc = wide_prepare(h);
     if (rc == (int)cudaErrorMemoryAllocation) { h->wide.no_room = true; (void)cudaGetLastError(); }

@@ -25,3 +25,32 @@ def test_cluster_attention(small, ctx_lens, scattered):  # noqa: F811
                                                     row_active=[int(x) for x in active] if active else None)
     assert float((out.float() - want.float()).abs().max()) <= 2.0 ** -6
     assert torch.equal(kv_got, kv_want)            # the active rows' new K/V bit-exactly, nothing else touched
+
+
+def test_attention_options_from_the_environment(cuda_device, monkeypatch):
+    """The environment's initial value of an attention option counts like one that is set: the kernel it speaks of (the
+    streaming one, whose order of sums shows in the caches' last bits) runs where the cluster kernel would."""
+    from dfb_b200 import native
+    from oracle import qwen3_decode as O
+    from tests import harness as H
+
+    g = H.oracle_geometry(layers=3, vocab=2048)
+    w = O.make_weights(g, seed=23, norm="random").to(torch.bfloat16)
+    history = torch.randn(tuple(O.new_kv_cache(g, 16, torch.bfloat16).shape), generator=torch.Generator().manual_seed(24))
+    contexts = [130, 399, 200, 256, 257, 300, 171, 380]
+
+    def caches(env, opt):
+        if env:
+            monkeypatch.setenv("DFB_ATTN_RING32", "1")
+        kv = history.to(torch.bfloat16).cuda()
+        dec = H.make_decoder(w, kv)
+        if opt:
+            dec.set_option(native.DFB_OPT_ATTN_RING32, 1)
+        dec.decode_host([7 * r for r in range(8)], contexts, [[2 * r, 2 * r + 1] for r in range(8)])
+        dec.close()
+        monkeypatch.delenv("DFB_ATTN_RING32", raising=False)
+        return kv
+
+    default, chosen = caches(False, False), caches(False, True)
+    assert not torch.equal(default, chosen)                 # another kernel, another order of sums
+    assert torch.equal(caches(True, False), chosen)
