@@ -137,6 +137,15 @@ ChainOptions options_from_environment() {
   return o;
 }
 const ChainOptions kDefaultOptions = options_from_environment();
+// whether two sets of options take a step's kernels the same way (how inputs and results travel aside)
+bool same_chain(const ChainOptions& a, const ChainOptions& b) {
+  auto kernels = [](const ChainOptions& o) {
+    return std::make_tuple(o.row_max_rows, o.attn_wide_ctas, o.carve_fp32, o.carve_mma, o.late_trigger, o.pair_gemv, o.bulk_x,
+                           o.look_ahead, o.lmhead_ahead_mb, o.tcgen05, o.carve_tc, o.attn_auto, o.attn_cluster, o.attn_chunk128,
+                           o.attn_ring32_min, o.reg_weights, o.attn_ring_min);
+  };
+  return kernels(a) == kernels(b);
+}
 
 // Function attributes are per device: remember what was set for (device, function).
 std::mutex g_attr_mu;
@@ -321,6 +330,7 @@ struct DfbHandle {
   int lmhead_ctas = 0;
   bool trace_on = false;
   ChainOptions opt = options_from_environment();   // tuning knobs of this decoder's kernel chain
+  bool slots_wide = true;        // steps of more than kMaxRows slots may take the wide kernels
   int step_mode = 0;             // 0: chain of per-op kernels (default); 1: one persistent kernel per step
   int persist_ctas = 0;          // grid of the persistent kernel (0 = one CTA per SM)
   int trace_entries = 0;         // timeline entries written by the last traced step
@@ -386,7 +396,6 @@ struct DfbHandle {
     unsigned int published = 0;
     std::map<int, cudaGraphExec_t> graphs;      // by groups of 8 rows, attention grid, sampling
   } wide;
-  bool tuned = false;                // an option that selects kernels has been set: no wide steps
   void drop_graphs() {
     for (auto& kv : graphs) { cudaGraphExecDestroy(kv.second.exec); cudaGraphDestroy(kv.second.graph); }
     graphs.clear();
@@ -1179,8 +1188,10 @@ int run_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, 
 }
 
 // ---- steps of 9 to 32 rows (dfb_wide.cuh) ------------------------------------------------------------------
+// (an option that takes other kernels speaks of those of 1 to 8 rows: such a decoder keeps to them)
 bool wide_usable(const DfbHandle* h) {
-  return h->full_geometry && !h->sharded() && h->step_mode == 0 && !h->tuned && h->m.vocab % 16 == 0 &&
+  return h->full_geometry && !h->sharded() && h->step_mode == 0 && h->slots_wide && h->lmhead_ctas == 0 &&
+         same_chain(h->opt, ChainOptions()) && h->m.vocab % 16 == 0 &&
          h->m.max_model_len <= kMaxSplits * kAttnChunk;
 }
 
@@ -1670,6 +1681,10 @@ int dfb_set_option(DfbHandle* h, int option, int value) {
       if (value == 1 && (!h->full_geometry || h->sharded())) return DFB_E_GEOMETRY;  // built for the whole model only
       h->step_mode = value;
       return 0;
+    case DFB_OPT_SLOTS_WIDE:
+      if (value != 0 && value != 1) return DFB_E_BAD_ARG;
+      h->slots_wide = value != 0;
+      return 0;
     case DFB_OPT_PERSIST_CTAS:
       if (value < 0 || value > 4096) return DFB_E_BAD_ARG;
       h->persist_ctas = value;
@@ -1684,8 +1699,6 @@ int dfb_set_option(DfbHandle* h, int option, int value) {
     default: return DFB_E_BAD_ARG;
   }
   // every option above that did not return may change which kernels a captured step holds
-  if (option != DFB_OPT_TRACE && option != DFB_OPT_PEER_WAIT_US && option != DFB_OPT_HOST_IO && option != DFB_OPT_PERSIST_CTAS)
-    h->tuned = true;
   h->drop_graphs();
   return 0;
 }

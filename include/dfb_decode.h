@@ -193,7 +193,8 @@ typedef struct DfbStatus {
 #define DFB_OPT_ATTN_RING 19    /* steps whose rows x ceil(context bound / 64) reach this value run the streaming attention
                                   kernel (one CTA per row and 64-position chunk for all KV heads, K/V through a
                                   shared-memory ring fed by bulk copies) instead of the register-resident one;
-                                  0 = never (default 200) */
+                                  0 = never (default 200).  Full and long steps take the cluster attention kernel
+                                  ahead of this one until one of 8, 19, 20, 21, 22 has been set */
 #define DFB_OPT_ATTN_CLUSTER 20 /* register-resident attention kernel: grids of at most this many CTAs with 2..16
                                   chunks per row launch the chunks of one (row, KV head) as a thread-block cluster
                                   that merges its partial results through distributed shared memory (no global
@@ -217,7 +218,10 @@ typedef struct DfbStatus {
                                   memory by a one-warp kernel, instead of copy nodes in the step's graph; 4 = with 2:
                                   the call returns when the sequence word that the kernel writes after the tokens
                                   has arrived (polled in pinned memory) instead of synchronising the stream
-                                  (default 6) */
+                                  (default 7) */
+#define DFB_OPT_SLOTS_WIDE 25   /* dfb_slots_step with more than DFB_MAX_ROWS live slots: 1 (default) = all of them in one
+                                  pass over the weights, as long as the options that choose kernels (3, 7-13, 15, 16,
+                                  18-23) have their default values; 0 = launches of DFB_MAX_ROWS rows */
 #define DFB_OPT_TRACE 4       /* 1: every kernel records its timeline (see dfb_read_trace); default 0 */
 
 /* Build a decoder for one model on the current device: validates the geometry,

@@ -1,5 +1,5 @@
 """Steps of 9 to 32 slots in one pass over the weights (``dfb_wide.cuh``) against the same step taken in launches of 8
-rows (which a tuning option selects): one, several and all rows of the last group of 8, contexts of one token, around
+rows (DFB_OPT_SLOTS_WIDE = 0): one, several and all rows of the last group of 8, contexts of one token, around
 chunk and block boundaries and of the full model length, sampled rows in some groups (the noise stream is the one of the
 launches of 8) and an error status.  One step from the same state: the new cache rows and the tokens."""
 
@@ -37,7 +37,7 @@ def _step(w, history, n, temperatures, wide, steps=1, use_graph=True, before_ste
     kv = history.clone()
     dec = H.make_decoder(w, kv, use_graph=use_graph)
     if not wide:
-        dec.set_option(native.DFB_OPT_BULK_X, 1)       # the default value; a decoder with a tuned chain steps 8 rows at a time
+        dec.set_option(native.DFB_OPT_SLOTS_WIDE, 0)
     dec.set_seed(5)
     rt = SlotRuntime(dec)
     first = 0
@@ -131,7 +131,7 @@ def test_serving_on_the_default_kernels(model, cuda_device, sampled):
         kv = history.clone()
         dec = H.make_decoder(w, kv)
         if not wide:
-            dec.set_option(native.DFB_OPT_BULK_X, 1)
+            dec.set_option(native.DFB_OPT_SLOTS_WIDE, 0)
         dec.set_seed(11)
         dec.warm(**kinds)
         sides.append((SlotRuntime(dec), dec, kv))
@@ -245,4 +245,19 @@ def test_no_room_for_the_wide_buffers(model, cuda_device):
         torch.cuda.empty_cache()
     assert [got] == want and torch.equal(kv, kv_want)
     assert dec.status()[0] == 0
+    dec.close()
+
+
+@pytest.mark.parametrize("option,value,wide", [("BULK_X", 1, True), ("ROW_GEMV", 1, True), ("LMHEAD_CTAS", 0, True), ("HOST_IO", 0, True),
+                                               ("SLOTS_WIDE", 0, False), ("BULK_X", 0, False), ("ROW_GEMV", 2, False),
+                                               ("LMHEAD_CTAS", 64, False), ("TCGEN05", 7, False)])
+def test_options_and_the_wide_steps(model, cuda_device, option, value, wide):
+    """The kernels of 1 to 8 rows that an option chooses are taken at any number of slots; an option set to the value it
+    has anyway chooses none."""
+    from dfb_b200 import native
+    g, w, history = model
+    dec = H.make_decoder(w, history.clone())
+    dec.set_option(getattr(native, "DFB_OPT_" + option), value)
+    assert dec._lib.dfb_warm_slots(dec._handle, 2048, 0, None) == 0
+    assert (_held(dec) > 0) == wide
     dec.close()
