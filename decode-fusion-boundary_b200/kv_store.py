@@ -46,7 +46,7 @@ def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> No
         raise TypeError("slot_mapping must be an int32 CUDA tensor")
     if n == 0:
         return
-    blocks, block_size, _, _ = k_cache.shape
+    blocks, block_size = k_cache.shape[:2]
     code = _store(key.data_ptr(), value.data_ptr(), k_stride, v_stride, k_cache.data_ptr(), v_cache.data_ptr(),
                   slot_mapping.data_ptr(), n, d, blocks * block_size, status.data_ptr() if status is not None else None,
                   _stream())

@@ -65,3 +65,18 @@ def test_store_kvcache_skips_and_reports_a_bad_slot(cuda_device):
     assert float(flat[5].float().sum()) == heads * dim and float(flat[7].float().sum()) == heads * dim
     assert float(k_cache.float().sum()) == 2 * heads * dim              # only the two valid rows were written
     assert float(v_cache.float().sum()) == 2 * 2.0 * heads * dim
+
+
+def test_caches_of_flat_rows(cuda_device):
+    """``[num_blocks, block_size, kv_heads * head_dim]`` caches are the same memory and are taken as well."""
+    from dfb_b200.kv_store import store_kvcache
+
+    key, value = (torch.randn(37, 8, 128, generator=torch.Generator().manual_seed(s)).to(torch.bfloat16).cuda() for s in (1, 2))
+    slots = torch.arange(100, 137, dtype=torch.int32, device="cuda")
+    k_cache, v_cache = (torch.zeros(3, 64, 1024, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    store_kvcache(key, value, k_cache, v_cache, slots)
+    torch.cuda.synchronize()
+    for cache, rows in ((k_cache, key), (v_cache, value)):
+        want = torch.zeros_like(cache)
+        want.flatten(0, 1)[100:137] = rows.flatten(1, 2)
+        assert torch.equal(cache, want)
