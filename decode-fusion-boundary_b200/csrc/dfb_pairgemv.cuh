@@ -129,7 +129,6 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
   const bool row_per_warp = kNorm && a.ids == nullptr && a.res_in != nullptr && a.tp_mode != 2;
   if (kNorm && row_per_warp) {
     // warp b owns batch row b; lane l owns the 16-byte pieces l, l + 32, l + 64, l + 96 of the row
-    if (a.late_trigger) pdl_launch_dependents();
     const int b = warp;
     unsigned char* xrow = xsb + b * SM::kRowStride;
     if (b < a.rows) {
@@ -169,7 +168,7 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
         for (int e = 0; e < 8; ++e) y[e] = round_bf16(x[c][e] * rstd) * wf[e];
         uint4 o;
         o.x = pack_bf16(y[0], y[1]); o.y = pack_bf16(y[2], y[3]); o.z = pack_bf16(y[4], y[5]); o.w = pack_bf16(y[6], y[7]);
-        *reinterpret_cast<uint4*>(xrow + 16 * (32 * c + lane)) = o;    // in place: this lane read exactly these bytes
+        *reinterpret_cast<uint4*>(xrow + 16 * (32 * c + lane)) = o;
       }
     } else {
 #pragma unroll
@@ -260,7 +259,7 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
   uint4 xa[4];   // B fragments: x[batch g], this lane's 8 columns of each 32-column block
 #pragma unroll
   for (int j = 0; j < 4; ++j) xa[j] = *reinterpret_cast<const uint4*>(xsb + g * SM::kRowStride + 2 * (kbase + 32 * j));
-  if (a.late_trigger) pdl_launch_dependents();
+  if (a.late_trigger) pdl_launch_dependents();     // behind the barrier: every row has been read
   if (threadIdx.x == 0) trace_max(a.trace, 4);
 
   // ---- main loop over this CTA's tiles ----
@@ -473,7 +472,7 @@ __global__ void __launch_bounds__(K / 256 * 32, 2) reg_store_gemv_kernel(const G
 #pragma unroll
   for (int j = 0; j < 8; ++j)
     xa[j] = g < a.rows ? ldg_cg(a.x + (size_t)g * K + kbase + 32 * j) : make_uint4(0, 0, 0, 0);
-  if (a.late_trigger) pdl_launch_dependents();
+  if (a.late_trigger) pdl_launch_dependents();     // behind the barrier: every row has been read
   if (threadIdx.x == 0) trace_max(a.trace, 4);
 
   for (int it = 0; tile < a.n_tiles; tile += stride, ++it) {

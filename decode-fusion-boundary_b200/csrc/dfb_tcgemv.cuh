@@ -308,7 +308,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemv_kernel(const __grid_con
           if (a.res_in) rv[c] = ldg_cg(a.res_in + (size_t)b * kTcK + 8 * (32 * c + lane));
         }
       }
-      if (a.late_trigger) pdl_launch_dependents();   // the successor's prefetch traffic starts after x is here
       float x[4][8];
       float ss = 0.f;
 #pragma unroll
@@ -318,6 +317,10 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemv_kernel(const __grid_con
         unpack8(rv[c], rf);
 #pragma unroll
         for (int e = 0; e < 8; ++e) { x[c][e] = hf[e] + rf[e]; ss = fmaf(x[c][e], x[c][e], ss); }
+      }
+      if (a.late_trigger) {       // the successor's prefetch traffic starts after x is here
+        named_sync(1, kTcProThreads);
+        pdl_launch_dependents();
       }
       if (a.res_out && blockIdx.x == 0 && b < a.rows) {
 #pragma unroll

@@ -439,3 +439,13 @@ def test_waiting_for_tokens_of_a_captured_step_is_refused(cuda_device):
         assert dec.decode_rows(ids[0], pos, bt) == want[0]
     assert dec.status()[0] == 0
     dec.close()
+
+
+@pytest.mark.parametrize("tcgen05", [0, 7])
+@pytest.mark.parametrize("lens", [(9, 300, 64, 5, 130), (33, 1)])
+def test_late_trigger(cuda_device, tcgen05, lens):
+    """Kernels that let their successor start once they have read their inputs: the same step."""
+    from dfb_b200 import native
+
+    _check(H.run_parity_case(layers=2, vocab=2048, prompt_lens=lens, steps=2, seed=19,
+                             options={native.DFB_OPT_LATE_TRIGGER: 1, native.DFB_OPT_TCGEN05: tcgen05}))
