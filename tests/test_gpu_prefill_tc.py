@@ -73,8 +73,8 @@ def test_prefix_cache_block_sizes(cuda_device, block_size, q_heads, kv_heads):
 @pytest.mark.parametrize("lens,growing", [((512,), False), ((385,), False), ((449,), True), ((1024,), True), ((513, 1), False),
                                           ((640, 65, 128), True), ((1088,), True)])
 def test_keys_split_over_both_tiles(cuda_device, q_heads, kv_heads, lens, growing):
-    """Batches whose 128-row items all have an SM: odd and even numbers of key tiles, rows whose first own tile holds no
-    visible key, maxima that keep growing, and (1,088 tokens, 16 heads) the first size past the line."""
+    """Batches small enough for the split form: odd and even numbers of key tiles, rows whose first own tile holds no
+    visible key, maxima that keep growing."""
     from dfb_b200.kv_store import prefill_attention
 
     rng = np.random.Generator(np.random.Philox(key=sum(lens) + q_heads))
@@ -195,3 +195,89 @@ def test_scale_of_either_sign(cuda_device, scale, new, cached):
         want = _reference(q[start:start + n], ks[i], vs[i], n, total[i], scale)
         assert float((got[start:start + n].float().cpu() - want).abs().max()) <= 2.0 ** -6
         start += n
+
+
+def _split(lens, q_heads, longest, rows_known=True):
+    """The launcher's rule: whether the keys of an item go to both tiles."""
+    tiles = len(lens) * -(-longest // 128)
+    if rows_known:
+        tiles = min(tiles, sum(lens) // 128 + len(lens))
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    return tiles * q_heads <= (2 if longest >= 1024 else 1) * sms
+
+
+@pytest.mark.parametrize("block_size", [4, 16, 64, 256])
+@pytest.mark.parametrize("q_heads,kv_heads", [(16, 8), (24, 24)])
+@pytest.mark.parametrize("bad", [False, True])
+def test_prefix_cache_above_the_line(cuda_device, block_size, q_heads, kv_heads, bad):
+    """Batches of the prefix cache that are too large for the split form: head pairs and single heads, blocks smaller than
+    a key tile, NaN behind the ends, a block id outside the cache (its keys are read as zeros, and reported)."""
+    from dfb_b200 import native
+    from dfb_b200.kv_store import prefill_attention
+
+    rng = np.random.Generator(np.random.Philox(key=block_size + q_heads))
+    case = [(129 + 16 * i + extra, 129 + 14 * i) for i, extra in enumerate((0, 1, 300, 64, 128, 7, 512, 63, 256, 65, 40, 1000))]
+    d, lens = 128, [q for _, q in case]
+    assert not _split(lens, q_heads, max(lens))
+    need = [-(-k // block_size) for k, _ in case]
+    pool = rng.permutation(sum(need) + 2).tolist()
+    kc, vc = (torch.from_numpy(rng.standard_normal((sum(need) + 2, block_size, kv_heads, d), dtype=np.float32)).to(BF)
+              for _ in range(2))
+    tables = [[pool.pop() for _ in range(m)] for m in need]
+    q = torch.from_numpy(rng.standard_normal((sum(lens), q_heads, d), dtype=np.float32)).to(BF)
+    for (k_len, _), t in zip(case, tables):
+        if k_len % block_size:
+            vc[t[-1], k_len % block_size:] = float("nan")
+    cu_q, cu_k = (torch.tensor(np.cumsum([0, *x]), dtype=torch.int32, device="cuda") for x in (lens, [k for k, _ in case]))
+    bt = torch.tensor([t + [0] * (max(need) - len(t)) for t in tables], dtype=torch.int32)
+    where = (5, 100 // block_size)
+    if bad:
+        bt[where] = sum(need) + 2
+    status = torch.zeros(4, dtype=torch.int32, device="cuda")
+    got = prefill_attention(q.cuda(), kc.cuda(), vc.cuda(), cu_q, max(lens), d ** -0.5, cu_seqlens_k=cu_k,
+                            block_table=bt.cuda(), status=status).float().cpu()
+    start = 0
+    for i, ((k_len, q_len), t) in enumerate(zip(case, tables)):
+        k, v = (x[t].flatten(0, 1)[:k_len].clone() for x in (kc, vc))
+        if bad and i == where[0]:
+            for x in (k, v):
+                x[where[1] * block_size:(where[1] + 1) * block_size] = 0
+        want = _reference(q[start:start + q_len], k, v, q_len, k_len, d ** -0.5)
+        assert float((got[start:start + q_len] - want).abs().max()) <= 2.0 ** -6, (k_len, q_len)
+        start += q_len
+    assert status.tolist()[:1] + status.tolist()[2:] == ([native.DFB_STATUS_BAD_BLOCK, where[0], sum(need) + 2] if bad else [0, 0, 0])
+
+
+@pytest.mark.parametrize("known", [True, False])
+@pytest.mark.parametrize("q_heads,kv_heads,lens", [
+    (16, 8, (264, 65, 129, 200)), (16, 8, (449,)), (8, 8, (511, 8, 136)),                     # split form
+    (16, 8, (520, 193, 640, 64, 321, 72)), (24, 24, (136, 300, 257, 255, 129)), (16, 8, (2048, 1, 1025, 512, 319, 200))])
+def test_entry_points_with_and_without_sizes(cuda_device, known, q_heads, kv_heads, lens):
+    """``dfb_prefill_attention`` does not know where the tensors end and fetches the ends of the sequences in boxes of 8 rows
+    and pieces; ``dfb_prefill_attention_rows`` may be told.  Ends around multiples of 8 and 64, the last one at the
+    tensors' end, NaN in the rows of the second sequence (or behind the only one's)."""
+    from dfb_b200 import native
+
+    lib, d, n = native.lib(), 128, sum(lens)
+    gen = torch.Generator().manual_seed(n + q_heads)
+    pad = 0 if len(lens) > 1 else 64             # rows of nobody behind a single sequence
+    q, k, v = (torch.randn(n + pad, h, d, generator=gen).to(BF) for h in (q_heads, kv_heads, kv_heads))
+    spoilt = range(lens[0], lens[0] + (lens[1] if pad == 0 else pad))
+    for x in (k, v):
+        x[spoilt.start:spoilt.stop] = float("nan")
+    dev = [x.cuda() for x in (q, k, v)]
+    out = torch.zeros(n + pad, q_heads, d, dtype=BF, device="cuda")
+    cu = torch.tensor(np.cumsum([0, *lens]), dtype=torch.int32, device="cuda")
+    args = [*(x.data_ptr() for x in dev), out.data_ptr(), cu.data_ptr(), None, len(lens), max(lens), q_heads * d, kv_heads * d,
+            kv_heads * d, q_heads * d, q_heads, kv_heads, d, d ** -0.5, None, 0, 0, 0, None]
+    stream = torch.cuda.current_stream().cuda_stream
+    code = lib.dfb_prefill_attention_rows(*args, n + pad, n + pad, stream) if known else lib.dfb_prefill_attention(*args, stream)
+    assert code == 0
+    got, start = out.float().cpu(), 0
+    for i, m in enumerate(lens):
+        rows = slice(start, start + m)
+        if i != 1:
+            want = _reference(q[rows], k[rows], v[rows], m, m, d ** -0.5)
+            assert float((got[rows] - want).abs().max()) <= 2.0 ** -6, (i, m)
+        start += m
+    assert float(got[n:].abs().sum()) == 0.0
