@@ -2082,6 +2082,9 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
     if (h->burst_steps) return DFB_E_BAD_ARG;
     DfbHandle::Wide& w = h->wide;
     int* hs = w.host_stage;
+    // (a row without a number has no largest logit: its token is none)
+    for (int r = 0; r < n_live; ++r)
+      if (h->slots[live[r]].token < 0 || h->slots[live[r]].token >= h->embed_rows()) return DFB_E_BAD_ARG;
     int halves = 0, wholes = 0;
     bool sampled = false;
     for (int r = 0; r < kWideRows; ++r) {

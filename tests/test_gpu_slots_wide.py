@@ -1,7 +1,8 @@
 """Steps of 9 to 32 slots in one pass over the weights (``dfb_wide.cuh``) against the same step taken in launches of 8
 rows (DFB_OPT_SLOTS_WIDE = 0): one, several and all rows of the last group of 8, contexts of one token, around
 chunk and block boundaries and of the full model length, sampled rows in some groups (the noise stream is the one of the
-launches of 8) and an error status.  One step from the same state: the new cache rows and the tokens."""
+launches of 8).  One step from the same state: the new cache rows and the tokens.  Also against the fp32 oracle, as a
+serving loop, with an error status, with options, without room for its buffers."""
 
 import numpy as np
 import pytest
@@ -261,3 +262,66 @@ def test_options_and_the_wide_steps(model, cuda_device, option, value, wide):
     assert dec._lib.dfb_warm_slots(dec._handle, 2048, 0, None) == 0
     assert (_held(dec) > 0) == wide
     dec.close()
+
+
+def _admitted(dec, n):
+    from dfb_b200.slots import SlotRuntime
+    rt, first = SlotRuntime(dec), 0
+    for i in range(n):
+        blocks = (LENGTHS[i] + 2) // 256 + 1           # room for three steps
+        rt.admit(i, 100 + 7 * i, LENGTHS[i], list(range(first, first + blocks)))
+        first += blocks
+    return rt
+
+
+def test_wide_step_reports_an_error_status(model, cuda_device):
+    """A status that a kernel has recorded (here one of a device-pointer step whose position lies beyond the model length)
+    comes back from the wide step that finds it, once; its tokens are those of a step without it."""
+    from dfb_b200 import native
+    g, w, history = model
+    want, _ = _step(w, history, 12, None, wide=True)
+    dec = H.make_decoder(w, history.clone())
+    rt = _admitted(dec, 12)
+    free = torch.tensor([[history.shape[2] - 1]], dtype=torch.int32, device="cuda")
+    dec.enqueue_rows(torch.tensor([5], device="cuda"), torch.tensor([5000], device="cuda"), free)
+    with pytest.raises(RuntimeError, match=rf"device status {native.DFB_STATUS_BAD_POSITION} .*value 5000"):
+        rt.step()
+    assert {i: rt.state(i)[1] for i in range(12)} == want[0] and rt.state(3)[2] == LENGTHS[3] + 1
+    assert set(rt.step()) == set(range(12))
+    code, st = dec.status()
+    assert code == 0 and st.device_status == 0
+    dec.close()
+
+
+@pytest.mark.parametrize("wide", [True, False])
+def test_a_row_without_a_token_is_refused(model, cuda_device, wide):
+    """A sequence whose cache holds NaN has no largest logit; the step after it is refused, as the host-buffer step refuses
+    a token outside the embedding table, and goes on without that sequence."""
+    from dfb_b200 import native
+    g, w, history = model
+    kv = history.clone()
+    kv[:, :, 0, 10] = float("nan")                         # a position of slot 0
+    dec = H.make_decoder(w, kv)
+    dec.set_option(native.DFB_OPT_SLOTS_WIDE, int(wide))
+    rt = _admitted(dec, 12)
+    out = rt.step()
+    assert out[0] >= g.vocab and all(0 <= out[i] < g.vocab for i in range(1, 12))
+    with pytest.raises(RuntimeError, match="bad argument"):
+        rt.step()
+    rt.retire(0)
+    assert set(rt.step()) == set(range(1, 12))
+    assert dec.status()[0] == 0
+    dec.close()
+
+
+@pytest.mark.parametrize("n", [9, 20, 32])
+def test_wide_step_against_the_oracle(model, cuda_device, n):
+    g, w, history = model
+    got, kv_got = _step(w, history, n, None, wide=True)
+    kv = history.cpu()
+    first = np.cumsum([0] + [x // 256 + 1 for x in LENGTHS[:n]])
+    tables = [list(range(first[i], first[i + 1])) for i in range(n)]
+    logits, tokens = O.decode_step(w, kv, O.rope_cos_sin_table(g), [100 + 7 * i for i in range(n)], LENGTHS[:n], tables)
+    assert float((kv_got.cpu().float() - kv.float()).abs().max()) <= 2.0 ** -5
+    for i in range(n):
+        assert H.token_gap_ok(logits[i].float(), got[0][i], int(tokens[i])), i
