@@ -896,13 +896,15 @@ int launch_attention(Launcher& L, DfbHandle* h, int layer, const bf16* qkv, cons
 }
 
 // CTAs per (row, KV head) of the cluster attention kernel for a step of `rows` rows with contexts up to `chunks` x 64
-// tokens, or 0 where the chunked kernels are the faster ones.  Measured for 1 to 8 rows x 64 to 2,000 tokens: it wins
+// tokens, or 0 where the chunked kernels are the faster ones.  Measured over 1 to 8 rows x 3 to 32 chunks, all rows equally
+// long, with 0, 2, 4 and 8 CTAs (us per step, 0 / chosen): it wins
 //   * when 128 positions per CTA, what a CTA holds in flight, cover the context and the grid is large enough for the
-//     chunked kernel's many small CTAs to start late (8 rows x 192 tokens: 573 against 611 us a step; 3 rows x 512: 570
-//     against 592; 2 rows x 512 not: 561 against 547);
-//   * when there is enough to stream: from 80 chunks on (8 rows x 1,024: 720 against 813 us; 5 rows x 1,024: 698 against
-//     737; 4 rows x 1,280: 708 against 732).  Below that (6 rows x 768: 692 against 651) its second, nearly empty pass
-//     costs more than the chunked kernel's merge.
+//     chunked kernel's many small CTAs to start late (5 rows x 4 chunks 603 / 556 with 2 CTAs, 8 x 4 619 / 580, 3 x 8 593 /
+//     569 with 4, 8 x 8 649 / 642; 2 x 8 not: 553 / 559);
+//   * when there is enough to stream: from 80 chunks on (5 x 16 737 / 697 with 4, 8 x 10 741 / 693, 8 x 32 940 / 887, 4 x 20
+//     730 / 708 with 8, 3 x 32 762 / 717).  Between the two (8 x 9 658 / 685, 6 x 12 652 / 693, 4 x 16 639 / 652 with 8) its
+//     second, nearly empty pass costs more than the chunked kernel's merge.
+// Nowhere is another number of CTAs more than 1 % faster, but for 1 to 4 rows x 3 or 4 chunks (2 CTAs: 2 %).
 // All CTAs have to be resident together, two per SM; 16-CTA clusters wait too long for sixteen free places at a time
 // (2 rows x 905 tokens: 8 us until the last one started).
 int attention_cluster(int rows, int chunks) {
@@ -1082,7 +1084,8 @@ int enqueue_whole_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const St
     p.tokens = h->tokens; p.status = h->status; p.ids_out = h->st_ids(); p.positions_out = h->st_pos();
     p.rows = rows; p.embed_rows = h->embed_rows(); p.slot = h->burst_slot;
     p.ring = h->burst_ring; p.ring_status = h->burst_status(); p.ring_done = h->burst_done();
-    if (h->use_pdl && !h->sharded() && h->step_mode == 0) DFB_CUDA(launch_overlapped(publish_tokens_kernel, dim3(1), dim3(32), 0, stream, p));
+    if (h->use_pdl && !h->sharded() && h->step_mode == 0)
+      DFB_CUDA(launch_overlapped(publish_tokens_kernel, dim3(1), dim3(32), 0, stream, p));
     else DFB_CUDA((publish_tokens_kernel<<<1, 32, 0, stream>>>(p), cudaGetLastError()));
   } else if (io.publish || (io.host && (h->opt.host_io & 2))) {
     cudaLaunchConfig_t cfg = {};
@@ -1253,7 +1256,7 @@ int enqueue_wide(DfbHandle* h, int chunks, bool half, bool sampling, cudaStream_
   DFB_CUDA(cudaMemcpyAsync(w.stage, w.host_stage, sizeof(int) * kWideRows * (4 + h->max_pages), cudaMemcpyHostToDevice, stream));
   Launcher L{stream, h->use_pdl, h->trace_on ? h->trace : nullptr};
   L.opt = &h->opt;
-  L.carve = 100;      // every kernel of this chain is sized to fit beside its neighbour in all of the shared memory
+  L.carve = 100;      // up to 24 rows every per-layer kernel fits beside its neighbour in all of the shared memory
   auto norm = [&](const bf16* x, const int* ids, const bf16* res_in, bf16* res_out, const void* nw, const void* wt) {
     GemvArgs a = {};
     a.trace = L.next_trace();
@@ -1783,14 +1786,14 @@ int dfb_store_kvcache(const void* key, const void* value, int64_t key_stride, in
 }
 
 int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens_q,
-                          const int32_t* cu_seqlens_k, int32_t batch, int32_t max_seqlen_q, int64_t q_stride,
-                          int64_t k_stride, int64_t v_stride, int64_t out_stride, int32_t q_heads, int32_t kv_heads,
-                          int32_t head_dim, float scale, const int32_t* block_tables, int32_t block_table_stride,
-                          int32_t block_size, int32_t num_blocks, int32_t* status, int64_t q_rows, int64_t kv_rows,
+                               const int32_t* cu_seqlens_k, int32_t batch, int32_t max_seqlen_q, int64_t q_stride,
+                               int64_t k_stride, int64_t v_stride, int64_t out_stride, int32_t q_heads, int32_t kv_heads,
+                               int32_t head_dim, float scale, const int32_t* block_tables, int32_t block_table_stride,
+                               int32_t block_size, int32_t num_blocks, int32_t* status, int64_t q_rows, int64_t kv_rows,
                                dfb_stream_t stream) {
   if (!q || !k || !v || !out || !cu_seqlens_q || batch < 1 || max_seqlen_q < 1) return DFB_E_BAD_ARG;
   if (head_dim != kHeadDim || q_heads < 1 || kv_heads < 1 || q_heads % kv_heads) return DFB_E_GEOMETRY;
-  // 16-byte pieces of K / V rows and 4-byte pieces of Q / out rows: aligned bases, strides in multiples of 8
+  // rows are moved in 16-byte pieces and TMA boxes: aligned bases, strides in multiples of 8 elements
   if (q_stride < (int64_t)q_heads * head_dim || out_stride < (int64_t)q_heads * head_dim ||
       k_stride < (int64_t)kv_heads * head_dim || v_stride < (int64_t)kv_heads * head_dim)
     return DFB_E_BAD_ARG;
@@ -1803,10 +1806,9 @@ int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void
     while ((1 << block_shift) < block_size) ++block_shift;
   }
   // The shortest prompts (whose lengths max_seqlen_q bounds on the host) stay on the mma.sync kernel: its 64-row CTAs
-  // start and finish sooner.  Measured, it is the faster one up to 192 tokens while its CTAs take half of the SMs (128
-  // tokens: 5.4 against 6.6 us, 2 x 128 5.5 against 6.6; 3 x 128 no longer: 7.9 against 6.7; 200 tokens 7.9 against
-  // 7.2), and up to 64 tokens while each has an SM (6 x 64: 6.2 against 7.0) or the other kernel would need a second
-  // round (24 x 64: 8.6 against 10.6; 12 x 64 not: 7.6 against 7.1).
+  // start and finish sooner.  Measured (us, against the better form of the other kernel): 1 token 2.9 / 6.5, 64 4.2 / 6.8, 128
+  // 5.6 / 6.8, 2 x 128 6.6 / 6.8, 3 x 128 no longer 10.1 / 7.0; 12 x 64 even 7.7 / 7.7, 24 x 64 9.9 / 12.6 (the other kernel
+  // would need a second round).  From 160 tokens of one prompt on it is behind: 7.8 / 7.6, 192 8.6 / 7.7, 200 9.4 / 7.8.
   const int64_t short_ctas = (int64_t)batch * ((max_seqlen_q + kPfTile - 1) / kPfTile) * q_heads;
   const int sms = sm_count_cached();
   const int64_t pair_items = (int64_t)batch * ((max_seqlen_q + kPfRows - 1) / kPfRows) * q_heads / 2;
@@ -1825,18 +1827,20 @@ int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void
     DFB_CUDA(launch_overlapped(prefill_short_kernel, grid, dim3(128), kPfShortSmemBytes, (cudaStream_t)stream, s));
     return 0;
   }
-  // query heads that share a KV head go in pairs where their number allows it
   // Small batches: one head per item and the keys split over its two tiles.  The chain of an item is half as long, but
-  // its key tiles serve one head instead of two, so a CTA fetches twice as much per step (1.7 us a step against
-  // 1.15: L2).  It wins while every item has an SM (512 tokens 13.6 -> 9.7 us; 700 new behind 1,024 cached 33.9 -> 29.9),
-  // and up to two items per SM when the longest prompt's chain dominates (2,048 tokens 37.9 -> 29.1, 1,500 + 200 + 37
-  // 30.1 -> 24.5, 2 x 1,024 22.4 -> 20.4; 4 x 512 not: 14.6 against 15.6).
+  // its key tiles serve one head instead of two, so that a CTA fetches twice as much per step (1.7 us a step against 1.15:
+  // L2).  It wins while every item has an SM (us, split / not: 512 tokens 11.0 / 15.1, 2 x 512 12.2 / 15.8, 700 new behind
+  // 1,024 cached 32.1 / 37.8), and up to two items per SM when the longest prompt's chain dominates (2,048 tokens 32.7 /
+  // 44.0, 1,500 + 200 + 37 26.2 / 34.6, 2 x 1,024 22.8 / 26.2; 4 x 512 even: 17.5 / 17.8; five prompts with 1,924 new tokens
+  // behind 4,352, the longest one 1,000, not: 46.3 / 41.0).
   int64_t tiles = (int64_t)batch * ((max_seqlen_q + kPfRows - 1) / kPfRows);
   if (q_rows > 0 && q_rows / kPfRows + batch < tiles) tiles = q_rows / kPfRows + batch;
   const bool split = tiles * q_heads <= (max_seqlen_q >= 1024 ? 2 : 1) * sms;
+  // query heads that share a KV head go in pairs where their number allows it
   const bool pairs = !split && (q_heads / kv_heads) % 2 == 0;
-  auto kernel = split ? (block_tables ? prefill_tc_kernel<true, false, true> : prefill_tc_kernel<false, false, true>) : block_tables ? (pairs ? prefill_tc_kernel<true, true> : prefill_tc_kernel<true, false>)
-                             : (pairs ? prefill_tc_kernel<false, true> : prefill_tc_kernel<false, false>);
+  auto kernel = split ? prefill_tc_kernel<false, false, true> : pairs ? prefill_tc_kernel<false, true> : prefill_tc_kernel<false, false>;
+  if (block_tables)
+    kernel = split ? prefill_tc_kernel<true, false, true> : pairs ? prefill_tc_kernel<true, true> : prefill_tc_kernel<true, false>;
   cudaError_t e = ensure_dynamic_smem((const void*)kernel, kPfSmemBytes);
   if (e != cudaSuccess) return (int)e;
   PrefillArgs a = {};
@@ -1864,7 +1868,8 @@ int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void
   if (rc) return rc;
   // one CTA per SM (all of its tensor memory), fewer when the longest sequence bounds the work items below that
   const int64_t rows = pairs || split ? kPfRows : 2 * kPfRows;
-  const int64_t most = split ? tiles * q_heads : (int64_t)batch * ((max_seqlen_q + rows - 1) / rows) * (pairs ? q_heads / 2 : q_heads);
+  const int64_t most = split ? tiles * q_heads
+                             : (int64_t)batch * ((max_seqlen_q + rows - 1) / rows) * (pairs ? q_heads / 2 : q_heads);
   const int grid = (int)(most < sm_count_cached() ? most : sm_count_cached());
   DFB_CUDA(launch_overlapped(kernel, dim3(grid), dim3(pf_threads(split)), kPfSmemBytes, (cudaStream_t)stream, a));
   return 0;
@@ -1875,7 +1880,9 @@ int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out
                           int64_t k_stride, int64_t v_stride, int64_t out_stride, int32_t q_heads, int32_t kv_heads,
                           int32_t head_dim, float scale, const int32_t* block_tables, int32_t block_table_stride,
                           int32_t block_size, int32_t num_blocks, int32_t* status, dfb_stream_t stream) {
-  return dfb_prefill_attention_rows(q, k, v, out, cu_seqlens_q, cu_seqlens_k, batch, max_seqlen_q, q_stride, k_stride, v_stride, out_stride, q_heads, kv_heads, head_dim, scale, block_tables, block_table_stride, block_size, num_blocks, status, 0, 0, stream);
+  return dfb_prefill_attention_rows(q, k, v, out, cu_seqlens_q, cu_seqlens_k, batch, max_seqlen_q, q_stride, k_stride,
+                                    v_stride, out_stride, q_heads, kv_heads, head_dim, scale, block_tables,
+                                    block_table_stride, block_size, num_blocks, status, 0, 0, stream);
 }
 
 int dfb_set_seed(DfbHandle* h, uint64_t seed) {
@@ -2028,8 +2035,8 @@ int dfb_decode_step_host_sampled(DfbHandle* h, int32_t rows, const int64_t* inpu
 
 // ---- fixed-slot runtime --------------------------------------------------------------------------------
 // The decode side of a continuous-batching engine: DFB_MAX_SLOTS fixed slots whose sequences come and go
-// between steps; a step packs the live slots, in slot order, into launches of at most DFB_MAX_ROWS rows (every
-// geometry is a cached graph, so a change of the live set never captures once dfb_warm has run), advances
+// between steps; a step packs the live slots, in slot order, into one launch of at most DFB_MAX_ROWS rows or one wide step
+// (every geometry is a cached graph, so a change of the live set never captures once dfb_warm has run), advances
 // tokens and positions on the host side of the slots, and reports which slots emitted.
 int dfb_slot_set(DfbHandle* h, int32_t slot, int32_t active, int64_t token, int64_t position,
                  const int32_t* block_table, int32_t cols, float temperature) {

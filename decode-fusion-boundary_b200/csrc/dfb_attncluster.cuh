@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kCaThreads, 2) cluster_attention_kernel(const 
   constexpr int kSrc = kCaWarps * E + 4;            // floats of one source CTA's partial results (+ 4: bank offset)
   constexpr float kLog2e = 1.4426950408889634f;
   if (!a.late_trigger) pdl_launch_dependents();
-  if (CS > 1) cluster_arrive_relaxed();             // completed before the first push: the peers are running by then
+  cluster_arrive_relaxed();                         // completed before the first push: the peers are running by then
   const int rank = blockIdx.x, kvh = blockIdx.y, row = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int pg = tid >> 4, l16 = tid & 15;
@@ -287,21 +287,13 @@ __global__ void __launch_bounds__(kCaThreads, 2) cluster_attention_kernel(const 
     // (maximum, sum) of head lane & 1 for CTA lane / 2
     const float hm = __shfl_sync(0xffffffffu, M, 8 * (lane & 1)), hs = __shfl_sync(0xffffffffu, sum, 8 * (lane & 1));
     const int idx = (second ? kHeadDim : 0) + 8 * l16;        // of the 256 values
-    if (CS > 1) {
-      cluster_wait();
-      const uint32_t dst = peer_smem(&red[rank * kSrc + warp * E + idx % E], idx / E);
-      st_peer_f4(dst, r[0], r[1], r[2], r[3]);
-      st_peer_f4(dst + 16, r[4], r[5], r[6], r[7]);
-      if ((lane >> 1) < CS) st_peer_f2(peer_smem(&ml[rank * kCaWarps + warp][lane & 1], lane >> 1), hm, hs);
-      cluster_arrive();
-      cluster_wait();
-    } else {
-      float4* dst = reinterpret_cast<float4*>(&red[warp * E + idx]);
-      dst[0] = make_float4(r[0], r[1], r[2], r[3]);
-      dst[1] = make_float4(r[4], r[5], r[6], r[7]);
-      if (lane < 2) ml[warp][lane] = make_float2(hm, hs);
-      __syncthreads();
-    }
+    cluster_wait();
+    const uint32_t dst = peer_smem(&red[rank * kSrc + warp * E + idx % E], idx / E);
+    st_peer_f4(dst, r[0], r[1], r[2], r[3]);
+    st_peer_f4(dst + 16, r[4], r[5], r[6], r[7]);
+    if ((lane >> 1) < CS) st_peer_f2(peer_smem(&ml[rank * kCaWarps + warp][lane & 1], lane >> 1), hm, hs);
+    cluster_arrive();
+    cluster_wait();
   }
   if (tid == 0) trace_max(a.trace, 6);
 

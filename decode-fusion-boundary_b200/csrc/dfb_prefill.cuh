@@ -1,6 +1,7 @@
 // Causal prefill attention over short prompts: the computation of dfb_prefilltc.cuh (flash_attn_varlen_func with
 // causal = True, layers/attention.py:64-70) on mma.sync, for launches that are over before a tcgen05 kernel
-// has filled its pipeline (one prompt of 128 tokens: 5.8 us against 8.6 us; of 512 tokens: 15.7 against 14.5):
+// has filled its pipeline (one prompt of 64 tokens: 4.2 us against 6.8; of 128 tokens: 5.6 against 6.8; of 200 tokens no
+// longer: 9.4 against 7.8):
 //
 //   * q [N, q_heads, 128], k / v [N, kv_heads, 128] bf16, tokens of all sequences back to back, sequence b =
 //     rows [cu_seqlens[b], cu_seqlens[b + 1]); grouped-query attention (q head h reads KV head

@@ -1,15 +1,17 @@
 // Causal prefill attention on the 5th-generation tensor cores: the reference's flash_attn_varlen_func call
 // (causal = True, layers/attention.py:64-70), for both of its cases.  Without a prefix cache K / V are the
 // fresh projections of the same tokens; with one they are read from the paged cache through the block tables,
-// the keys of a sequence outnumber its queries, and query i attends to keys 0 .. i + (keys - queries).
+// the keys of a sequence outnumber its queries, and query i attends to keys 0 .. i + (keys - queries).  Two 128-row query
+// tiles per CTA, P in tensor memory as the A operand and warps of its own for the rescaling are the published FlashAttention
+// method for this architecture.
 //
 //   * A work item is 128 query rows of the two query heads that share a KV head (an even number of query heads
 //     per KV head), or 256 query rows of one head (an odd number): two M = 128 tiles that share every K / V
 //     tile.  Persistent CTAs, one per SM, walk the items from the longest to the shortest.
 //   * Warp 10 loads the two Q tiles and a ring of eight 16 KB stages (K and V tiles of 64 keys) with TMA boxes
 //     (128-byte swizzle), the end of a sequence as 8-row boxes and 16-byte cp.async pieces.
-//   * Warps 8 and 9 issue tcgen05.mma, each for one tile: S = Q K^T (K-major operands from shared memory) and O += P V with P as the A
-//     operand in tensor memory and V as an MN-major B operand.  Tensor memory holds O of both tiles (128 columns
+//   * Warps 8 and 9 issue tcgen05.mma, each for one tile: S = Q K^T (K-major operands from shared memory) and O += P V
+//     with P as the A operand in tensor memory and V as an MN-major B operand.  Tensor memory holds O of both tiles (128 columns
 //     each) and two S buffers per tile (64 columns); P overwrites the first half of its S.  S(j + 1) is computed
 //     while the softmax works on S(j), so the softmax never waits for a matrix product.  MMAs of one issuing
 //     thread execute in order: S(j + 2) may be issued behind the P V that still reads P(j) from the same columns.
@@ -265,8 +267,8 @@ struct PfWalk {
 // item of CTA `cta` in round r: rounds alternate direction, so that nobody always gets the longer one
 __device__ __forceinline__ int pf_item_index(int r, int cta, int ctas) { return r * ctas + ((r & 1) ? ctas - 1 - cta : cta); }
 
-// SPLIT (small batches; the rule is where the kernel is launched): an item is 128 query rows of ONE head, and tile t takes the key
-// tiles 2 i + t: half as long a chain for the few CTAs of a short batch.  The tiles exchange 64 columns of O each and
+// SPLIT (small batches; the rule is where the kernel is launched): an item is 128 query rows of ONE head, and tile t
+// takes the key tiles 2 i + t: half as long a chain for the few CTAs of a short batch.  The tiles exchange 64 columns of O each and
 // write the columns that they have merged.
 template <bool PAGED, bool PAIRS, bool SPLIT = false>
 __global__ void __launch_bounds__(pf_threads(SPLIT), 1) prefill_tc_kernel(const __grid_constant__ PrefillArgs a) {
@@ -399,8 +401,8 @@ __global__ void __launch_bounds__(pf_threads(SPLIT), 1) prefill_tc_kernel(const 
     // ------------------------------ loader ------------------------------
     // A tile is one TMA box per 64 columns where it may be fetched whole: inside its sequence, or (Q and K, whose
     // rows past the end change nothing that is stored) inside the tensor, or anywhere when the maps end with the tensor
-    // and fill up with zeros (V: only where the sequence ends with it, since another sequence's rows may hold anything).  The end of a sequence comes as boxes
-    // of 8 rows and, for what is left, as 16-byte pieces; V rows past it are zeros, since they meet
+    // and fill up with zeros (V: only where the sequence ends with it, since another sequence's rows may hold anything).
+    // The end of a sequence comes as boxes of 8 rows and, for what is left, as 16-byte pieces; V rows past it are zeros, since they meet
     // probabilities of zero.
     const int piece = lane & 15, row0 = lane >> 4;          // 16-byte piece of a row, even or odd rows
     uint64_t* pend[2] = {nullptr, nullptr};     // barriers of the pieces not yet announced, oldest first

@@ -4,7 +4,8 @@
 //   * wide_norm_kernel: QKV, gate / up and the LM head (K = 1024, residual add + RMSNorm in front), the layout of
 //     pair_gemv_kernel (16 weight rows on M, 8 batch rows on N, 8 warps splitting K): a weight fragment is read from shared
 //     memory once and multiplied with NG groups.  x stays in shared memory (8 NG rows), so that the kernel keeps
-//     within 128 registers and 170 KB and its CTAs start beside their predecessor's.  Clusters of four CTAs share the
+//     within 128 registers and, up to 24 rows, its CTAs start beside their predecessor's (gate / up of 32 rows
+//     takes 241 KB with o_proj and 257 with down_proj, of the SM's 228; the LM head takes an SM for itself).  Clusters of four CTAs share the
 //     norm: each normalises a quarter of the rows and writes them into all four shared memories (every CTA reading
 //     all rows of h and of the residual took 14 MB from L2 in a launch; gate / up, 20 rows: 7.3 -> 5.9 us).
 //   * wide_store_kernel: o_proj and down_proj.  A cluster of four CTAs shares 32 weight rows, each with a quarter of K: x is
