@@ -25,7 +25,7 @@
 // exactly 1, and the row sum adds the rounded values.  Both count: with O rescaled only when a maximum has grown by
 // more than 2^8 the error against 64 bits was 2-8 % larger, with a sum over the unrounded values as well 11-24 % (scores
 // of four times the usual spread; 1-5 % at the usual one), which was 8-12 % of the time (4 x 2,048 tokens 72.7 us
-// against 81.4, the thirteen prompts below 117 against 134, split form 512 tokens 10.5 against 11.0).
+// against 82.5, the thirteen prompts below 117 against 134, split form 512 tokens 10.5 against 11.0).
 //
 // What bounds it: per 64 keys the two tiles need 1,250 clocks of MMA (512 for P V, 800 for S, whose N = 64 reads Q
 // from shared memory twice as often as N = 128 would; measured with nothing else in the CTA) and 1,024
@@ -36,7 +36,7 @@
 // then follow one another), one issuing warp for both tiles (2,400), a quarter to a half of the exponentials as polynomials
 // on the FMA pipe (2-5 % slower), the next scores fetched during this tile's exponentials (2 % slower).
 // Short batches are bound by the chain of dependent tiles instead: 512 tokens 11.0 us, 1,024 tokens 17.2.
-// 4 x 2,048 tokens: 81 us = 845 TFLOP/s (mma.sync: 307 us); thirteen prompts of 1 to 2,048 tokens: 134 us (449).
+// 4 x 2,048 tokens: 82.5 us = 833 TFLOP/s (mma.sync: 307 us); thirteen prompts of 1 to 2,048 tokens: 134 us (449).
 // Every wait is bounded: on expiry the CTA's abort flag is raised, every role drains, status 3 is recorded and
 // the tensor memory released.
 #pragma once

@@ -428,8 +428,8 @@ int dfb_store_kvcache(const void* key, const void* value, int64_t key_stride, in
  *     are found through block_tables[b, position / block_size] (device int32 [batch, block_table_stride]), and
  *     query i attends to keys 0 .. i + (keys - queries) (the mask aligned to the last key, as FlashAttention).
  * All tensors bf16, row strides in elements; head_dim 128, grouped-query attention with q_heads a multiple of
- * kv_heads.  fp32 accumulation and softmax, probabilities rounded to bf16 before they multiply V (as
- * FlashAttention does).  A block id outside [0, num_blocks) is never followed: the key row is read as zeros and
+ * kv_heads; a scale of either sign.  fp32 accumulation and softmax, probabilities rounded to bf16 against the row's
+ * running maximum before they multiply V and before they are summed.  A block id outside [0, num_blocks) is never followed: the key row is read as zeros and
  * `status` (NULL, or a device int32[4]) receives {DFB_STATUS_BAD_BLOCK, kernel id, sequence, block id}.
  * Allocates nothing, synchronises nothing. */
 int dfb_prefill_attention(const void* q, const void* k, const void* v, void* out, const int32_t* cu_seqlens_q,
