@@ -413,7 +413,10 @@ __global__ void __launch_bounds__(256, 2) wide_store_kernel(const GemvArgs a) {
     const float v = (recv[tid] + recv[64 * NG + tid]) + (recv[2 * 64 * NG + tid] + recv[3 * 64 * NG + tid]);
     a.out[(size_t)(8 * n + (q & 7)) * a.out_stride + tile * 32 + 8 * rank + (q >> 3)] = __float2bfloat16_rn(v);
   }
-  if (!copy_ok) report_status(a.status, kStatusCopyTimeout, kKernelWide, blockIdx.x, kModeStore);
+  if (!copy_ok) {   // as above
+    report_status(a.status, kStatusCopyTimeout, kKernelWide, blockIdx.x, kModeStore);
+    mbar_wait_bounded(full, 0);
+  }
   if (tid == 0) trace_max(a.trace, 2);
 }
 
