@@ -275,7 +275,7 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
 #pragma unroll
     for (int s = 0; s < PSTAGES; ++s) {
       if ((int)blockIdx.x + s * stride >= a.n_tiles) break;
-      if (!mbar_wait_bounded(&full[s], 0)) copy_ok = false;
+      if (!mbar_wait_warp(&full[s], 0)) copy_ok = false;
       const unsigned char* w0p = stage_base + s * SM::kStageBytes + g * SM::kRowStride + 2 * kbase;
       const unsigned char* w1p = w0p + 8 * SM::kRowStride;
       float c[4][4];
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(256, 2) pair_gemv_kernel(const GemvArgs a) {
   } else
   for (int tile = blockIdx.x; tile < a.n_tiles; tile += stride, ++it) {
     const int s = it % kStagesOr1;
-    if (!kReg && !mbar_wait_bounded(&full[s], (it / kStagesOr1) & 1)) { copy_ok = false; break; }
+    if (!kReg && !mbar_wait_warp(&full[s], (it / kStagesOr1) & 1)) { copy_ok = false; break; }
     const unsigned char* w0p = stage_base + s * SM::kStageBytes + g * SM::kRowStride + 2 * kbase;
     const unsigned char* w1p = w0p + 8 * SM::kRowStride;
     float c[4][4];

@@ -102,7 +102,7 @@ row_gemv_kernel(const GemvArgs a) {
       if (b < a.rows) {
         uint2 hv, rv = make_uint2(0, 0);
         if (bulk_x) {
-          if (b == 0 && !mbar_wait_bounded(&xbar, 0))
+          if (b == 0 && !mbar_wait_warp(&xbar, 0))
             report_status(a.status, kStatusCopyTimeout, kKernelGemv, blockIdx.x, 0);
           hv = reinterpret_cast<const uint2*>(xs[b])[tid];
           rv = reinterpret_cast<const uint2*>(reinterpret_cast<const unsigned char*>(xs[b]) + 2 * K)[tid];

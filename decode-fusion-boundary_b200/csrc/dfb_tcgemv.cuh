@@ -155,6 +155,16 @@ __device__ __forceinline__ bool tc_wait(uint64_t* bar, uint32_t parity, volatile
   return false;
 }
 
+// The same by a whole warp, through its first lane (see mbar_wait_warp).
+__device__ __forceinline__ bool tc_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
+#pragma unroll 1
+  for (int i = 0; i < kMbarSpinLimit; ++i) {
+    if (mbar_try_wait_warp(bar, parity)) return true;
+    if ((i & 255) == 255 && __any_sync(0xffffffffu, *abort_flag)) return false;
+  }
+  return false;
+}
+
 // MT = 2 x (weight rows per tile): 64 for QKV (32 rows per tile), 128 for gate/up (32 gate + 32 up rows)
 // and for the LM head (64 rows per tile, persistent CTAs).
 //
@@ -370,7 +380,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) tc_gemv_kernel(const __grid_con
     bool ok = true;
     for (int tile = blockIdx.x; tile < n_tiles; tile += stride, ++it) {
       const int buf = it & 1;
-      if (!named_sync_and(2, 128, tc_wait(&acc_full[buf], (it >> 1) & 1, abort_flag))) { ok = false; break; }
+      if (!named_sync_and(2, 128, tc_wait_warp(&acc_full[buf], (it >> 1) & 1, abort_flag))) { ok = false; break; }
       tc_fence_after();
       // this lane's 8 useful columns (its half of K) of every issuer's accumulator
       float v[kTcIssuers][8];
