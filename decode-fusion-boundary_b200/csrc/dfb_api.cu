@@ -1193,10 +1193,14 @@ int run_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, 
 // ---- steps of 9 to 32 rows (dfb_wide.cuh) ------------------------------------------------------------------
 // (an option that takes other kernels speaks of those of 1 to 8 rows: such a decoder keeps to them)
 bool wide_usable(const DfbHandle* h) {
-  return h->full_geometry && !h->sharded() && h->step_mode == 0 && h->slots_wide && h->lmhead_ctas == 0 &&
+  return h->full_geometry && !h->sharded() && h->step_mode == 0 && h->slots_wide && h->lmhead_ctas == 0 && 2 * h->sm_count >= kWideRows &&
          same_chain(h->opt, ChainOptions()) && h->m.vocab % 16 == 0 &&
          h->m.max_model_len <= kMaxSplits * kAttnChunk;
 }
+
+// ids | positions | active | temperatures | block tables | attention kernel: chunk, 0, (row and chunk, position) of its CTAs
+size_t wide_stage_ints(const DfbHandle* h) { return (size_t)kWideRows * (4 + h->max_pages) + 2 + 4 * h->sm_count; }
+int* wide_chunk_word(const DfbHandle* h, int* stage) { return stage + kWideRows * (4 + h->max_pages); }
 
 int wide_prepare(DfbHandle* h) {
   DfbHandle::Wide& w = h->wide;
@@ -1204,7 +1208,7 @@ int wide_prepare(DfbHandle* h) {
   const DfbModelDesc& m = h->m;
   size_t off = 0;
   auto carve = [&](size_t bytes) { size_t o = off; off += (bytes + 255) & ~(size_t)255; return o; };
-  const size_t stage_ints = kWideRows * (4 + h->max_pages);
+  const size_t stage_ints = wide_stage_ints(h);
   const size_t o_stage = carve(sizeof(int) * stage_ints), o_h = carve(sizeof(bf16) * kWideRows * m.hidden);
   const size_t o_r0 = carve(sizeof(bf16) * kWideRows * m.hidden), o_r1 = carve(sizeof(bf16) * kWideRows * m.hidden);
   const size_t o_qkv = carve(sizeof(bf16) * kWideRows * h->qkv_rows()), o_attn = carve(sizeof(bf16) * kWideRows * h->q_size());
@@ -1248,12 +1252,12 @@ void launch_wide_store(Launcher& L, const GemvArgs& a, int n) {
   L.launch(kernel, dim3(n / 32 * kWideCluster), dim3(256), a, true, smem, kWideCluster);
 }
 
-// the step's kernels for NG groups of 8 rows; `chunks`: grid of the attention kernel, of 32 (half) or 64 positions each
+// the step's kernels for NG groups of 8 rows; `chunks`: grid of the attention kernel
 template <int NG>
-int enqueue_wide(DfbHandle* h, int chunks, bool half, bool sampling, cudaStream_t stream) {
+int enqueue_wide(DfbHandle* h, int chunks, bool sampling, cudaStream_t stream) {
   const DfbModelDesc& m = h->m;
   DfbHandle::Wide& w = h->wide;
-  DFB_CUDA(cudaMemcpyAsync(w.stage, w.host_stage, sizeof(int) * kWideRows * (4 + h->max_pages), cudaMemcpyHostToDevice, stream));
+  DFB_CUDA(cudaMemcpyAsync(w.stage, w.host_stage, sizeof(int) * wide_stage_ints(h), cudaMemcpyHostToDevice, stream));
   Launcher L{stream, h->use_pdl, h->trace_on ? h->trace : nullptr};
   L.opt = &h->opt;
   L.carve = 100;      // up to 24 rows every per-layer kernel fits beside its neighbour in all of the shared memory
@@ -1281,14 +1285,14 @@ int enqueue_wide(DfbHandle* h, int chunks, bool half, bool sampling, cudaStream_
     AttnArgs a = {};
     a.qkv = w.qkv; a.qkv_stride = h->qkv_rows(); a.q_size = h->q_size(); a.kv_size = h->kv_size();
     a.positions = w.stage + kWideRows; a.row_active = w.stage + 2 * kWideRows; a.block_tables = w.stage + 4 * kWideRows;
-    a.bt_stride = h->max_pages; a.packed_rows = kWideRows;
+    a.bt_stride = h->max_pages; a.chunk = wide_chunk_word(h, w.stage);
     a.q_norm = (const bf16*)lw.q_norm; a.k_norm = (const bf16*)lw.k_norm; a.cos_sin = m.rope_cos_sin; a.eps = m.eps;
     a.scale = 1.0f / sqrtf((float)m.head_dim);
     a.k_cache = (bf16*)m.k_cache + (size_t)l * h->kv_layer_elems; a.v_cache = (bf16*)m.v_cache + (size_t)l * h->kv_layer_elems;
     a.block_size = m.block_size; a.kv_heads = m.kv_heads; a.num_blocks = m.num_blocks; a.max_pos = m.max_model_len;
     a.out = w.attn; a.part_o = w.part_o; a.part_ml = w.part_ml; a.tickets = w.tickets; a.status = h->status;
     a.trace = L.next_trace();
-    auto attn = half ? paged_attention_ring_kernel<kAttnChunk / 2> : paged_attention_ring_kernel<kAttnChunk>;
+    auto attn = paged_attention_ring_kernel<0>;
     DFB_CUDA(ensure_dynamic_smem((const void*)attn, kRingSmemBytes));
     L.launch(attn, dim3(chunks), dim3(kRingThreads), a, true, kRingSmemBytes);
     launch_wide_store<2048, NG>(L, store(w.attn, lw.wo), m.hidden);
@@ -1311,28 +1315,39 @@ int enqueue_wide(DfbHandle* h, int chunks, bool half, bool sampling, cudaStream_
   return 0;
 }
 
-// Kernels and attention grid of a wide step of `rows` (9 to 32) rows whose contexts come to `halves` 32-position or
-// `wholes` 64-position chunks.  A chunk is a serial walk for its CTA (1.1 us per 8 positions), so the shorter ones are taken
-// while all of their CTAs are resident together, two per SM (10 rows x 512: 903 against 1,000 us per step; 20 rows with
-// 330 of them not).
-struct WideGeometry { int groups, chunks; bool half; };
-int wide_grid(int chunks) {      // few grids, so that few graphs: the attention CTAs without a chunk leave at once
+// Kernels and attention grid of a wide step of `rows` (9 to 32) rows.
+struct WideGeometry { int groups, chunks; };
+// Positions per CTA of the attention kernel.  A chunk is a serial walk for its CTA (1.1 us per 8 positions), so it is as short
+// as lets all CTAs be resident together, two per SM, and 32 positions at least (a row has 64 partial results).  A CTA more
+// than that waits for another to end, and every chunk costs its CTA the norm and rotation of eight heads and a merge.  us per
+// step, chunks of 32 positions where they fit and of 64 otherwise -> this rule: 20 rows, 5 - 1,500 tokens 1,058 -> 1,022; 20
+// rows of 200 - 2,030 1,429 -> 1,215; 32 of them 1,584 -> 1,482; 9 of them 1,065 -> 1,021; 24 x 512 1,075 -> 1,034; where the
+// rule takes the same chunk as before within 1 % (16 x 512 930 -> 924, 9 - 32 rows below 200 tokens).
+int wide_chunk(const DfbHandle* h, const int* positions, int rows) {
+  const int places = 2 * h->sm_count;
+  long total = 0;
+  for (int r = 0; r < rows; ++r) total += positions[r] + 1;
+  int chunk = (int)(total / places) & ~7;      // no shorter one can do
+  if (chunk < kAttnChunk / 2) chunk = kAttnChunk / 2;
+  for (;; chunk += 8) {
+    int ctas = 0;
+    for (int r = 0; r < rows; ++r) ctas += positions[r] / chunk + 1;
+    if (ctas <= places) return chunk;          // (at the longest context at the latest)
+  }
+}
+int wide_grid(const DfbHandle* h, int chunks) {      // few grids, so that few graphs: the attention CTAs without a chunk leave at once
   int grid = 64;
   while (grid < chunks) grid <<= 1;
-  return grid;
-}
-WideGeometry wide_geometry(const DfbHandle* h, int rows, int halves, int wholes) {
-  const bool half = halves <= 2 * h->sm_count;
-  return {(rows + 7) / 8, wide_grid(half ? halves : wholes), half};
+  return grid < 2 * h->sm_count ? grid : 2 * h->sm_count;
 }
 
 int enqueue_wide_step(DfbHandle* h, const WideGeometry& g, bool sampling, cudaStream_t s) {
-  return g.groups == 2 ? enqueue_wide<2>(h, g.chunks, g.half, sampling, s) : g.groups == 3 ? enqueue_wide<3>(h, g.chunks, g.half, sampling, s)
-                                                                               : enqueue_wide<4>(h, g.chunks, g.half, sampling, s);
+  return g.groups == 2 ? enqueue_wide<2>(h, g.chunks, sampling, s) : g.groups == 3 ? enqueue_wide<3>(h, g.chunks, sampling, s)
+                                                                       : enqueue_wide<4>(h, g.chunks, sampling, s);
 }
 
 int get_wide_graph(DfbHandle* h, const WideGeometry& g, bool sampling, cudaGraphExec_t* out) {
-  const int key = (((g.chunks * 8 + g.groups) * 2 + (g.half ? 1 : 0)) * 2 + (sampling ? 1 : 0)) * 2 + (h->use_pdl ? 1 : 0);
+  const int key = ((g.chunks * 8 + g.groups) * 2 + (sampling ? 1 : 0)) * 2 + (h->use_pdl ? 1 : 0);
   auto it = h->wide.graphs.find(key);
   if (it == h->wide.graphs.end()) {
     cudaGraph_t graph = nullptr;
@@ -1351,25 +1366,21 @@ int get_wide_graph(DfbHandle* h, const WideGeometry& g, bool sampling, cudaGraph
   return 0;
 }
 
-// Buffers, and the graphs of every wide step with contexts up to `max_context` (7 per group count at 2,048 tokens).
+// Buffers, and the graphs of every wide step with contexts up to `max_context` (four per group count at most).
 int warm_wide(DfbHandle* h, int max_context, bool sampling) {
   h->wide.no_room = false;
   int rc = wide_prepare(h);
   if (rc || !h->use_graph) return rc;
   constexpr int kHalf = kAttnChunk / 2;
   for (int groups = 2; groups <= kWideRows / 8; ++groups) {
-    const int halves = 8 * groups * ((max_context + kHalf - 1) / kHalf), wholes = 8 * groups * ((max_context + kAttnChunk - 1) / kAttnChunk);
-    const int resident = 2 * h->sm_count;
-    for (int half = 1; half >= 0; --half) {
-      if (!half && halves <= resident) break;
-      // whole chunks begin where the half ones no longer fit: at more than half as many
-      const int last = wide_grid(half ? (halves < resident ? halves : resident) : wholes);
-      for (int grid = wide_grid(half ? 1 : resident / 2 + 1); grid <= last; grid <<= 1)
-        for (int s = 0; s < (sampling ? 2 : 1); ++s) {
-          cudaGraphExec_t exec;
-          rc = get_wide_graph(h, WideGeometry{groups, grid, half != 0}, s != 0, &exec);
-          if (rc) return rc;
-        }
+    const int last = wide_grid(h, 8 * groups * ((max_context + kHalf - 1) / kHalf));
+    for (int chunks = 1, grid = 0; grid < last; chunks = grid + 1) {
+      grid = wide_grid(h, chunks);
+      for (int s = 0; s < (sampling ? 2 : 1); ++s) {
+        cudaGraphExec_t exec;
+        rc = get_wide_graph(h, WideGeometry{groups, grid}, s != 0, &exec);
+        if (rc) return rc;
+      }
     }
   }
   return 0;
@@ -2092,7 +2103,6 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
     // (a row without a number has no largest logit: its token is none)
     for (int r = 0; r < n_live; ++r)
       if (h->slots[live[r]].token < 0 || h->slots[live[r]].token >= h->embed_rows()) return DFB_E_BAD_ARG;
-    int halves = 0, wholes = 0;
     bool sampled = false;
     for (int r = 0; r < kWideRows; ++r) {
       const bool on = r < n_live;
@@ -2105,10 +2115,17 @@ int dfb_slots_step(DfbHandle* h, long long* sampled_tokens, int32_t* emitted, df
       int* bt = hs + 4 * kWideRows + r * h->max_pages;
       const int cols = on ? (int)s->table.size() : 0;
       for (int c = 0; c < h->max_pages; ++c) bt[c] = c < cols ? s->table[c] : 0;
-      if (on) { halves += (int)(s->position / (kAttnChunk / 2)) + 1; wholes += (int)(s->position / kAttnChunk) + 1; }
       sampled = sampled || t > 1e-10f;
     }
-    const int rc = wide_step(h, wide_geometry(h, n_live, halves, wholes), sampled, (cudaStream_t)stream);
+    const int chunk = wide_chunk(h, hs + kWideRows, n_live);
+    int* ctas = wide_chunk_word(h, hs);
+    ctas[0] = chunk; ctas[1] = 0;
+    ctas += 2;
+    int chunks = 0;
+    for (int r = 0; r < n_live; ++r)
+      for (int c = 0; c <= hs[kWideRows + r] / chunk; ++c, ++chunks) { ctas[2 * chunks] = r << 16 | c; ctas[2 * chunks + 1] = hs[kWideRows + r]; }
+    for (int c = chunks; c < 2 * h->sm_count; ++c) ctas[2 * c] = -1;
+    const int rc = wide_step(h, WideGeometry{(n_live + 7) / 8, wide_grid(h, chunks)}, sampled, (cudaStream_t)stream);
     if (rc == (int)cudaErrorMemoryAllocation && h->use_graph) {      // (of its graph: nothing has run)
       h->wide.no_room = true;
       (void)cudaGetLastError();

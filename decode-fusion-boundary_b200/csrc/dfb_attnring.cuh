@@ -95,31 +95,29 @@ __device__ __forceinline__ float warp_sum(float v) {
 }
 
 // CH: context positions per CTA, 64 or 32 (half as many stages per CTA and twice the CTAs: mid-size grids then
-// cover every SM, and three of a CTA's four stages are in flight before the dependency resolves).
+// cover every SM, and three of a CTA's four stages are in flight before the dependency resolves); 0: up to 32 rows of
+// uneven lengths, whose contexts are cut into chunks of a.chunk[0] positions (a multiple of 8) and dealt to a 1-D grid, so
+// that it is as large as the work; a.chunk[2 + 2 i] = row << 16 | chunk of CTA i (-1: none), then the row's position.  The
+// host takes the chunk that gives every CTA a place, two per SM, and no CTA a second turn (wide_chunk in dfb_api.cu).
+constexpr int kRingMaxSplits = 64;                   // chunks of a row with CH = 0: of 32 positions at least
+constexpr int kRingMaxBlocks = 33;                   // blocks that a chunk can touch: 2,048 positions in blocks of 64
 template <int CH>
 __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(const AttnArgs a) {
-  static_assert(CH == kAttnChunk || 2 * CH == kAttnChunk, "64 or 32 positions per CTA");
+  static_assert(CH == 0 || CH == kAttnChunk || 2 * CH == kAttnChunk, "64 or 32 positions per CTA, or what the step says");
+  constexpr bool kPacked = CH == 0;
+  const int chunk = kPacked ? *a.chunk : CH;
   if (!a.late_trigger) pdl_launch_dependents();
   int split = blockIdx.x, row = blockIdx.y;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (a.packed_rows) {
-    // up to 32 rows of uneven lengths: CTA i takes the i-th chunk of all rows' chunks one after the other, so that the
-    // grid is as large as the work (20 rows: 165 CTAs instead of 20 x 32); a negative position = no row
-    const int p = lane < a.packed_rows ? a.positions[lane] : -1;
-    const int n = p < 0 ? 0 : (min(p, a.max_pos - 1) + CH) / CH;
-    int end = n;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const int up = __shfl_up_sync(0xffffffffu, end, d);
-      if (lane >= d) end += up;
-    }
-    const unsigned before = __ballot_sync(0xffffffffu, end <= split);      // rows that end before this chunk
-    row = __popc(before);
-    if (row >= 32) return;
-    split -= __shfl_sync(0xffffffffu, end - n, row);
+  int2 mine = make_int2(0, 0);
+  if (kPacked) {      // the CTA's chunk (with its row's position: one trip to L2 less in front of the first copies)
+    mine = reinterpret_cast<const int2*>(a.chunk + 2)[blockIdx.x];
+    if (mine.x < 0) return;
+    row = mine.x >> 16;
+    split = mine.x & 0xffff;
   }
   if (tid == 0) { trace_min(a.trace, 0); trace_max(a.trace, 4); }
-  int pos = a.positions[row];
+  int pos = kPacked ? mine.y : a.positions[row];
   bool write_ok = true;
   if (pos < 0 || pos >= a.max_pos) {
     report_status(a.status, kStatusBadPosition, kKernelAttention, row, pos);
@@ -127,11 +125,11 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
     write_ok = false;
   }
   int ctx = pos + 1;
-  int nsplits = (ctx + CH - 1) / CH;
-  if (!a.packed_rows && nsplits > (int)gridDim.x) {   // the host's context bound was too small (see paged_attention_kernel)
+  int nsplits = (ctx + chunk - 1) / chunk;
+  if (!kPacked && nsplits > (int)gridDim.x) {   // the host's context bound was too small (see paged_attention_kernel)
     if (split == 0) report_status(a.status, kStatusBadGrid, kKernelAttention, row, pos);
     nsplits = (int)gridDim.x;
-    ctx = nsplits * CH;
+    ctx = nsplits * chunk;
     pos = ctx - 1;
     write_ok = false;
   }
@@ -144,37 +142,50 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
   __shared__ __align__(16) __nv_bfloat16 knew[kRingHeads][kHeadDim];
   __shared__ __align__(16) __nv_bfloat16 vnew[kRingHeads][kHeadDim];
 
-  const int start = split * CH;
-  const int end = min(ctx, start + CH);
+  const int start = split * chunk;
+  const int end = min(ctx, start + chunk);
   const bool owner = split == nsplits - 1;
   const int nsub = (end - start + kRingPos - 1) / kRingPos;
-  int bt_col = start / a.block_size;
-  if (a.bt_cols > 0 && bt_col >= a.bt_cols) {
-    report_status(a.status, kStatusBadBlock, kKernelAttention, row, -1 - bt_col);
-    bt_col = a.bt_cols - 1;
-    write_ok = false;
-  }
-  int block = a.block_tables[row * a.bt_stride + bt_col];
-  if (block < 0 || block >= a.num_blocks) {
-    report_status(a.status, kStatusBadBlock, kKernelAttention, row, block);
-    block = 0;
-    write_ok = false;
+  // the blocks that the chunk touches (one, but for the step's own chunk lengths)
+  __shared__ int blocks[kPacked ? kRingMaxBlocks : 1];
+  const int col0 = start / a.block_size, cols = kPacked ? (end - 1) / a.block_size - col0 + 1 : 1;
+  if (tid < cols) {
+    int bt_col = col0 + tid;
+    if (a.bt_cols > 0 && bt_col >= a.bt_cols) {
+      report_status(a.status, kStatusBadBlock, kKernelAttention, row, -1 - bt_col);
+      bt_col = a.bt_cols - 1;
+      write_ok = false;
+    }
+    int block = a.block_tables[row * a.bt_stride + bt_col];
+    if (block < 0 || block >= a.num_blocks) {
+      report_status(a.status, kStatusBadBlock, kKernelAttention, row, block);
+      block = 0;
+      write_ok = false;
+    }
+    blocks[tid] = block;
   }
   const size_t tok_stride = (size_t)kRingHeads * kHeadDim;
-  const size_t chunk_base = ((size_t)block * a.block_size + (start % a.block_size)) * tok_stride;
+  // element of position p of the chunk (a stage of 8 positions lies in one block; a division would stand in the way of a refill)
+  const int in_block0 = start - col0 * a.block_size;
+  auto element = [&](int p) -> size_t {
+    int off = in_block0 + p - start, i = 0;
+    if (kPacked)
+      for (; off >= a.block_size; off -= a.block_size) ++i;
+    return ((size_t)blocks[i] * a.block_size + off) * tok_stride;
+  };
 
   if (tid == 0) {
 #pragma unroll
     for (int s = 0; s < kRingStages; ++s) { mbar_init(&full[s], 1); done[s] = 0u; }
     fence_mbar_init();
   }
-  __syncthreads();
+  write_ok = !__syncthreads_or(!write_ok);
 
   // one elected lane requests stage j: the 8 positions' K rows as one copy, their V rows as another
   auto issue_stage = [&](int j) {
     const int s = j % kRingStages;
     mbar_expect_tx(&full[s], (uint32_t)kRingStageBytes);
-    const size_t off = chunk_base + (size_t)(j * kRingPos) * tok_stride;
+    const size_t off = element(start + j * kRingPos);
     bulk_g2s(ring_smem + s * kRingStageBytes, a.k_cache + off, kRingPos * kRingRowBytes, &full[s]);
     bulk_g2s(ring_smem + s * kRingStageBytes + kRingPos * kRingRowBytes, a.v_cache + off, kRingPos * kRingRowBytes, &full[s]);
   };
@@ -241,7 +252,7 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
 
   if (owner && write_ok && (a.row_active == nullptr || a.row_active[row] != 0)) {
     // the new token's K / V of this head into the cache: lanes 0-15 the 16-byte pieces of K, lanes 16-31 of V
-    const size_t off = chunk_base + (size_t)(pos - start) * tok_stride + (size_t)warp * kHeadDim + 8 * (lane & 15);
+    const size_t off = element(pos) + (size_t)warp * kHeadDim + 8 * (lane & 15);
     const uint4 piece = reinterpret_cast<const uint4*>(lane < 16 ? knew[warp] : vnew[warp])[lane & 15];
     *reinterpret_cast<uint4*>((lane < 16 ? a.k_cache : a.v_cache) + off) = piece;
   }
@@ -352,7 +363,7 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
     *reinterpret_cast<uint2*>(out) = make_uint2(pack_bf16(o0[0] / l0, o0[1] / l0), pack_bf16(o0[2] / l0, o0[3] / l0));
     *reinterpret_cast<uint2*>(out + kHeadDim) = make_uint2(pack_bf16(o1[0] / l1, o1[1] / l1), pack_bf16(o1[2] / l1, o1[3] / l1));
   } else {
-    const size_t pidx = ((size_t)row * a.kv_heads + warp) * (a.packed_rows ? kMaxSplits * kAttnChunk / CH : kMaxSplits);
+    const size_t pidx = ((size_t)row * a.kv_heads + warp) * (kPacked ? kRingMaxSplits : kMaxSplits);
     float* po = a.part_o + (pidx + split) * 2 * kHeadDim + 4 * lane;
     *reinterpret_cast<float4*>(po) = make_float4(o0[0], o0[1], o0[2], o0[3]);
     *reinterpret_cast<float4*>(po + kHeadDim) = make_float4(o1[0], o1[1], o1[2], o1[3]);
@@ -369,9 +380,9 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
     }
     last = __shfl_sync(0xffffffffu, last, 0);
     if (last) {
-      // lane s holds (max, sum) of chunks s and (CH = 32, packed) s + 32 for both heads; weights by shuffle, partial
+      // lane s holds (max, sum) of chunks s and (CH = 0) s + 32 for both heads; weights by shuffle, partial
       // outputs 8 chunks at a time
-      constexpr int W = CH < kAttnChunk ? 2 : 1;
+      constexpr int W = kPacked ? 2 : 1;
       float2 ml0[W], ml1[W];
       float M0 = -INFINITY, M1 = -INFINITY, S0 = 0.f, S1 = 0.f, w0[W], w1[W];
 #pragma unroll

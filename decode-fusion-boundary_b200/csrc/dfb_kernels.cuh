@@ -582,7 +582,7 @@ struct AttnArgs {
   int kv_heads;
   int num_blocks;
   int max_pos;
-  int packed_rows;              // streaming kernel: 0 = grid (chunk, row); else the 1-D grid walks the chunks of so many rows
+  const int* chunk;             // streaming kernel with a 1-D grid: positions of a chunk, 0, (row << 16 | chunk, position) of every CTA
   int ctx_limit;                // cluster kernel: contexts beyond this are an error (the caller's bound)
   int* status;                  // [4]: code, kernel id, index, observed value
   __nv_bfloat16* out;           // [rows, q_size]

@@ -13,7 +13,7 @@
 //     dependency; all of it is in flight at once, in registers.  The parts meet in the shared memory of the CTA that
 //     finishes the row (down_proj, 20 rows, two CTAs: 5.1 us, four: 4.2 us).
 //
-// 20 rows, 5 - 1,500 tokens: 1,066 us per step, of which attention 15 us per layer (paged_attention_ring_kernel on a packed
+// 20 rows, 5 - 1,500 tokens: 1,022 us per step, of which attention 13.5 us per layer (paged_attention_ring_kernel on a packed
 // list of chunks), LM head 80 us.
 // Bound by mma.sync's issue rate (one per 38 clocks and sub-partition: 0.3 us per group and gate / up tile of 16 rows) and
 // by the latency of the dependent launches.  Rows beyond the live ones are computed and ignored.

@@ -325,3 +325,36 @@ def test_wide_step_against_the_oracle(model, cuda_device, n):
     assert float((kv_got.cpu().float() - kv.float()).abs().max()) <= 2.0 ** -5
     for i in range(n):
         assert H.token_gap_ok(logits[i].float(), got[0][i], int(tokens[i])), i
+
+
+@pytest.mark.parametrize("block_size,lengths", [
+    (256, [2030 - 11 * i for i in range(9)]),                     # chunks of 64 positions and more, four blocks and a rest
+    (256, [1200 + 37 * i for i in range(20)]),                    # of about 110: across the ends of blocks
+    (64, [1990 - 9 * i for i in range(32)]),                      # of about 220 in blocks of 64: four or five blocks each
+    (192, [511, 0, 1, 63, 64, 191, 192, 193, 2047, 1535, 1536, 1537, 1000, 999, 40, 39, 41]),
+    (64, [31, 32, 33, 7, 8, 0, 63, 64, 65])])                     # of 32, the shortest
+def test_chunks_of_every_length(cuda_device, block_size, lengths):
+    """The attention of a wide step cuts the contexts into chunks that follow their sum: from 32 positions on, across block
+    boundaries, several blocks long.  One step against launches of 8 rows; the blocks of a row lie scattered."""
+    from dfb_b200 import native
+    from dfb_b200.slots import SlotRuntime
+    g = H.oracle_geometry(layers=2, vocab=2048, block_size=block_size)
+    w = O.make_weights(g, seed=17, norm="random").to(BF)
+    need = [n // block_size + 1 for n in lengths]
+    order = np.random.Generator(np.random.Philox(key=8)).permutation(sum(need)).tolist()
+    tables = [[order.pop() for _ in range(k)] for k in need]
+    history = (torch.randn(tuple(O.new_kv_cache(g, sum(need), BF).shape), generator=torch.Generator().manual_seed(3)) * 0.5).to(BF).cuda()
+    sides = []
+    for wide in (1, 0):
+        kv = history.clone()
+        dec = H.make_decoder(w, kv)
+        dec.set_option(native.DFB_OPT_SLOTS_WIDE, wide)
+        rt = SlotRuntime(dec)
+        for i, (n, table) in enumerate(zip(lengths, tables)):
+            rt.admit(i, 100 + 7 * i, n, table)
+        rt.step()
+        assert dec.status()[0] == 0
+        dec.close()
+        sides.append(kv)
+    assert torch.equal((sides[0] != history).any(dim=-1), (sides[1] != history).any(dim=-1))
+    assert float((sides[0].float() - sides[1].float()).abs().max()) <= 2.0 ** -5       # (as above: layer 2's new rows)
