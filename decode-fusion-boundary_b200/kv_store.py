@@ -5,9 +5,14 @@ by ``dfb_store_kvcache`` (no Triton, no CPU fallback)."""
 
 from __future__ import annotations
 
+import struct
+
 # Looked up at the first call (the package imports without torch and without the built library) and kept: one call of
 # store_kvcache on a short prompt takes a few microseconds, of which the imports and attribute chains of a call were two.
 _torch = _store = _prefill = _check = _stream = _bf16 = _i32 = _device = _empty = None
+# the arguments of the two native calls as one block of 64-bit words (a bytes object of its own per call): ctypes takes
+# 1.5 us to convert twelve arguments one by one, 0.5 for the block
+_store_words, _prefill_words = struct.Struct("12q").pack, struct.Struct("15qd8q").pack
 
 
 def _load():
@@ -17,7 +22,7 @@ def _load():
     from . import native
 
     lib = native.lib()
-    _store, _prefill, _check = lib.dfb_store_kvcache, lib.dfb_prefill_attention_rows, native.check
+    _store, _prefill, _check = lib.dfb_store_kvcache_words, lib.dfb_prefill_attention_words, native.check
     _bf16, _i32, _device, _empty = torch.bfloat16, torch.int32, torch.cuda.current_device, torch.empty
     # the raw handle of the current stream; the public call builds a Stream object (1 us) around it
     raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
@@ -38,7 +43,7 @@ def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> No
     v_stride, v_head, v_one = value.stride()
     assert k_one == 1 and v_one == 1
     assert k_head == head_dim and v_head == head_dim
-    assert k_cache.stride(1) == d and v_cache.stride(1) == d
+    assert k_cache.stride()[1] == d and v_cache.stride()[1] == d
     assert slot_mapping.numel() == n
     if key.dtype != _bf16 or k_cache.dtype != _bf16:
         raise TypeError("store_kvcache moves bf16 rows")
@@ -46,10 +51,10 @@ def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> No
         raise TypeError("slot_mapping must be an int32 CUDA tensor")
     if n == 0:
         return
-    blocks, block_size = k_cache.shape[:2]
-    code = _store(key.data_ptr(), value.data_ptr(), k_stride, v_stride, k_cache.data_ptr(), v_cache.data_ptr(),
-                  slot_mapping.data_ptr(), n, d, blocks * block_size, status.data_ptr() if status is not None else None,
-                  _stream())
+    shape = k_cache.shape
+    code = _store(_store_words(key.data_ptr(), value.data_ptr(), k_stride, v_stride, k_cache.data_ptr(), v_cache.data_ptr(),
+                               slot_mapping.data_ptr(), n, d, shape[0] * shape[1],
+                               status.data_ptr() if status is not None else 0, _stream()))
     if code:
         _check(code, "dfb_store_kvcache")
 
@@ -85,15 +90,15 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
         assert k_strides[1] == head_dim and v_strides[1] == head_dim
         num_blocks = block_size = 0
         k_stride, v_stride = k_strides[0], v_strides[0]
-        bt_ptr, bt_stride = None, 0
+        bt_ptr, bt_stride = 0, 0
     out = _empty((n, q_heads, head_dim), dtype=_bf16, device=q.device)
     if n == 0:
         return out
-    code = _prefill(
+    code = _prefill(_prefill_words(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_seqlens_q.data_ptr(),
-        cu_seqlens_k.data_ptr() if cu_seqlens_k is not None else None, cu_seqlens_q.numel() - 1, int(max_seqlen_q),
+        cu_seqlens_k.data_ptr() if cu_seqlens_k is not None else 0, cu_seqlens_q.numel() - 1, int(max_seqlen_q),
         q_stride, k_stride, v_stride, q_heads * head_dim, q_heads, kv_heads, head_dim, float(softmax_scale), bt_ptr,
-        bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else None, n, kv_rows, _stream())
+        bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else 0, n, kv_rows, _stream()))
     if code:
         _check(code, "dfb_prefill_attention")
     return out

@@ -53,7 +53,8 @@ EXPORTS = (
     "dfb_tp_open_loopback", "dfb_decode_step_host_sampled", "dfb_set_seed", "dfb_launch_lmhead_sample",
     "dfb_decode_burst_enqueue", "dfb_decode_burst_collect", "dfb_decode_burst_host", "dfb_warm", "dfb_warm_slots",
     "dfb_store_kvcache", "dfb_slot_set", "dfb_slot_get", "dfb_slots_step", "dfb_slots_run",
-    "dfb_prefill_attention", "dfb_wait_tokens", "dfb_prefill_attention_rows",
+    "dfb_prefill_attention", "dfb_wait_tokens", "dfb_prefill_attention_rows", "dfb_store_kvcache_words",
+    "dfb_prefill_attention_words",
 )
 
 
@@ -150,6 +151,7 @@ def lib() -> C.CDLL:
     L.dfb_prefill_attention.argtypes = [vp, vp, vp, vp, vp, vp, i32, i32, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                                         i32, i32, i32, f32, vp, i32, i32, i32, vp, vp]
     L.dfb_prefill_attention_rows.argtypes = L.dfb_prefill_attention.argtypes[:-1] + [C.c_int64, C.c_int64, vp]
+    L.dfb_store_kvcache_words.argtypes = L.dfb_prefill_attention_words.argtypes = [C.c_char_p]
     L.dfb_slot_set.argtypes = [vp, i32, i32, C.c_int64, C.c_int64, vp, i32, f32]
     L.dfb_slot_get.argtypes = [vp, i32, vp, vp, vp]
     L.dfb_slots_step.argtypes = [vp, vp, vp, vp]

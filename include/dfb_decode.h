@@ -415,6 +415,9 @@ int dfb_launch_lmhead_sample(DfbHandle* h, const void* hidden_in, const void* re
 int dfb_store_kvcache(const void* key, const void* value, int64_t key_stride, int64_t value_stride, void* k_cache,
                       void* v_cache, const int32_t* slot_mapping, int32_t n_tokens, int32_t row_elems,
                       int64_t num_slots, int32_t* status, dfb_stream_t stream);
+/* The same with its arguments, in their order, as 64-bit words (integers and pointers as they are): for bindings that
+ * convert arguments one by one. */
+int dfb_store_kvcache_words(const int64_t* words);
 
 /* Causal prefill attention over the prompt tokens of `batch` sequences laid back to back: the reference's
  * flash_attn_varlen_func(..., causal=True[, block_table=...]) call of layers/attention.py:64-70, both cases.
@@ -444,6 +447,8 @@ int dfb_prefill_attention_rows(const void* q, const void* k, const void* v, void
                           int64_t k_stride, int64_t v_stride, int64_t out_stride, int32_t q_heads, int32_t kv_heads,
                           int32_t head_dim, float scale, const int32_t* block_tables, int32_t block_table_stride,
                           int32_t block_size, int32_t num_blocks, int32_t* status, int64_t q_rows, int64_t kv_rows, dfb_stream_t stream);
+/* The same with its arguments, in their order, as 64-bit words; the scale as a double. */
+int dfb_prefill_attention_words(const int64_t* words);
 
 /* Final add+RMSNorm, tied LM head and greedy argmax WITHOUT any allocation.
  * (No counterpart in the reference: its LM head always runs inside a decoder

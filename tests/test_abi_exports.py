@@ -82,3 +82,23 @@ def test_prefill_attention_argument_checks_need_no_device():
     assert lib.dfb_prefill_attention(*bad) == -1
     bad = list(ok); bad[16] = one                # a block table without its geometry
     assert lib.dfb_prefill_attention(*bad) == -1
+
+
+def test_calls_by_words_check_as_the_others_do():
+    """The two prefill calls that take their arguments as a block of 64-bit words hand every word to its place."""
+    import struct
+    lib = native.lib()
+    one = 16
+    store = (one, one, 1024, 1024, one, one, one, 1, 1024, 10, 0, 0)
+    for i, value, want in ((0, 0, -1), (1, one + 2, -1), (2, 512, -1), (3, 512, -1), (4, 0, -1), (5, 0, -1), (6, 0, -1), (7, -1, -1),
+                           (7, 0, 0), (8, 1020, -1), (9, 0, -1)):
+        words = list(store)
+        words[i] = value
+        assert lib.dfb_store_kvcache_words(struct.pack("12q", *words)) == want, (i, value)
+        words[10:] = [None, None]
+        assert lib.dfb_store_kvcache(*words) == want
+    prefill = (one, one, one, one, one, 0, 1, 8, 4096, 4096, 4096, 2048, 16, 8, 128, 0.088, 0, 0, 0, 0, 0, 0, 0, 0)
+    for i, value, want in ((0, 0, -1), (4, 0, -1), (8, 1000, -1), (9, 4100, -1), (11, 8, -1), (13, 5, -2), (14, 64, -2), (16, one, -1)):
+        words = list(prefill)
+        words[i] = value
+        assert lib.dfb_prefill_attention_words(struct.pack("15qd8q", *words)) == want, (i, value)
