@@ -844,8 +844,12 @@ int launch_attention(Launcher& L, DfbHandle* h, int layer, const bf16* qkv, cons
   const int ctas = nsplit * m.kv_heads * rows;
   if (nsplit_arg >= kClusterFlag) {
     a.ctx_limit = nsplit * kAttnChunk;
-    a.late_trigger = L.opt->late_trigger;
     const int cs = 2 << (nsplit_arg / kClusterFlag - 1);
+    // o_proj is let in behind this kernel's own dependency: CTAs of o_proj that come while QKV still runs take the places of
+    // this kernel's clusters (us per step, early / late: 3 x 300 tokens 564 / 550, 4 x 300 575 / 562, 5 x 1,000 695 / 690, 8 x
+    // 520 652.6 / 650.0, 8 x 1,000 720.8 / 717.7, 8 x 2,000 883.9 / 882.3).  Not the small grids with two CTAs (8 x 150 567.6 /
+    // 570.4) nor the chunked kernels (3 x 520 606 / 600, but 3 x 150 539 / 564, 5 x 520 626 / 633, 418 + 97 + 650 sampled slower).
+    a.late_trigger = L.opt->late_trigger || cs >= 4;
     auto kernel = cs == 8 ? cluster_attention_kernel<8> : cs == 4 ? cluster_attention_kernel<4> : cluster_attention_kernel<2>;
     L.launch(kernel, dim3(cs, m.kv_heads, rows), dim3(kCaThreads), a, true, 0, cs);
     return L.err;
