@@ -15,6 +15,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <new>
@@ -1802,15 +1803,22 @@ int dfb_store_kvcache(const void* key, const void* value, int64_t key_stride, in
 
 // Both prefill entry points once more, with their arguments in one block of 64-bit words: a ctypes call converts its
 // arguments one by one (0.1 us each), which is as much as the launch (us per call: KV write of 37 tokens 6.4 -> 5.3,
-// prefill attention of a prompt of up to 160 tokens 10.7 -> 8.6).
+// prefill attention of a prompt of up to 160 tokens 10.7 -> 8.6).  A word that does not fit its 32-bit argument is refused:
+// cut to 32 bits, 2^32 tokens would be none, and the call a success.
+static bool words_fit(const int64_t* w, std::initializer_list<int> narrow) {
+  for (int i : narrow)
+    if (w[i] != (int32_t)w[i]) return false;
+  return true;
+}
+
 int dfb_store_kvcache_words(const int64_t* w) {
-  if (!w) return DFB_E_BAD_ARG;
+  if (!w || !words_fit(w, {7, 8})) return DFB_E_BAD_ARG;
   return dfb_store_kvcache((const void*)w[0], (const void*)w[1], w[2], w[3], (void*)w[4], (void*)w[5], (const int32_t*)w[6],
                            (int32_t)w[7], (int32_t)w[8], w[9], (int32_t*)w[10], (dfb_stream_t)w[11]);
 }
 
 int dfb_prefill_attention_words(const int64_t* w) {
-  if (!w) return DFB_E_BAD_ARG;
+  if (!w || !words_fit(w, {6, 7, 12, 13, 14, 17, 18, 19})) return DFB_E_BAD_ARG;
   double scale;
   memcpy(&scale, &w[15], sizeof(scale));
   return dfb_prefill_attention_rows((const void*)w[0], (const void*)w[1], (const void*)w[2], (void*)w[3], (const int32_t*)w[4],

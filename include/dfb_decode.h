@@ -416,7 +416,7 @@ int dfb_store_kvcache(const void* key, const void* value, int64_t key_stride, in
                       void* v_cache, const int32_t* slot_mapping, int32_t n_tokens, int32_t row_elems,
                       int64_t num_slots, int32_t* status, dfb_stream_t stream);
 /* The same with its arguments, in their order, as 64-bit words (integers and pointers as they are): for bindings that
- * convert arguments one by one. */
+ * convert arguments one by one.  A 32-bit argument whose word is larger is a bad argument. */
 int dfb_store_kvcache_words(const int64_t* words);
 
 /* Causal prefill attention over the prompt tokens of `batch` sequences laid back to back: the reference's

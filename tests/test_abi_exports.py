@@ -102,3 +102,23 @@ def test_calls_by_words_check_as_the_others_do():
         words = list(prefill)
         words[i] = value
         assert lib.dfb_prefill_attention_words(struct.pack("15qd8q", *words)) == want, (i, value)
+
+
+def test_words_beyond_32_bits_are_refused():
+    """A count that does not fit its argument is not cut to one that does: 2^32 tokens are not none, 2^32 + 1 sequences
+    not one."""
+    import struct
+    lib = native.lib()
+    one = 16
+    store = (one, one, 1024, 1024, one, one, one, 0, 1024, 10, 0, 0)
+    for i in (7, 8):
+        for off in (1 << 32, -(1 << 32), 1 << 31, 1 << 62):
+            words = list(store)
+            words[i] += off
+            assert lib.dfb_store_kvcache_words(struct.pack("12q", *words)) == -1, (i, off)
+    prefill = (one, one, one, one, one, one, 1, 8, 4096, 4096, 4096, 2048, 16, 8, 128, 0.088, one, 4, 256, 8, 0, 0, 0, 0)
+    for i in (6, 7, 12, 13, 14, 17, 18, 19):
+        for off in (1 << 32, -(1 << 32)):
+            words = list(prefill)
+            words[i] += off
+            assert lib.dfb_prefill_attention_words(struct.pack("15qd8q", *words)) == -1, (i, off)
