@@ -33,7 +33,7 @@ def _load():
 def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> None:
     """``key`` / ``value``: ``[N, kv_heads, head_dim]`` bf16 CUDA tensors (any row
     stride); ``k_cache`` / ``v_cache``: one layer's ``[num_blocks, block_size,
-    kv_heads, head_dim]`` views; ``slot_mapping``: int32 ``[N]``, -1 = skip.
+    kv_heads, head_dim]`` views, bf16 and dense; ``slot_mapping``: int32 ``[N]``, -1 = skip.
     ``status``: optional int32 CUDA tensor ``[4]`` that receives a bad slot."""
     if _torch is None:
         _load()
@@ -43,17 +43,23 @@ def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> No
     v_stride, v_head, v_one = value.stride()
     assert k_one == 1 and v_one == 1
     assert k_head == head_dim and v_head == head_dim
-    assert k_cache.stride()[1] == d and v_cache.stride()[1] == d
+    v_rows, v_heads, v_dim = value.shape
+    assert v_rows >= n and v_heads * v_dim >= d
+    # slot s is row s of both caches: their blocks lie one behind the other, and V has as many as K
+    k_shape, v_shape, k_strides, v_strides = k_cache.shape, v_cache.shape, k_cache.stride(), v_cache.stride()
+    slots = k_shape[0] * k_shape[1]
+    assert k_strides[1] == d and v_strides[1] == d and v_shape[0] * v_shape[1] >= slots
+    assert k_strides[0] == k_shape[1] * d or k_shape[0] == 1
+    assert v_strides[0] == v_shape[1] * d or v_shape[0] == 1
     assert slot_mapping.numel() == n
-    if key.dtype != _bf16 or k_cache.dtype != _bf16:
+    if key.dtype != _bf16 or value.dtype != _bf16 or k_cache.dtype != _bf16 or v_cache.dtype != _bf16:
         raise TypeError("store_kvcache moves bf16 rows")
     if slot_mapping.dtype != _i32 or not slot_mapping.is_cuda:
         raise TypeError("slot_mapping must be an int32 CUDA tensor")
     if n == 0:
         return
-    shape = k_cache.shape
     code = _store(_store_words(key.data_ptr(), value.data_ptr(), k_stride, v_stride, k_cache.data_ptr(), v_cache.data_ptr(),
-                               slot_mapping.data_ptr(), n, d, shape[0] * shape[1],
+                               slot_mapping.data_ptr(), n, d, slots,
                                status.data_ptr() if status is not None else 0, _stream()))
     if code:
         _check(code, "dfb_store_kvcache")
