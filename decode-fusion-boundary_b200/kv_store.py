@@ -83,26 +83,37 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
         raise TypeError("prefill_attention takes bf16 tensors")
     if cu_seqlens_q.dtype != _i32 or not cu_seqlens_q.is_cuda:
         raise TypeError("cu_seqlens_q must be an int32 CUDA tensor")
+    batch = cu_seqlens_q.numel() - 1
+    if cu_seqlens_k is not None:
+        if cu_seqlens_k.dtype != _i32 or not cu_seqlens_k.is_cuda:
+            raise TypeError("cu_seqlens_k must be an int32 CUDA tensor")
+        assert cu_seqlens_k.numel() > batch
+    # K and V are read at the same places: V has what K has
     if block_table is not None:
-        num_blocks, block_size, kv_heads = k.shape[:3]
+        num_blocks, block_size, kv_heads, k_dim = k.shape
+        v_blocks, v_block_size, v_heads, v_dim = v.shape
         k_stride, v_stride, kv_rows = k_strides[1], v_strides[1], 0
         assert k_strides[2] == head_dim and v_strides[2] == head_dim and k_strides[0] == block_size * k_stride
-        if block_table.dtype != _i32 or block_table.stride(-1) != 1 or cu_seqlens_k is None:
-            raise TypeError("the prefix-cache case needs an int32 block table and cu_seqlens_k")
+        assert v_blocks >= num_blocks and v_block_size == block_size and (v_strides[0] == block_size * v_stride or v_blocks == 1)
+        if block_table.dtype != _i32 or not block_table.is_cuda or block_table.stride(-1) != 1 or cu_seqlens_k is None:
+            raise TypeError("the prefix-cache case needs an int32 CUDA block table and cu_seqlens_k")
+        assert block_table.shape[0] >= batch
         bt_ptr, bt_stride = block_table.data_ptr(), block_table.stride(0)
     else:
-        kv_rows, kv_heads = k.shape[:2]
-        kv_rows = min(kv_rows, v.shape[0])
+        k_rows, kv_heads, k_dim = k.shape
+        v_rows, v_heads, v_dim = v.shape
+        kv_rows = min(k_rows, v_rows)
         assert k_strides[1] == head_dim and v_strides[1] == head_dim
         num_blocks = block_size = 0
         k_stride, v_stride = k_strides[0], v_strides[0]
         bt_ptr, bt_stride = 0, 0
+    assert v_heads >= kv_heads and k_dim == head_dim and v_dim == head_dim
     out = _empty((n, q_heads, head_dim), dtype=_bf16, device=q.device)
     if n == 0:
         return out
     code = _prefill(_prefill_words(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_seqlens_q.data_ptr(),
-        cu_seqlens_k.data_ptr() if cu_seqlens_k is not None else 0, cu_seqlens_q.numel() - 1, int(max_seqlen_q),
+        cu_seqlens_k.data_ptr() if cu_seqlens_k is not None else 0, batch, int(max_seqlen_q),
         q_stride, k_stride, v_stride, q_heads * head_dim, q_heads, kv_heads, head_dim, float(softmax_scale), bt_ptr,
         bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else 0, n, kv_rows, _stream()))
     if code:

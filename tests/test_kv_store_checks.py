@@ -68,3 +68,44 @@ def test_store_refuses(calls, changed):
     with pytest.raises((AssertionError, TypeError)):
         kv_store.store_kvcache(**store_args(**changed))
     assert not calls
+
+
+def prefill_args(cached=False, **changed):
+    q = torch.zeros(6, 16, 128, dtype=BF)
+    kv = (cache(), cache()) if cached else (rows(6), rows(6))
+    args = dict(q=q, k=kv[0], v=kv[1], cu_seqlens_q=ints(3), max_seqlen_q=4, softmax_scale=0.125)
+    if cached:
+        args.update(cu_seqlens_k=ints(3), block_table=ints(2, 5))
+    args.update(changed)
+    return args
+
+
+@pytest.mark.parametrize("cached,changed", [
+    (False, dict()), (False, dict(cu_seqlens_k=ints(3))), (False, dict(v=torch.zeros(6, 4096, dtype=BF)[:, 3072:].view(6, 8, 128))),
+    (False, dict(k=rows(9))), (False, dict(v=rows(9))), (False, dict(cu_seqlens_k=ints(7))), (True, dict()), (True, dict(v=cache(6))),
+    (True, dict(k=torch.zeros(2, 4, 64, 8, 128, dtype=BF)[0], block_table=ints(3, 8)[:, :2])),
+    (True, dict(k=cache(1), v=torch.zeros(1, 2, 64, 8, 128, dtype=BF)[:, 0]))])
+def test_prefill_takes(calls, cached, changed):
+    a = prefill_args(cached, **changed)
+    out = kv_store.prefill_attention(**a)
+    k, v, cu_k, table = a["k"], a["v"], a.get("cu_seqlens_k"), a.get("block_table")
+    assert tuple(out.shape) == (6, 16, 128) and out.dtype == BF
+    assert calls == [("_prefill", (
+        a["q"].data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), a["cu_seqlens_q"].data_ptr(),
+        0 if cu_k is None else cu_k.data_ptr(), 2, 4, 2048, k.stride(int(cached)), v.stride(int(cached)), 2048, 16, 8, 128, 0.125,
+        table.data_ptr() if cached else 0, table.stride(0) if cached else 0, 64 if cached else 0, len(k) if cached else 0, 0, 6,
+        0 if cached else min(len(k), len(v)), 0))]
+
+
+@pytest.mark.parametrize("cached,changed", [
+    (False, dict(v=rows(6, 4))), (False, dict(cu_seqlens_k=ints(3, dtype=torch.int64))), (False, dict(cu_seqlens_k=ints(2))),
+    (False, dict(cu_seqlens_k=torch.zeros(3, dtype=torch.int32))), (False, dict(v=torch.zeros(6, 8, 256, dtype=BF)[:, :, :128])),
+    (False, dict(k=rows(6)[:, :, :64])), (False, dict(v=rows(6, dtype=torch.float16))), (False, dict(cu_seqlens_q=ints(3, dtype=torch.int64))),
+    (True, dict(v=cache(3))), (True, dict(v=cache(8, 32))), (True, dict(v=torch.zeros(4, 2, 64, 8, 128, dtype=BF)[:, 1])),
+    (True, dict(k=cache(8)[::2])), (True, dict(v=cache(heads=4))), (True, dict(cu_seqlens_k=ints(3, dtype=torch.int64))),
+    (True, dict(cu_seqlens_k=ints(2))), (True, dict(cu_seqlens_k=None)), (True, dict(block_table=torch.zeros(2, 5, dtype=torch.int32))),
+    (True, dict(block_table=ints(2, 5, dtype=torch.int64))), (True, dict(block_table=ints(1, 5)))])
+def test_prefill_refuses(calls, cached, changed):
+    with pytest.raises((AssertionError, TypeError)):
+        kv_store.prefill_attention(**prefill_args(cached, **changed))
+    assert not calls
