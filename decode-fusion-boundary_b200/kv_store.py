@@ -23,10 +23,11 @@ def _load():
 
     lib = native.lib()
     _store, _prefill, _check = lib.dfb_store_kvcache_words, lib.dfb_prefill_attention_words, native.check
-    _bf16, _i32, _device, _empty = torch.bfloat16, torch.int32, torch.cuda.current_device, torch.empty
-    # the raw handle of the current stream; the public call builds a Stream object (1 us) around it
-    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    _stream = (lambda: raw(_device())) if raw else (lambda: torch.cuda.current_stream().cuda_stream)
+    _bf16, _i32, _empty = torch.bfloat16, torch.int32, torch.empty
+    # the raw handle of the current stream; the public call builds a Stream object (1 us) around it, and the public call for the
+    # device asks first whether CUDA is up, as it is once a tensor lies there (0.2 us against 0.1)
+    _stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (lambda device: torch.cuda.current_stream().cuda_stream)
+    _device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
     _torch = torch
 
 
@@ -46,11 +47,13 @@ def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> No
     v_rows, v_heads, v_dim = value.shape
     assert v_rows >= n and v_heads * v_dim >= d
     # slot s is row s of both caches: their blocks lie one behind the other, and V has as many as K
-    k_shape, v_shape, k_strides, v_strides = k_cache.shape, v_cache.shape, k_cache.stride(), v_cache.stride()
-    slots = k_shape[0] * k_shape[1]
-    assert k_strides[1] == d and v_strides[1] == d and v_shape[0] * v_shape[1] >= slots
-    assert k_strides[0] == k_shape[1] * d or k_shape[0] == 1
-    assert v_strides[0] == v_shape[1] * d or v_shape[0] == 1
+    shape = k_cache.shape
+    slots = shape[0] * shape[1]
+    if not (k_cache.is_contiguous() and v_cache.is_contiguous() and k_cache.numel() == slots * d and v_cache.shape == shape):
+        v_shape, k_strides, v_strides = v_cache.shape, k_cache.stride(), v_cache.stride()
+        assert k_strides[1] == d and v_strides[1] == d and v_shape[0] * v_shape[1] >= slots
+        assert k_strides[0] == shape[1] * d or shape[0] == 1
+        assert v_strides[0] == v_shape[1] * d or v_shape[0] == 1
     assert slot_mapping.numel() == n
     if key.dtype != _bf16 or value.dtype != _bf16 or k_cache.dtype != _bf16 or v_cache.dtype != _bf16:
         raise TypeError("store_kvcache moves bf16 rows")
@@ -60,7 +63,7 @@ def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> No
         return
     code = _store(_store_words(key.data_ptr(), value.data_ptr(), k_stride, v_stride, k_cache.data_ptr(), v_cache.data_ptr(),
                                slot_mapping.data_ptr(), n, d, slots,
-                               status.data_ptr() if status is not None else 0, _stream()))
+                               status.data_ptr() if status is not None else 0, _stream(_device())))
     if code:
         _check(code, "dfb_store_kvcache")
 
@@ -115,7 +118,7 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
         q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), cu_seqlens_q.data_ptr(),
         cu_seqlens_k.data_ptr() if cu_seqlens_k is not None else 0, batch, int(max_seqlen_q),
         q_stride, k_stride, v_stride, q_heads * head_dim, q_heads, kv_heads, head_dim, float(softmax_scale), bt_ptr,
-        bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else 0, n, kv_rows, _stream()))
+        bt_stride, block_size, num_blocks, status.data_ptr() if status is not None else 0, n, kv_rows, _stream(_device())))
     if code:
         _check(code, "dfb_prefill_attention")
     return out

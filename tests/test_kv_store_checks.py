@@ -22,7 +22,8 @@ def calls(monkeypatch):
     seen = []
     for name, form in (("_store", "12q"), ("_prefill", "15qd8q")):
         monkeypatch.setattr(kv_store, name, lambda words, name=name, form=form: seen.append((name, struct.unpack(form, words))) and 0)
-    monkeypatch.setattr(kv_store, "_stream", lambda: 0)
+    monkeypatch.setattr(kv_store, "_device", lambda: 3)
+    monkeypatch.setattr(kv_store, "_stream", lambda device: 4096 + device)
     return seen
 
 
@@ -56,7 +57,7 @@ def test_store_takes(calls, changed):
     n, kc = len(args["key"]), args["k_cache"]
     assert [c for c in calls] == ([] if n == 0 else [("_store", (
         args["key"].data_ptr(), args["value"].data_ptr(), 1024, args["value"].stride(0), kc.data_ptr(), args["v_cache"].data_ptr(),
-        args["slot_mapping"].data_ptr(), n, 1024, kc.shape[0] * kc.shape[1], 0, 0))])
+        args["slot_mapping"].data_ptr(), n, 1024, kc.shape[0] * kc.shape[1], 0, 4099))])
 
 
 @pytest.mark.parametrize("changed", [
@@ -94,7 +95,7 @@ def test_prefill_takes(calls, cached, changed):
         a["q"].data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), a["cu_seqlens_q"].data_ptr(),
         0 if cu_k is None else cu_k.data_ptr(), 2, 4, 2048, k.stride(int(cached)), v.stride(int(cached)), 2048, 16, 8, 128, 0.125,
         table.data_ptr() if cached else 0, table.stride(0) if cached else 0, 64 if cached else 0, len(k) if cached else 0, 0, 6,
-        0 if cached else min(len(k), len(v)), 0))]
+        0 if cached else min(len(k), len(v)), 4099))]
 
 
 @pytest.mark.parametrize("cached,changed", [
