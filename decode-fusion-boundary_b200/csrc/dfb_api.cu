@@ -1200,7 +1200,7 @@ int run_step(DfbHandle* h, int rows, int nsplit, int bt_cols, const StepIo& io, 
 bool wide_usable(const DfbHandle* h) {
   return h->full_geometry && !h->sharded() && h->step_mode == 0 && h->slots_wide && h->lmhead_ctas == 0 && 2 * h->sm_count >= kWideRows &&
          same_chain(h->opt, ChainOptions()) && h->m.vocab % 16 == 0 &&
-         h->m.max_model_len <= kMaxSplits * kAttnChunk;
+         h->m.max_model_len <= kMaxContext;
 }
 
 // ids | positions | active | temperatures | block tables | attention kernel: chunk, 0, (row and chunk, position) of its CTAs
@@ -1218,8 +1218,8 @@ int wide_prepare(DfbHandle* h) {
   const size_t o_r0 = carve(sizeof(bf16) * kWideRows * m.hidden), o_r1 = carve(sizeof(bf16) * kWideRows * m.hidden);
   const size_t o_qkv = carve(sizeof(bf16) * kWideRows * h->qkv_rows()), o_attn = carve(sizeof(bf16) * kWideRows * h->q_size());
   const size_t o_act = carve(sizeof(bf16) * kWideRows * m.intermediate);
-  const size_t o_po = carve(sizeof(float) * kWideRows * m.kv_heads * kWideSplits * 2 * kHeadDim);
-  const size_t o_ml = carve(sizeof(float2) * kWideRows * m.kv_heads * kWideSplits * 2);
+  const size_t o_po = carve(sizeof(float) * kWideRows * m.kv_heads * kRingMaxSplits * 2 * kHeadDim);
+  const size_t o_ml = carve(sizeof(float2) * kWideRows * m.kv_heads * kRingMaxSplits * 2);
   const size_t o_tk = carve(sizeof(unsigned) * (kWideRows * m.kv_heads + 1)), o_seq = carve(sizeof(unsigned));
   const size_t o_parts = carve(sizeof(ArgmaxPart) * kWideRows * h->sm_count), o_tok = carve(sizeof(int) * kWideRows);
   void* slab = nullptr;
@@ -1323,7 +1323,7 @@ int enqueue_wide(DfbHandle* h, int chunks, bool sampling, cudaStream_t stream) {
 // Kernels and attention grid of a wide step of `rows` (9 to 32) rows.
 struct WideGeometry { int groups, chunks; };
 // Positions per CTA of the attention kernel.  A chunk is a serial walk for its CTA (1.1 us per 8 positions), so it is as short
-// as lets all CTAs be resident together, two per SM, and 32 positions at least (a row has 64 partial results).  A CTA more
+// as lets all CTAs be resident together, two per SM, and kRingMinChunk positions at least.  A CTA more
 // than that waits for another to end, and every chunk costs its CTA the norm and rotation of eight heads and a merge.  us per
 // step, chunks of 32 positions where they fit and of 64 otherwise -> this rule: 20 rows, 5 - 1,500 tokens 1,058 -> 1,022; 20
 // rows of 200 - 2,030 1,429 -> 1,215; 32 of them 1,584 -> 1,482; 9 of them 1,065 -> 1,021; 24 x 512 1,075 -> 1,034; where the
@@ -1332,9 +1332,9 @@ int wide_chunk(const DfbHandle* h, const int* positions, int rows) {
   const int places = 2 * h->sm_count;
   long total = 0;
   for (int r = 0; r < rows; ++r) total += positions[r] + 1;
-  int chunk = (int)(total / places) & ~7;      // no shorter one can do
-  if (chunk < kAttnChunk / 2) chunk = kAttnChunk / 2;
-  for (;; chunk += 8) {
+  int chunk = (int)(total / places) / kRingPos * kRingPos;      // no shorter one can do
+  if (chunk < kRingMinChunk) chunk = kRingMinChunk;
+  for (;; chunk += kRingPos) {
     int ctas = 0;
     for (int r = 0; r < rows; ++r) ctas += positions[r] / chunk + 1;
     if (ctas <= places) return chunk;          // (at the longest context at the latest)
@@ -1376,9 +1376,8 @@ int warm_wide(DfbHandle* h, int max_context, bool sampling) {
   h->wide.no_room = false;
   int rc = wide_prepare(h);
   if (rc || !h->use_graph) return rc;
-  constexpr int kHalf = kAttnChunk / 2;
   for (int groups = 2; groups <= kWideRows / 8; ++groups) {
-    const int last = wide_grid(h, 8 * groups * ((max_context + kHalf - 1) / kHalf));
+    const int last = wide_grid(h, 8 * groups * ((max_context + kRingMinChunk - 1) / kRingMinChunk));
     for (int chunks = 1, grid = 0; grid < last; chunks = grid + 1) {
       grid = wide_grid(h, chunks);
       for (int s = 0; s < (sampling ? 2 : 1); ++s) {
@@ -1434,8 +1433,8 @@ int dfb_create(const DfbModelDesc* d, DfbHandle** out) {
   const bool i_ok = inter == 3072 || inter == 1536 || inter == 768 || inter == 384;
   if (d->hidden != 1024 || d->head_dim != kHeadDim || d->q_heads != 2 * d->kv_heads || d->kv_heads < 1 ||
       d->kv_heads > 8 || d->layers < 1 || d->vocab % kTileRows || d->vocab < kTileRows || !q_ok || !i_ok ||
-      d->max_model_len < 1 || d->max_model_len > kMaxSplits * kAttnChunk || d->block_size < kAttnChunk ||
-      d->block_size % kAttnChunk || d->num_blocks < 1)
+      d->max_model_len < 1 || d->max_model_len > kMaxContext || d->block_size < kMinBlock ||
+      d->block_size % kMinBlock || d->num_blocks < 1)
     return DFB_E_GEOMETRY;
   if (!d->embed || !d->final_norm || !d->rope_cos_sin || !d->layer_weights || !d->k_cache || !d->v_cache)
     return DFB_E_BAD_ARG;

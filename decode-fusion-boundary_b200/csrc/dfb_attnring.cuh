@@ -2,8 +2,8 @@
 // computation as paged_attention_kernel (q/k RMSNorm + RoPE + KV-cache write +
 // split-KV attention with an in-kernel merge), organised for streaming.
 //
-// A CTA owns one batch row and one chunk of 64 context positions for ALL eight
-// KV heads.  In the cache ([block][position][kv_head][128]) the eight heads of a
+// A CTA owns one batch row and one chunk of its context (64 or 32 positions, or
+// as many as the step says) for ALL eight KV heads.  In the cache ([block][position][kv_head][128]) the eight heads of a
 // position are one contiguous 2 KB run for K and one for V, and consecutive
 // positions of a block follow one another, so a stage of 8 positions is ONE
 // bulk copy (TMA, completion on an mbarrier) of 16 KB for K and one for V into
@@ -42,7 +42,6 @@ constexpr int kRingStages = 3;
 constexpr int kRingHeads = 8;                        // KV heads = warps
 constexpr int kRingRowBytes = kRingHeads * kHeadDim * 2;         // one position: 2 KB, dense
 constexpr int kRingStageBytes = 2 * kRingPos * kRingRowBytes;    // K rows, then V rows
-constexpr int kRingSubs = kAttnChunk / kRingPos;     // stages a full chunk goes through
 constexpr int kRingThreads = 32 * kRingHeads;
 constexpr int kRingSmemBytes = kRingStages * kRingStageBytes + 128;
 constexpr int kKernelAttnRing = 7;
@@ -99,8 +98,13 @@ __device__ __forceinline__ float warp_sum(float v) {
 // uneven lengths, whose contexts are cut into chunks of a.chunk[0] positions (a multiple of 8) and dealt to a 1-D grid, so
 // that it is as large as the work; a.chunk[2 + 2 i] = row << 16 | chunk of CTA i (-1: none), then the row's position.  The
 // host takes the chunk that gives every CTA a place, two per SM, and no CTA a second turn (wide_chunk in dfb_api.cu).
-constexpr int kRingMaxSplits = 64;                   // chunks of a row with CH = 0: of 32 positions at least
-constexpr int kRingMaxBlocks = 33;                   // blocks that a chunk can touch: 2,048 positions in blocks of 64
+constexpr int kRingMinChunk = kAttnChunk / 2;                      // shortest chunk with CH = 0
+constexpr int kRingMaxSplits = kMaxContext / kRingMinChunk;        // chunks of a row then: stride and size of its partial results
+constexpr int kRingMaxBlocks = kMaxContext / kMinBlock + 1;        // blocks that a chunk can touch, wherever it begins
+static_assert(kRingMaxSplits * kRingMinChunk >= kMaxContext, "partial results for the longest context in the shortest chunks");
+static_assert(kRingMaxSplits <= 64, "the merge holds two chunks per lane");
+static_assert(kRingMinChunk % kRingPos == 0 && kMinBlock % kRingPos == 0, "a stage lies in one chunk and in one block");
+static_assert(kRingMaxBlocks <= kRingThreads, "one thread per block of a chunk");
 template <int CH>
 __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(const AttnArgs a) {
   static_assert(CH == 0 || CH == kAttnChunk || 2 * CH == kAttnChunk, "64 or 32 positions per CTA, or what the step says");
@@ -132,6 +136,11 @@ __global__ void __launch_bounds__(kRingThreads, 2) paged_attention_ring_kernel(c
     ctx = nsplits * chunk;
     pos = ctx - 1;
     write_ok = false;
+  }
+  if (kPacked && (chunk < kRingMinChunk || chunk % kRingPos || chunk > (kRingMaxBlocks - 1) * a.block_size || nsplits > kRingMaxSplits)) {
+    // (nothing that the host stages: every CTA of the row leaves, so that no ticket is taken)
+    if (split == 0) report_status(a.status, kStatusBadGrid, kKernelAttnRing, row, chunk);
+    return;
   }
   if (split >= nsplits) return;
 

@@ -29,7 +29,9 @@ constexpr int kTileRows = 8;          // weight rows per tile = N of mma.m16n8k1
 constexpr int kAttnThreads = 128;
 constexpr int kAttnChunk = 64;        // context positions per attention CTA
 constexpr int kHeadDim = 128;
-constexpr int kMaxSplits = 32;        // 2048 / kAttnChunk
+constexpr int kMaxSplits = 32;
+constexpr int kMaxContext = kMaxSplits * kAttnChunk;   // longest model length
+constexpr int kMinBlock = kAttnChunk;                  // shortest block of the cache, and what its length is a multiple of
 
 enum GemvMode : int {
   kModeStore = 0,      // plain x, bf16 store            (o_proj, down_proj)

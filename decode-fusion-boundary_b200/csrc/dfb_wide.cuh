@@ -28,7 +28,6 @@ namespace dfb {
 
 constexpr int kWideRows = 32;                        // = DFB_MAX_SLOTS
 constexpr int kKernelWide = 8;
-constexpr int kWideSplits = 2 * kMaxSplits;           // partial results of a row: chunks of 32 positions at least
 constexpr int kWideCluster = 4;                       // CTAs that share the norm (QKV, gate / up) or K (o_proj, down_proj)
 
 template <int NG, int MODE>

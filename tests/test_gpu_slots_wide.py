@@ -327,23 +327,39 @@ def test_wide_step_against_the_oracle(model, cuda_device, n):
         assert H.token_gap_ok(logits[i].float(), got[0][i], int(tokens[i])), i
 
 
-@pytest.mark.parametrize("block_size,lengths", [
-    (256, [2030 - 11 * i for i in range(9)]),                     # chunks of 64 positions and more, four blocks and a rest
-    (256, [1200 + 37 * i for i in range(20)]),                    # of about 110: across the ends of blocks
-    (64, [1990 - 9 * i for i in range(32)]),                      # of about 220 in blocks of 64: four or five blocks each
-    (192, [511, 0, 1, 63, 64, 191, 192, 193, 2047, 1535, 1536, 1537, 1000, 999, 40, 39, 41]),
-    (64, [31, 32, 33, 7, 8, 0, 63, 64, 65])])                     # of 32, the shortest
-def test_chunks_of_every_length(cuda_device, block_size, lengths):
+def _chunk(lengths, places=2 * 148):
+    """Positions per CTA that a wide step takes: the shortest multiple of 8 from 32 on with a place for every CTA."""
+    return next(c for c in range(32, 2049, 8) if sum(n // c + 1 for n in lengths) <= places)
+
+
+@pytest.mark.parametrize("chunk,block_size,lengths", [
+    (72, 256, [2030 - 11 * i for i in range(10)]),                # across the ends of blocks
+    (112, 256, [1200 + 37 * i for i in range(20)]),
+    (216, 64, [1990 - 9 * i for i in range(32)]),                 # four or five blocks each
+    (232, 64, [2046 - i % 3 for i in range(32)]),                 # the longest there is
+    (232, 256, [2046 - i % 3 for i in range(32)]),
+    (40, 192, [511, 0, 1, 63, 64, 191, 192, 193, 2047, 1535, 1536, 1537, 1000, 999, 40, 39, 41]),
+    (32, 64, [i % 8 for i in range(29)] + [2046, 1023, 2047]),    # the shortest: 64 partial results, the last of the last row among them
+    (32, 64, [31, 32, 33, 7, 8, 0, 63, 64, 65])])
+def test_chunks_of_every_length(cuda_device, chunk, block_size, lengths):
     """The attention of a wide step cuts the contexts into chunks that follow their sum: from 32 positions on, across block
-    boundaries, several blocks long.  One step against launches of 8 rows; the blocks of a row lie scattered."""
+    boundaries, several blocks long.  Two steps, between them some sequences retire and the list of chunks gets shorter, against
+    launches of 8 rows: tokens, and the caches; the blocks of a row lie scattered."""
     from dfb_b200 import native
     from dfb_b200.slots import SlotRuntime
+    if torch.cuda.get_device_properties(0).multi_processor_count == 148:
+        assert _chunk(lengths) == chunk
     g = H.oracle_geometry(layers=2, vocab=2048, block_size=block_size)
     w = O.make_weights(g, seed=17, norm="random").to(BF)
-    need = [n // block_size + 1 for n in lengths]
+    signs = torch.from_numpy(np.random.Generator(np.random.Philox(key=18)).integers(0, 2, g.hidden)).to(BF) * 2 - 1
+    w.embed.copy_(torch.randn(g.vocab, g.hidden, generator=torch.Generator().manual_seed(19)) * 0.5)       # (as in `model`)
+    w.embed[1::2] = w.embed[0::2] * signs
+    w.final_norm.copy_(signs)
+    need = [min(n + 1, 2047) // block_size + 1 for n in lengths]
     order = np.random.Generator(np.random.Philox(key=8)).permutation(sum(need)).tolist()
     tables = [[order.pop() for _ in range(k)] for k in need]
     history = (torch.randn(tuple(O.new_kv_cache(g, sum(need), BF).shape), generator=torch.Generator().manual_seed(3)) * 0.5).to(BF).cuda()
+    leave = [i for i in range(len(lengths)) if i % 3 == 1][:len(lengths) - 9]
     sides = []
     for wide in (1, 0):
         kv = history.clone()
@@ -352,9 +368,22 @@ def test_chunks_of_every_length(cuda_device, block_size, lengths):
         rt = SlotRuntime(dec)
         for i, (n, table) in enumerate(zip(lengths, tables)):
             rt.admit(i, 100 + 7 * i, n, table)
-        rt.step()
+        tokens = [rt.step()]
+        for i in leave:
+            rt.retire(i)
+        tokens.append(rt.step())
         assert dec.status()[0] == 0
         dec.close()
-        sides.append(kv)
-    assert torch.equal((sides[0] != history).any(dim=-1), (sides[1] != history).any(dim=-1))
-    assert float((sides[0].float() - sides[1].float()).abs().max()) <= 2.0 ** -5       # (as above: layer 2's new rows)
+        sides.append((kv, tokens))
+    (kv, tokens), (want_kv, want) = sides
+    assert tokens == want and set(tokens[0]) == set(range(len(lengths)))
+    assert set(tokens[1]) == {i for i, n in enumerate(lengths) if i not in leave and n < 2047}
+    assert torch.equal((kv != history).any(dim=-1), (want_kv != history).any(dim=-1))
+    # A new value of layer 2 is a dot product of 1,024 normalised inputs, each of which may lie an ulp (2^-8) apart on the two
+    # sides: 2^-8 rms, 4.5 times that among 2^16 values.  Four roundings follow (the product, two of the norm, the rotation), each
+    # an ulp of the value and its rotation partner.
+    new = (want_kv != history).any(dim=-1)
+    got, ref = kv[new].float(), want_kv[new].float()
+    pair = torch.hypot(ref[:, :64], ref[:, 64:]).repeat(1, 2)
+    bound = 2.0 ** -8 * (4 * pair + 4.5 * ref.square().mean(dim=-1, keepdim=True).sqrt())
+    assert bool(((got - ref).abs() <= bound).all()), float(((got - ref).abs() / bound).max())
