@@ -85,23 +85,33 @@ def test_prefill_attention_argument_checks_need_no_device():
 
 
 def test_calls_by_words_check_as_the_others_do():
-    """The two prefill calls that take their arguments as a block of 64-bit words hand every word to its place."""
+    """The two prefill calls that take their arguments as a block of 64-bit words refuse what the typed ones refuse, word for
+    word.  What has no check on the host (slots, scale, status, row counts, stream, and which of two pointers is which) is seen
+    by the GPU tests alone, whose calls all go this way."""
     import struct
     lib = native.lib()
     one = 16
+    pointer = lambda w, at: [None if i in at and x == 0 else x for i, x in enumerate(w)]
     store = (one, one, 1024, 1024, one, one, one, 1, 1024, 10, 0, 0)
-    for i, value, want in ((0, 0, -1), (1, one + 2, -1), (2, 512, -1), (3, 512, -1), (4, 0, -1), (5, 0, -1), (6, 0, -1), (7, -1, -1),
-                           (7, 0, 0), (8, 1020, -1), (9, 0, -1)):
+    for i, value, want in ((0, 0, -1), (0, one + 2, -1), (1, 0, -1), (1, one + 2, -1), (2, 512, -1), (2, 1028, -1), (3, 512, -1), (3, 1028, -1),
+                           (4, 0, -1), (4, one + 2, -1), (5, 0, -1), (5, one + 2, -1), (6, 0, -1), (7, -1, -1), (7, 0, 0), (8, 1020, -1),
+                           (8, 0, -1), (9, 0, -1)):
         words = list(store)
         words[i] = value
         assert lib.dfb_store_kvcache_words(struct.pack("12q", *words)) == want, (i, value)
-        words[10:] = [None, None]
-        assert lib.dfb_store_kvcache(*words) == want
-    prefill = (one, one, one, one, one, 0, 1, 8, 4096, 4096, 4096, 2048, 16, 8, 128, 0.088, 0, 0, 0, 0, 0, 0, 0, 0)
-    for i, value, want in ((0, 0, -1), (4, 0, -1), (8, 1000, -1), (9, 4100, -1), (11, 8, -1), (13, 5, -2), (14, 64, -2), (16, one, -1)):
-        words = list(prefill)
-        words[i] = value
-        assert lib.dfb_prefill_attention_words(struct.pack("15qd8q", *words)) == want, (i, value)
+        assert lib.dfb_store_kvcache(*pointer(words, (0, 1, 4, 5, 6, 10, 11))) == want, (i, value)
+    fresh = (one, one, one, one, one, 0, 1, 8, 4096, 4096, 4096, 2048, 16, 8, 128, 0.088, 0, 0, 0, 0, 0, 0, 0, 0)
+    cached = fresh[:5] + (one,) + fresh[6:16] + (one, 4, 256, 8, 0, 0, 0, 0)
+    both = ((0, 0, -1), (1, 0, -1), (2, 0, -1), (3, 0, -1), (0, 18, -1), (1, 18, -1), (2, 18, -1), (3, 18, -1), (4, 0, -1), (6, 0, -1),
+            (6, -1, -1), (7, 0, -1), (7, -1, -1), (8, 1000, -1), (8, 4100, -1), (9, 512, -1), (9, 4100, -1), (10, 512, -1), (10, 4100, -1),
+            (11, 8, -1), (11, 2052, -1), (12, 0, -2), (12, 15, -2), (13, 0, -2), (13, 5, -2), (14, 64, -2))
+    for base, changes in ((fresh, both + ((16, one, -1),)),
+                          (cached, both + ((5, 0, -1), (17, 0, -1), (18, 0, -1), (18, 192, -2), (19, 0, -1)))):
+        for i, value, want in changes:
+            words = list(base)
+            words[i] = value
+            assert lib.dfb_prefill_attention_words(struct.pack("15qd8q", *words)) == want, (i, value)
+            assert lib.dfb_prefill_attention_rows(*pointer(words, (0, 1, 2, 3, 4, 5, 16, 20, 23))) == want, (i, value)
 
 
 def test_words_beyond_32_bits_are_refused():
