@@ -38,14 +38,15 @@ def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> No
     ``status``: optional int32 CUDA tensor ``[4]`` that receives a bad slot."""
     if _torch is None:
         _load()
-    n, num_heads, head_dim = key.shape
+    rows = key.shape
+    n, num_heads, head_dim = rows
     d = num_heads * head_dim
     k_stride, k_head, k_one = key.stride()
     v_stride, v_head, v_one = value.stride()
     assert k_one == 1 and v_one == 1
     assert k_head == head_dim and v_head == head_dim
-    v_rows, v_heads, v_dim = value.shape
-    assert v_rows >= n and v_heads * v_dim >= d
+    v_rows = value.shape
+    assert v_rows == rows or (v_rows[0] >= n and v_rows[1] * v_rows[2] >= d)
     # slot s is row s of both caches: their blocks lie one behind the other, and V has as many as K
     shape = k_cache.shape
     slots = shape[0] * shape[1]
@@ -55,7 +56,7 @@ def store_kvcache(key, value, k_cache, v_cache, slot_mapping, status=None) -> No
         assert k_strides[0] == shape[1] * d or shape[0] == 1
         assert v_strides[0] == v_shape[1] * d or v_shape[0] == 1
     assert slot_mapping.numel() == n
-    if key.dtype != _bf16 or value.dtype != _bf16 or k_cache.dtype != _bf16 or v_cache.dtype != _bf16:
+    if not (key.dtype is value.dtype is k_cache.dtype is v_cache.dtype is _bf16):
         raise TypeError("store_kvcache moves bf16 rows")
     if slot_mapping.dtype != _i32 or not slot_mapping.is_cuda:
         raise TypeError("slot_mapping must be an int32 CUDA tensor")
