@@ -846,10 +846,12 @@ int launch_attention(Launcher& L, DfbHandle* h, int layer, const bf16* qkv, cons
   if (nsplit_arg >= kClusterFlag) {
     a.ctx_limit = nsplit * kAttnChunk;
     const int cs = 2 << (nsplit_arg / kClusterFlag - 1);
-    // o_proj is let in behind this kernel's own dependency: CTAs of o_proj that come while QKV still runs take the places of
-    // this kernel's clusters (us per step, early / late: 3 x 300 tokens 564 / 550, 4 x 300 575 / 562, 5 x 1,000 695 / 690, 8 x
-    // 520 652.6 / 650.0, 8 x 1,000 720.8 / 717.7, 8 x 2,000 883.9 / 882.3).  Not the small grids with two CTAs (8 x 150 567.6 /
-    // 570.4) nor the chunked kernels (3 x 520 606 / 600, but 3 x 150 539 / 564, 5 x 520 626 / 633, 418 + 97 + 650 sampled slower).
+    // Clusters of 4 and 8 let o_proj in behind their own dependency wait, whatever the option says.  Measured, not explained
+    // (us per step, trigger at the start / behind the wait; runs differ by 0.5): with 4 CTAs 3 x 300 tokens 564 / 551, 4 x 300 577 /
+    // 565, 3 x 500 568 / 555, 6 x 450 636 / 629, 8 x 500 655.4 / 653.7, 5 x 1,000 703 / 696, 8 x 640 707 / 704, 8 x 2,000 898 / 895;
+    // with 8 3 x 1,750 717.5 / 711.5, 3 x 2,000 720 / 714, 4 x 1,300 718 / 713, 4 x 1,700 734 / 730, 4 x 2,040 739.5 / 737, 2,040 + 600
+    // + 1,200 + 300 688.4 / 686.3, 1,900 + 97 + 418 even.  Not the small grids with two CTAs (8 x 150 567.6 / 570.4) nor the
+    // chunked kernels (3 x 520 606 / 600, but 3 x 150 539 / 564, 5 x 520 626 / 633, 418 + 97 + 650 sampled slower).
     a.late_trigger = L.opt->late_trigger || cs >= 4;
     auto kernel = cs == 8 ? cluster_attention_kernel<8> : cs == 4 ? cluster_attention_kernel<4> : cluster_attention_kernel<2>;
     L.launch(kernel, dim3(cs, m.kv_heads, rows), dim3(kCaThreads), a, true, 0, cs);

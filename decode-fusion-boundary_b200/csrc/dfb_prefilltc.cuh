@@ -312,9 +312,8 @@ __global__ void __launch_bounds__(pf_threads(SPLIT), 1) prefill_tc_kernel(const 
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   pdl_wait();      // nothing above reads what an earlier kernel wrote
-  // Behind the wait: a call after the next one would otherwise take SMs before the next one has begun (us per call, calls queued
-  // back to back, trigger before / behind the wait: 512 tokens 11.6 / 11.1, 640 13.9 / 12.4, 400 11.3 / 10.7, 300 + 200 + 100
-  // 11.4 / 10.6; large batches even).
+  // Behind the wait.  Measured, not explained (us per call, calls queued back to back, trigger before / behind the wait: 512 tokens
+  // 11.6 / 11.1, 640 13.9 / 12.4, 400 11.3 / 10.7, 300 + 200 + 100 11.4 / 10.6; large batches even).
   pdl_launch_dependents();
   static_assert(!SPLIT || !PAIRS, "the split form takes one head at a time");
   PfWalk<PAIRS, SPLIT> walk;

@@ -170,8 +170,9 @@ typedef struct DfbStatus {
                                         kernels of the FP32 chain ask for as shared memory (default 12) */
 #define DFB_OPT_SMEM_CARVEOUT_MMA 10 /* the same for the tensor-core chains (default 50; 100 when a per-layer
                                         projection runs on tcgen05) */
-#define DFB_OPT_LATE_TRIGGER 11 /* FP32 chain: 0 (default) = a kernel lets its successor start (and request its
-                                  weights) at once, 1 = only after it has read its own inputs */
+#define DFB_OPT_LATE_TRIGGER 11 /* chains of 1 to 8 rows: 0 (default) = a kernel lets its successor start (and request its
+                                  weights) at once, 1 = only after it has read its own inputs.  The cluster attention
+                                  with 4 or 8 CTAs per (row, KV head) always does the latter */
 #define DFB_OPT_PAIR_GEMV 12    /* mma.sync chain, K = 1024: 1 (default) = 16 weight rows per MMA (pair_gemv_kernel),
                                   0 = 8 weight rows per MMA (stream_gemv_kernel) */
 #define DFB_OPT_BULK_X 13       /* FP32 chain: 1 (default) = the fused norm fetches x and the residual with bulk
