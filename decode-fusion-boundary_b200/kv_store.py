@@ -94,8 +94,9 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
         assert cu_seqlens_k.numel() > batch
     # K and V are read at the same places: V has what K has
     if block_table is not None:
-        num_blocks, block_size, kv_heads, k_dim = k.shape
-        v_blocks, v_block_size, v_heads, v_dim = v.shape
+        num_blocks, block_size, kv_heads = k.shape[:3]
+        v_blocks, v_block_size, v_heads = v.shape[:3]
+        k_rows, v_rows = num_blocks * block_size, v_blocks * v_block_size
         k_stride, v_stride, kv_rows = k_strides[1], v_strides[1], 0
         assert k_strides[2] == head_dim and v_strides[2] == head_dim and k_strides[0] == block_size * k_stride
         assert v_blocks >= num_blocks and v_block_size == block_size and (v_strides[0] == block_size * v_stride or v_blocks == 1)
@@ -104,14 +105,14 @@ def prefill_attention(q, k, v, cu_seqlens_q, max_seqlen_q: int, softmax_scale: f
         assert block_table.shape[0] >= batch
         bt_ptr, bt_stride = block_table.data_ptr(), block_table.stride(0)
     else:
-        k_rows, kv_heads, k_dim = k.shape
-        v_rows, v_heads, v_dim = v.shape
+        k_rows, kv_heads = k.shape[:2]
+        v_rows, v_heads = v.shape[:2]
         kv_rows = min(k_rows, v_rows)
         assert k_strides[1] == head_dim and v_strides[1] == head_dim
         num_blocks = block_size = 0
         k_stride, v_stride = k_strides[0], v_strides[0]
         bt_ptr, bt_stride = 0, 0
-    assert v_heads >= kv_heads and k_dim == head_dim and v_dim == head_dim
+    assert v_heads >= kv_heads and k.numel() == k_rows * kv_heads * head_dim and v.numel() == v_rows * v_heads * head_dim
     out = _empty((n, q_heads, head_dim), dtype=_bf16, device=q.device)
     if n == 0:
         return out

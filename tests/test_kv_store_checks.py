@@ -83,7 +83,8 @@ def prefill_args(cached=False, **changed):
 
 @pytest.mark.parametrize("cached,changed", [
     (False, dict()), (False, dict(cu_seqlens_k=ints(3))), (False, dict(v=torch.zeros(6, 4096, dtype=BF)[:, 3072:].view(6, 8, 128))),
-    (False, dict(k=rows(9))), (False, dict(v=rows(9))), (False, dict(cu_seqlens_k=ints(7))), (True, dict()), (True, dict(v=cache(6))),
+    (False, dict(k=rows(9))), (False, dict(v=rows(9))), (False, dict(v=rows(6, 16))), (False, dict(cu_seqlens_k=ints(7))),
+    (False, dict(k=rows(6).view(6, 8, 2, 64), v=rows(6).view(6, 8, 1, 128))), (True, dict(k=cache().view(4, 64, 8, 2, 64))), (True, dict()), (True, dict(v=cache(6))),
     (True, dict(k=torch.zeros(2, 4, 64, 8, 128, dtype=BF)[0], block_table=ints(3, 8)[:, :2])),
     (True, dict(k=cache(1), v=torch.zeros(1, 2, 64, 8, 128, dtype=BF)[:, 0]))])
 def test_prefill_takes(calls, cached, changed):
